@@ -126,6 +126,15 @@ __device__ __forceinline__ int gather_polygon(const double* __restrict__ v, cons
     return len;
 }
 
+// The bits of a float64, opaque to the compiler: tests on the bits of a plain
+// reinterpretation (zero, finite, not NaN) are recognised and turned back
+// into float64 comparisons, each 20 cycles of the float64 unit.
+__device__ __forceinline__ unsigned long long dbits(double x) {
+    unsigned long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
+}
+
 // Monotone 64-bit integer key of a float64 (non-NaN): x < y <=> key(x) < key(y),
 // with -0.0 and +0.0 sharing one key (they compare equal as floats).
 __device__ __forceinline__ unsigned long long fkey(double x) {

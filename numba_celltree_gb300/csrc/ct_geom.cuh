@@ -393,18 +393,18 @@ __device__ __forceinline__ double clip_area(const dpt* polygon, int n_poly, cons
 // for that clip edge.  Order comparisons and zero tests run on integer keys.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ bool g_notnan(double x) {
-    return ((unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull) <= 0x7ff0000000000000ull;
+    return (dbits(x) & 0x7fffffffffffffffull) <= 0x7ff0000000000000ull;
 }
 __device__ __forceinline__ bool g_finite(double x) {
-    return ((unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull) < 0x7ff0000000000000ull;
+    return (dbits(x) & 0x7fffffffffffffffull) < 0x7ff0000000000000ull;
 }
 // x == 0.0 (either sign)
-__device__ __forceinline__ bool g_zero(double x) { return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull; }
+__device__ __forceinline__ bool g_zero(double x) { return (dbits(x) << 1) == 0ull; }
 // x > y, false when either is NaN (the float64 comparison)
 __device__ __forceinline__ bool g_gt(double x, double y) { return g_notnan(x) && g_notnan(y) && fkey(x) > fkey(y); }
 // x == y as values for finite x, y (bit patterns equal, or both zeros)
 __device__ __forceinline__ bool g_eq_finite(double x, double y) {
-    unsigned long long a = (unsigned long long)__double_as_longlong(x), b = (unsigned long long)__double_as_longlong(y);
+    unsigned long long a = dbits(x), b = dbits(y);
     return a == b || ((a | b) << 1) == 0ull;
 }
 // b - a == (0, 0): both coordinates finite and equal

@@ -9,8 +9,10 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "ct_common.cuh"
+#include "ct_clip.cuh"
 #include "ct_geom.cuh"
 #include "ct_internal.h"
 #include "ct_locf.cuh"
@@ -1498,43 +1500,87 @@ __global__ void k_sat(const double* __restrict__ va, const int64_t* __restrict__
     out[i] = (uint8_t)r;
 }
 
+// One pair's area by the general clip (polygons in local memory).
+__device__ __noinline__ double clip_pair_general(const double4* __restrict__ boxes, const double* __restrict__ va,
+                                                 const int64_t* __restrict__ fa, int Ka, int64_t ia,
+                                                 const double* __restrict__ vb, const int64_t* __restrict__ fb,
+                                                 int Kb, int64_t ib, unsigned int* __restrict__ err) {
+    dpt a[CT_MAX_N_VERTEX], b[CT_MAX_N_VERTEX];
+    dpt A[CT_CLIP_MAX], B[CT_CLIP_MAX];
+    int la = 4;
+    if (boxes) {
+        const double4 q = boxes[ia];
+        a[0] = mkp(q.x, q.z);
+        a[1] = mkp(q.y, q.z);
+        a[2] = mkp(q.y, q.w);
+        a[3] = mkp(q.x, q.w);
+    } else {
+        la = load_poly(va, fa, Ka, ia, a);
+    }
+    int lb = load_poly(vb, fb, Kb, ib, b);
+    bool of = false;
+    const double area = clip_area_conv(a, la, b, lb, A, B, &of);
+    if (of) set_error(err, CT_DEVERR_CLIP);
+    return area;
+}
+
 // area_of_intersection sutherland_hodgman.py:151-168 (subject: face of a,
-// clipper: face of b)
+// clipper: face of b) and, with `boxes`, box_area_of_intersection 171-187
+// (subject: the box).
 // `order`: NULL, or a permutation of the pairs (processing order only:
 // pairs of equal polygon lengths side by side, so a warp's lanes run the
 // same number of clip edges; results stay at their pair's index).
-__global__ void k_clip_area(const double* __restrict__ va, const int64_t* __restrict__ fa, int Ka,
-                            const double* __restrict__ vb, const int64_t* __restrict__ fb, int Kb,
-                            const int64_t* __restrict__ ia, const int64_t* __restrict__ ib, int64_t n,
-                            const int* __restrict__ order, double* __restrict__ out, unsigned int* __restrict__ err) {
+__global__ void k_clip_area(const double4* __restrict__ boxes, const double* __restrict__ va,
+                            const int64_t* __restrict__ fa, int Ka, const double* __restrict__ vb,
+                            const int64_t* __restrict__ fb, int Kb, const int64_t* __restrict__ ia,
+                            const int64_t* __restrict__ ib, int64_t n, const int* __restrict__ order,
+                            double* __restrict__ out, unsigned int* __restrict__ err) {
     int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int64_t i = order ? (int64_t)order[t] : t;
-    dpt a[CT_MAX_N_VERTEX], b[CT_MAX_N_VERTEX];
-    dpt A[CT_CLIP_MAX], B[CT_CLIP_MAX];
-    int la = load_poly(va, fa, Ka, ia[i], a);
-    int lb = load_poly(vb, fb, Kb, ib[i], b);
-    bool of = false;
-    out[i] = clip_area_conv(a, la, b, lb, A, B, &of);
-    if (of) set_error(err, CT_DEVERR_CLIP);
+    out[i] = clip_pair_general(boxes, va, fa, Ka, ia[i], vb, fb, Kb, ib[i], err);
 }
 
-// box_area_of_intersection sutherland_hodgman.py:171-187 (subject: the box)
-__global__ void k_box_area(const double4* __restrict__ boxes, const double* __restrict__ vb,
-                           const int64_t* __restrict__ fb, int Kb, const int64_t* __restrict__ ibox,
-                           const int64_t* __restrict__ iface, int64_t n, const int* __restrict__ order,
-                           double* __restrict__ out, unsigned int* __restrict__ err) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The same for polygons of at most CL_SLOTS (subject) and KT (clipper)
+// vertices: ct_clip.cuh, the general clip where it does not apply.
+template <int KT, bool BOX>
+__global__ void __launch_bounds__(CL_THREADS) k_clip_area_small(
+    const double4* __restrict__ boxes, const double2* __restrict__ va, const int64_t* __restrict__ fa, int Ka,
+    const double2* __restrict__ vb, const int64_t* __restrict__ fb, int Kb, const int64_t* __restrict__ ia,
+    const int64_t* __restrict__ ib, int64_t n, const int* __restrict__ order, double* __restrict__ out,
+    unsigned int* __restrict__ err) {
+    __shared__ ClipCols<KT> S;
+    const int tid = threadIdx.x;
+    const int64_t t = (int64_t)blockIdx.x * CL_THREADS + tid;
     if (t >= n) return;
-    int64_t i = order ? (int64_t)order[t] : t;
-    double4 q = boxes[ibox[i]];
-    dpt a[4] = {mkp(q.x, q.z), mkp(q.y, q.z), mkp(q.y, q.w), mkp(q.x, q.w)};
-    dpt b[CT_MAX_N_VERTEX];
-    dpt A[CT_CLIP_MAX], B[CT_CLIP_MAX];
-    int lb = load_poly(vb, fb, Kb, iface[i], b);
-    bool of = false;
-    out[i] = clip_area_conv(a, 4, b, lb, A, B, &of);
-    if (of) set_error(err, CT_DEVERR_CLIP);
+    const int64_t i = order ? (int64_t)order[t] : t;
+    const int64_t ja = ia[i], jb = ib[i];
+    int64_t kb[KT];
+    int lb = Kb;
+#pragma unroll
+    for (int k = 0; k < KT; k++) kb[k] = k < Kb ? fb[jb * Kb + k] : CT_FILL_VALUE;
+#pragma unroll
+    for (int k = KT - 1; k >= 3; k--)
+        if (k < Kb && kb[k] == CT_FILL_VALUE) lb = k;
+    int la = 4;
+    if (BOX) {
+        const double4 q = boxes[ja];
+        S.v[0][tid] = make_double2(q.x, q.z);
+        S.v[1][tid] = make_double2(q.y, q.z);
+        S.v[2][tid] = make_double2(q.y, q.w);
+        S.v[3][tid] = make_double2(q.x, q.w);
+    } else {
+        const int64_t* face = fa + ja * Ka;
+        la = polygon_length(face, Ka);
+        for (int k = 0; k < la; k++) S.v[k][tid] = va[face[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < KT; k++)
+        if (k < lb) S.c[k][tid] = vb[kb[k]];
+    double area;
+    if (!clip_area_small<KT, BOX>(S, tid, la, lb, &area))
+        area = clip_pair_general(boxes, (const double*)va, fa, Ka, ja, (const double*)vb, fb, Kb, jb, err);
+    out[i] = area;
 }
 
 // 6-bit class of a pair: the polygon lengths (3 .. 10) of its two faces
@@ -1898,6 +1944,32 @@ int ct_pack_box_index(ct_tree* t, void* scratch, size_t scratch_bytes, void* str
 }
 
 // block sizes of the traversal kernels (the tree's launch shape, else the defaults)
+// Polygons of up to 8 vertices take the shared-memory clip, longer ones the
+// general one (shared memory of a block: 31, 33 and 41 KB for clippers of up
+// to 3, 4 and 8 vertices).
+static void launch_clip_area(const double4* boxes, const double* va, const int64_t* fa, int Ka, const double* vb,
+                             const int64_t* fb, int Kb, const int64_t* ia, const int64_t* ib, int64_t n,
+                             const int* order, double* out, unsigned int* err, cudaStream_t st) {
+    const unsigned grid = grid_of(n, CL_THREADS);
+    const double2 *a = (const double2*)va, *b = (const double2*)vb;
+    if (Ka > CL_SLOTS || Kb > 8 || Ka < 3 || Kb < 3 || (((uintptr_t)va | (uintptr_t)vb) & 15))
+        k_clip_area<<<grid_of(n, 128), 128, 0, st>>>(boxes, va, fa, Ka, vb, fb, Kb, ia, ib, n, order, out, err);
+    else {
+        auto go = [&](auto kt) {
+            constexpr int KT = decltype(kt)::value;
+            if (boxes)
+                k_clip_area_small<KT, true><<<grid, CL_THREADS, 0, st>>>(boxes, a, fa, Ka, b, fb, Kb, ia, ib, n,
+                                                                         order, out, err);
+            else
+                k_clip_area_small<KT, false><<<grid, CL_THREADS, 0, st>>>(boxes, a, fa, Ka, b, fb, Kb, ia, ib, n,
+                                                                          order, out, err);
+        };
+        if (Kb <= 3) go(std::integral_constant<int, 3>());
+        else if (Kb <= 4) go(std::integral_constant<int, 4>());
+        else go(std::integral_constant<int, 8>());
+    }
+}
+
 static int box_threads(const ct_tree* t) {
     int b = t->tune_query_threads;
     return (b == 64 || b == 128 || b == 256) ? b : 256;
@@ -2084,8 +2156,7 @@ int ct_area_of_intersection_ordered(const double* va, const int64_t* fa, int32_t
                                     const int64_t* fb, int32_t Kb, const int64_t* ia, const int64_t* ib, int64_t n,
                                     const int32_t* order, double* out, unsigned int* error_word, void* stream) {
     if (n == 0) return CT_OK;
-    k_clip_area<<<grid_of(n, 128), 128, 0, (cudaStream_t)stream>>>(va, fa, Ka, vb, fb, Kb, ia, ib, n, order, out,
-                                                                    error_word);
+    launch_clip_area(nullptr, va, fa, Ka, vb, fb, Kb, ia, ib, n, order, out, error_word, (cudaStream_t)stream);
     CT_CHECK_LAUNCH("area_of_intersection");
     return CT_OK;
 }
@@ -2100,8 +2171,8 @@ int ct_box_area_of_intersection_ordered(const double* boxes, const double* vb, c
                                         const int64_t* ibox, const int64_t* iface, int64_t n, const int32_t* order,
                                         double* out, unsigned int* error_word, void* stream) {
     if (n == 0) return CT_OK;
-    k_box_area<<<grid_of(n, 128), 128, 0, (cudaStream_t)stream>>>((const double4*)boxes, vb, fb, Kb, ibox, iface, n,
-                                                                   order, out, error_word);
+    launch_clip_area((const double4*)boxes, nullptr, nullptr, 4, vb, fb, Kb, ibox, iface, n, order, out, error_word,
+                     (cudaStream_t)stream);
     CT_CHECK_LAUNCH("box_area_of_intersection");
     return CT_OK;
 }
