@@ -98,14 +98,9 @@ enum { LF_OUTSIDE = 0, LF_INSIDE = 1, LF_UNSURE = 2 };
 // rounding of absolute coordinates, so the float64 crossing abscissa is also
 // resolved.  Otherwise the polygon is UNSURE.
 template <int KT>
-__device__ __forceinline__ int leaf_filter_local(const PtSplit& P, float dabs, float tolf,
-                                                 const float4* __restrict__ cell, int len) {
+__device__ __forceinline__ int leaf_filter_delta(float dx, float dy, float errd, float dabs, float tolf,
+                                                 const float2* __restrict__ rel, int len) {
     const float u = 5.9604644775390625e-08f;
-    if (len < 3) return LF_UNSURE;
-    float4 o = cell[0];
-    const float2* rel = reinterpret_cast<const float2*>(cell + 1);
-    float dx, dy, errd;
-    local_delta(P, o, &dx, &dy, &errd);
     float dmax = fmaxf(fabsf(dx), fabsf(dy));
     float2 rl = rel[len - 2];
     float ux = rl.x - dx, uy = rl.y - dy;
@@ -134,6 +129,15 @@ __device__ __forceinline__ int leaf_filter_local(const PtSplit& P, float dabs, f
         uy = vy;
     }
     return parity ? LF_INSIDE : LF_OUTSIDE;
+}
+
+template <int KT>
+__device__ __forceinline__ int leaf_filter_local(const PtSplit& P, float dabs, float tolf,
+                                                 const float4* __restrict__ cell, int len) {
+    if (len < 3) return LF_UNSURE;
+    float dx, dy, errd;
+    local_delta(P, cell[0], &dx, &dy, &errd);
+    return leaf_filter_delta<KT>(dx, dy, errd, dabs, tolf, reinterpret_cast<const float2*>(cell + 1), len);
 }
 
 // Float32 filter for point_on_edge (geometry_utils.py:226-238): true when the
