@@ -554,6 +554,34 @@ int ct_write_item_candidates(const ct_tree* tree, int32_t mode, const double* se
 int ct_segment_candidate_ranges(const int64_t* item_off, const int64_t* item_cnt, int64_t n,
                                 const int64_t* item_cand_off, const int64_t* item_cand_cnt, int64_t n_items,
                                 int64_t* cand_off, int64_t* cand_cnt, void* stream);
+/* Spatial order of box (kind 0) or segment (kind 1) queries (no upstream
+ * counterpart): a permutation by the 16-bit Morton key of the query's middle
+ * over the tree's bbox, so that queries processed together read the same
+ * nodes and cells; ct_gather_rows takes the queries (4 doubles each) to that
+ * order. */
+size_t ct_spatial_order_workspace_size(int64_t n);
+int ct_spatial_order(const double* queries, int64_t n, int32_t kind, const double* bbox_host4, int32_t* order,
+                     void* workspace, size_t workspace_bytes, void* stream);
+int ct_gather_rows(const double* queries, const int32_t* order, int64_t n, double* out, void* stream);
+
+/* From candidates to results in three calls: the cell test with one byte per
+ * candidate; every segment's hit count (at counts[order[s]] for candidate
+ * segment s, or counts[s]), their exclusive scan, total and largest
+ * (synchronises the stream); and the hits of every segment sorted by t
+ * (sort_intersections_by_edge geometry_utils.py:564-574) and written at its
+ * offset. */
+int ct_test_edge_candidates_u8(const ct_tree* tree, int32_t mode, const double* segs, const int32_t* cand_seg,
+                               const int32_t* cand_pos, int64_t n_cand, uint8_t* keep, double* xy, void* stream);
+size_t ct_edge_hit_counts_workspace_size(int64_t n);
+int ct_edge_hit_counts(const uint8_t* keep, const int64_t* cand_off, const int64_t* cand_cnt, const int32_t* order,
+                       int64_t n, int64_t* counts, int64_t* offsets, void* workspace, size_t workspace_bytes,
+                       int64_t* total_host, int64_t* longest_host, void* stream);
+size_t ct_finish_edge_hits_workspace_size(int64_t total, int64_t longest);
+int ct_finish_edge_hits(const ct_tree* tree, const double* segs, const int32_t* order, const uint8_t* keep,
+                        const int32_t* cand_pos, const double* xy_cand, const int64_t* cand_off,
+                        const int64_t* cand_cnt, int64_t n, const int64_t* counts, const int64_t* offsets,
+                        int64_t total, int64_t longest, int64_t* ii, int64_t* jj, double* xy, void* workspace,
+                        size_t workspace_bytes, void* stream);
 /* Diagnostics for tests of the segment test's float32 certificates (face
  * trees): per (segment, leaf position) pair, out[3t] = upstream's float64
  * Cohen-Sutherland verdict (1 accept, 0 reject), out[3t+1] = the float32

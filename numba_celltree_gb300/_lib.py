@@ -220,6 +220,16 @@ SIGNATURES = {
     "ct_count_item_candidates": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P]),
     "ct_write_item_candidates": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "ct_segment_candidate_ranges": (ctypes.c_int, [_P, _P, _I64, _P, _P, _I64, _P, _P, _P]),
+    "ct_spatial_order_workspace_size": (_SZ, [_I64]),
+    "ct_spatial_order": (ctypes.c_int, [_P, _I64, _I32, _P, _P, _P, _SZ, _P]),
+    "ct_gather_rows": (ctypes.c_int, [_P, _P, _I64, _P, _P]),
+    "ct_test_edge_candidates_u8": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _P]),
+    "ct_edge_hit_counts_workspace_size": (_SZ, [_I64]),
+    "ct_edge_hit_counts": (ctypes.c_int, [_P, _P, _P, _P, _I64, _P, _P, _P, _SZ, ctypes.POINTER(_I64),
+                                          ctypes.POINTER(_I64), _P]),
+    "ct_finish_edge_hits_workspace_size": (_SZ, [_I64, _I64]),
+    "ct_finish_edge_hits": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _P, _P, _P, _P, _P, _P, _I64, _P, _P, _I64,
+                                           _I64, _P, _P, _P, _P, _SZ, _P]),
     "ct_test_edge_candidates": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _P]),
     "ct_compact_edge_hits": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _P, _I64, _P, _P, _P, _P, _P, _I64, _P, _P,
                                             _P, _P, _P, _P]),

@@ -1212,10 +1212,10 @@ __device__ __forceinline__ int edge_face_fast(const TreeQ& T, dpt a, dpt b, int 
 
 // The cell test of every candidate (compute_edge_face_intersect
 // query.py:309-328 / compute_edge_edge_intersect 292-306).
-template <int MODE>
+template <int MODE, typename KeepT>
 __global__ void __launch_bounds__(128) k_edge_test(TreeQ T, const double4* __restrict__ segs,
                                                    const int* __restrict__ cseg, const int* __restrict__ cj,
-                                                   int64_t nc, int64_t* __restrict__ keep, double4* __restrict__ xy) {
+                                                   int64_t nc, KeepT* __restrict__ keep, double4* __restrict__ xy) {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += (int64_t)gridDim.x * blockDim.x) {
         double4 s4 = segs[cseg[t]];
         dpt a = mkp(s4.x, s4.y), b = mkp(s4.z, s4.w);
@@ -1411,7 +1411,8 @@ __global__ void k_tkeys(const double4* __restrict__ segs, const int64_t* __restr
     idx[r] = r;
 }
 
-__device__ __forceinline__ bool kless(unsigned long long ka, int64_t ia, unsigned long long kb, int64_t ib) {
+template <typename I>
+__device__ __forceinline__ bool kless(unsigned long long ka, I ia, unsigned long long kb, I ib) {
     return ka < kb || (ka == kb && ia < ib);
 }
 
@@ -1487,8 +1488,8 @@ __global__ void __launch_bounds__(SORT_T) k_segsort(const int64_t* __restrict__ 
 // last).  (key, idx) pairs are unique, so the order is the stable sort's.
 constexpr int WARP_SORT_MAX = 128;
 
-template <int E>
-__device__ __forceinline__ void warp_bitonic(unsigned long long (&k)[E], int64_t (&x)[E], int lane) {
+template <int E, typename I>
+__device__ __forceinline__ void warp_bitonic(unsigned long long (&k)[E], I (&x)[E], int lane) {
     const unsigned FULL = 0xffffffffu;
 #pragma unroll
     for (int size = 2; size <= 32 * E; size <<= 1) {
@@ -1506,7 +1507,7 @@ __device__ __forceinline__ void warp_bitonic(unsigned long long (&k)[E], int64_t
                             const unsigned long long tk = k[r];
                             k[r] = k[rp];
                             k[rp] = tk;
-                            const int64_t tx = x[r];
+                            const I tx = x[r];
                             x[r] = x[rp];
                             x[rp] = tx;
                         }
@@ -1516,7 +1517,7 @@ __device__ __forceinline__ void warp_bitonic(unsigned long long (&k)[E], int64_t
 #pragma unroll
                 for (int r = 0; r < E; r++) {
                     const unsigned long long pk = __shfl_xor_sync(FULL, k[r], j);
-                    const int64_t px = __shfl_xor_sync(FULL, x[r], j);
+                    const I px = __shfl_xor_sync(FULL, x[r], j);
                     const bool asc = ((r * 32 + lane) & size) == 0;
                     const bool lower = (lane & j) == 0;
                     const bool pless = kless(pk, px, k[r], x[r]);
@@ -1542,7 +1543,7 @@ __device__ __forceinline__ void warp_sort_segment(const unsigned long long* __re
         k[r] = e < c ? kA[o + e] : ~0ull;
         x[r] = e < c ? iA[o + e] : INT64_MAX;
     }
-    warp_bitonic<E>(k, x, lane);
+    warp_bitonic(k, x, lane);
 #pragma unroll
     for (int r = 0; r < E; r++) {
         const int64_t e = r * 32 + lane;
@@ -1584,6 +1585,255 @@ __global__ void k_gather_results(const int64_t* __restrict__ perm, int64_t total
     int64_t s = perm[r];
     jj_out[r] = jj_in[s];
     xy_out[r] = xy_in[s];
+}
+
+// ---------------------------------------------------------------------------
+// From the tested candidates to the results: every segment's hits counted,
+// and, with the offsets known, each segment's hits sorted by t and written in
+// place at once (segments of up to 128 hits by a warp, longer ones by a
+// block).  The candidates may be grouped by segments in another order than
+// the results (`order`: result segment of candidate segment s).  Against
+// compacting the hits, then keys, sort and gather as passes over all results
+// (31M hits of 1M segments: 2.6 ms) this reads the hits once and writes the
+// results once (1.3 ms).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_hit_counts(const uint8_t* __restrict__ keep,
+                                                    const int64_t* __restrict__ coff,
+                                                    const int64_t* __restrict__ ccnt, const int* __restrict__ order,
+                                                    int64_t n, int64_t* __restrict__ counts,
+                                                    unsigned long long* __restrict__ longest) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    int64_t most = 0;
+    for (int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < n; s += warps) {
+        const int64_t c0 = coff[s], m = ccnt[s];
+        int64_t c = 0;
+        for (int64_t k = 0; k < m; k += 32)
+            c += __popc(__ballot_sync(0xffffffffu, k + lane < m && keep[c0 + k + lane]));
+        most = max(most, c);
+        if (lane == 0) counts[order ? (int64_t)order[s] : s] = c;
+    }
+    if (lane == 0 && most > 0) atomicMax(longest, (unsigned long long)most);
+}
+
+struct HitSort {
+    const double4* segs;   // in candidate order
+    const int* order;
+    const uint8_t* keep;
+    const int* cj;
+    const int64_t* bbi;
+    const double4* xy_c;
+    const int64_t *coff, *ccnt, *counts, *offsets;
+    int64_t *ii, *jj;
+    double4* xy;
+};
+
+// sort key of candidate r of a segment from a with direction ab
+__device__ __forceinline__ unsigned long long hit_key(const HitSort& H, int64_t r, double4 s) {
+    const double2 c = *reinterpret_cast<const double2*>(H.xy_c + r);
+    const double abx = s.z - s.x, aby = s.w - s.y;
+    const double acx = c.x - s.x, acy = c.y - s.y;
+    return tkey(acx * abx + acy * aby);
+}
+
+__device__ __forceinline__ void hit_write(const HitSort& H, int64_t out, int64_t seg, int64_t r) {
+    H.ii[out] = seg;
+    H.jj[out] = H.bbi[H.cj[r]];
+    H.xy[out] = H.xy_c[r];
+}
+
+template <int E>
+__device__ __forceinline__ void hit_sort_warp(const HitSort& H, const unsigned long long* sk, const unsigned* si,
+                                              int c, int64_t o, int64_t i, int64_t c0, int lane) {
+    unsigned long long k[E];
+    unsigned x[E];
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const int e = r * 32 + lane;
+        k[r] = e < c ? sk[e] : ~0ull;
+        x[r] = e < c ? si[e] : ~0u;
+    }
+    warp_bitonic(k, x, lane);
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const int e = r * 32 + lane;
+        if (e < c) hit_write(H, o + e, i, c0 + x[r]);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_finish_warp(HitSort H, int64_t n, int* __restrict__ list,
+                                                     unsigned long long* __restrict__ nlist) {
+    __shared__ unsigned long long keys[8][WARP_SORT_MAX];
+    __shared__ unsigned idx[8][WARP_SORT_MAX];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long* sk = keys[w];
+    unsigned* si = idx[w];
+    const int64_t warps = (int64_t)gridDim.x * 8;
+    for (int64_t s = (int64_t)blockIdx.x * 8 + w; s < n; s += warps) {
+        const int64_t i = H.order ? (int64_t)H.order[s] : s;
+        const int64_t c = H.counts[i];
+        if (c == 0) continue;
+        if (c > WARP_SORT_MAX) {
+            if (lane == 0) list[atomicAdd(nlist, 1ull)] = (int)s;
+            continue;
+        }
+        const int64_t c0 = H.coff[s], m = H.ccnt[s], o = H.offsets[i];
+        const double4 sg = H.segs[s];
+        int have = 0;
+        for (int64_t k = 0; k < m; k += 32) {
+            const bool hit = k + lane < m && H.keep[c0 + k + lane];
+            const unsigned b = __ballot_sync(0xffffffffu, hit);
+            if (hit) {
+                const int p = have + __popc(b & ((1u << lane) - 1u));
+                sk[p] = hit_key(H, c0 + k + lane, sg);
+                si[p] = (unsigned)(k + lane);
+            }
+            have += __popc(b);
+        }
+        __syncwarp();
+        if (c <= 32) hit_sort_warp<1>(H, sk, si, (int)c, o, i, c0, lane);
+        else if (c <= 64) hit_sort_warp<2>(H, sk, si, (int)c, o, i, c0, lane);
+        else hit_sort_warp<4>(H, sk, si, (int)c, o, i, c0, lane);
+        __syncwarp();
+    }
+}
+
+constexpr int FIN_T = 256;
+constexpr int FIN_SMEM = 8 * WARP_SORT_MAX;  // hits a block sorts in shared memory
+
+// c (<= FIN_SMEM) pairs in (k[0], x[0]): sorted by warps in runs of 128, then
+// merged by ranks; returns the buffer (0 / 1) that holds the result.
+__device__ __forceinline__ int block_sort(unsigned long long (*k)[FIN_SMEM], unsigned (*x)[FIN_SMEM], int c) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int b0 = w * WARP_SORT_MAX;
+    if (b0 < c) {
+        unsigned long long kr[4];
+        unsigned xr[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int e = b0 + r * 32 + lane;
+            kr[r] = e < c ? k[0][e] : ~0ull;
+            xr[r] = e < c ? x[0][e] : ~0u;
+        }
+        warp_bitonic(kr, xr, lane);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int e = b0 + r * 32 + lane;
+            if (e < c) {
+                k[0][e] = kr[r];
+                x[0][e] = xr[r];
+            }
+        }
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int wd = WARP_SORT_MAX; wd < c; wd <<= 1) {
+        for (int t = threadIdx.x; t < c; t += FIN_T) {
+            const int run = t / wd, own = run * wd, plo = min((run ^ 1) * wd, c), phi = min(plo + wd, c);
+            const unsigned long long mk = k[cur][t];
+            const unsigned mx = x[cur][t];
+            int lo = plo, hi = phi;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (kless(k[cur][mid], x[cur][mid], mk, mx)) lo = mid + 1;
+                else hi = mid;
+            }
+            const int dst = (run & ~1) * wd + (t - own) + (lo - plo);
+            k[cur ^ 1][dst] = mk;
+            x[cur ^ 1][dst] = mx;
+        }
+        __syncthreads();
+        cur ^= 1;
+    }
+    return cur;
+}
+
+// Longer segments (listed), one block each: hits collected in any order (the
+// (key, candidate) pairs are unique), sorted in shared memory up to FIN_SMEM,
+// else in sorted runs of that many merged by ranks in global memory (gk / gx:
+// two buffers of `total` pairs).
+__global__ void __launch_bounds__(FIN_T) k_finish_block(HitSort H, const int* __restrict__ list,
+                                                        const unsigned long long* __restrict__ nlist, int64_t total,
+                                                        unsigned long long* __restrict__ gk,
+                                                        unsigned* __restrict__ gx) {
+    __shared__ unsigned long long k[2][FIN_SMEM];
+    __shared__ unsigned x[2][FIN_SMEM];
+    __shared__ unsigned long long fill;
+    const int lane = threadIdx.x & 31;
+    const int64_t nl = (int64_t)*nlist;
+    for (int64_t li = blockIdx.x; li < nl; li += gridDim.x) {
+        const int64_t s = list[li], i = H.order ? (int64_t)H.order[s] : s;
+        const int64_t c = H.counts[i], c0 = H.coff[s], m = H.ccnt[s], o = H.offsets[i];
+        const bool small = c <= FIN_SMEM;
+        const double4 sg = H.segs[s];
+        __syncthreads();
+        if (threadIdx.x == 0) fill = 0;
+        __syncthreads();
+        for (int64_t t0 = 0; t0 < m; t0 += FIN_T) {
+            const int64_t t = t0 + threadIdx.x;
+            const bool hit = t < m && H.keep[c0 + t];
+            const unsigned b = __ballot_sync(0xffffffffu, hit);
+            unsigned long long p = 0;
+            if (lane == 0 && b) p = atomicAdd(&fill, (unsigned long long)__popc(b));
+            p = __shfl_sync(0xffffffffu, p, 0) + __popc(b & ((1u << lane) - 1u));
+            if (hit) {
+                const unsigned long long key = hit_key(H, c0 + t, sg);
+                if (small) {
+                    k[0][p] = key;
+                    x[0][p] = (unsigned)t;
+                } else {
+                    gk[o + p] = key;
+                    gx[o + p] = (unsigned)t;
+                }
+            }
+        }
+        __syncthreads();
+        if (small) {
+            const int cur = block_sort(k, x, (int)c);
+            for (int t = threadIdx.x; t < c; t += FIN_T) hit_write(H, o + t, i, c0 + x[cur][t]);
+            continue;
+        }
+        for (int64_t r0 = 0; r0 < c; r0 += FIN_SMEM) {
+            const int rc = (int)min((int64_t)FIN_SMEM, c - r0);
+            for (int t = threadIdx.x; t < rc; t += FIN_T) {
+                k[0][t] = gk[o + r0 + t];
+                x[0][t] = gx[o + r0 + t];
+            }
+            __syncthreads();
+            const int cur = block_sort(k, x, rc);
+            for (int t = threadIdx.x; t < rc; t += FIN_T) {
+                gk[o + r0 + t] = k[cur][t];
+                gx[o + r0 + t] = x[cur][t];
+            }
+            __syncthreads();
+        }
+        unsigned long long *ka = gk + o, *kb = gk + total + o;
+        unsigned *xa = gx + o, *xb = gx + total + o;
+        for (int64_t wd = FIN_SMEM; wd < c; wd <<= 1) {
+            for (int64_t t = threadIdx.x; t < c; t += FIN_T) {
+                const int64_t run = t / wd, own = run * wd, plo = min((run ^ 1) * wd, c), phi = min(plo + wd, c);
+                const unsigned long long mk = ka[t];
+                const unsigned mx = xa[t];
+                int64_t lo = plo, hi = phi;
+                while (lo < hi) {
+                    const int64_t mid = (lo + hi) >> 1;
+                    if (kless(ka[mid], xa[mid], mk, mx)) lo = mid + 1;
+                    else hi = mid;
+                }
+                const int64_t dst = (run & ~(int64_t)1) * wd + (t - own) + (lo - plo);
+                kb[dst] = mk;
+                xb[dst] = mx;
+            }
+            __syncthreads();
+            unsigned long long* tk = ka;
+            ka = kb;
+            kb = tk;
+            unsigned* tx = xa;
+            xa = xb;
+            xb = tx;
+        }
+        for (int64_t t = threadIdx.x; t < c; t += FIN_T) hit_write(H, o + t, i, c0 + xa[t]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2059,6 +2309,29 @@ __global__ void k_work_keys(const double4* __restrict__ q, int64_t n, int kind, 
         int k = (w > 0.0f) ? (int)floorf(4.0f * log2f(w)) + 128 : 0;  // NaN -> 0
         key[i] = (unsigned)min(max(k, 0), 255);
     }
+}
+
+// 16-bit Morton key of a box's (kind 0) or segment's (kind 1) middle on a
+// 256 x 256 grid over the tree's bbox (outside and NaN: the nearest cell, 0).
+__global__ void k_spatial_keys(const double4* __restrict__ q, int64_t n, int kind, double x0, double y0, float sx,
+                               float sy, unsigned* __restrict__ key) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double4 v = q[i];
+        const float a = (float)(v.x - x0), c = (float)(v.z - (kind == 0 ? y0 : x0));
+        const float b = (float)(v.y - (kind == 0 ? x0 : y0)), d = (float)(v.w - y0);
+        const float mx = kind == 0 ? a + b : a + c, my = kind == 0 ? c + d : b + d;
+        unsigned k = 0;
+        const unsigned gx = (unsigned)fminf(fmaxf(0.5f * mx * sx, 0.0f), 255.0f);
+        const unsigned gy = (unsigned)fminf(fmaxf(0.5f * my * sy, 0.0f), 255.0f);
+        for (int b2 = 0; b2 < 8; b2++) k |= (((gx >> b2) & 1u) << (2 * b2)) | (((gy >> b2) & 1u) << (2 * b2 + 1));
+        key[i] = k;
+    }
+}
+
+__global__ void k_gather_rows(const double4* __restrict__ q, const int* __restrict__ order, int64_t n,
+                              double4* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = q[order[i]];
 }
 
 TreeQ make_q(const ct_tree* t) {
@@ -2836,9 +3109,11 @@ int ct_test_edge_candidates(const ct_tree* t, int32_t mode, const double* segs, 
     TreeQ T = make_q(t);
     unsigned g = (unsigned)std::min<int64_t>(grid_of(n_cand, 128), 152 * 64);
     if (mode == 0)
-        k_edge_test<0><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep, (double4*)xy);
+        k_edge_test<0, int64_t><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep,
+                                                   (double4*)xy);
     else
-        k_edge_test<1><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep, (double4*)xy);
+        k_edge_test<1, int64_t><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep,
+                                                   (double4*)xy);
     CT_CHECK_LAUNCH("test_edge_candidates");
     return CT_OK;
 }
@@ -2856,6 +3131,121 @@ int ct_compact_edge_hits(const ct_tree* t, const int64_t* keep, const int64_t* p
         k_edge_seg_counts<<<(unsigned)std::min<int64_t>(grid_of(n, 256), 152 * 32), 256, 0, st>>>(
             cand_off, cand_cnt, keep, pos, n_cand, n, offsets, counts);
     CT_CHECK_LAUNCH("compact_edge_hits");
+    return CT_OK;
+}
+
+size_t ct_spatial_order_workspace_size(int64_t n) {
+    size_t nn = (size_t)(n > 0 ? n : 1);
+    return 3 * ((4 * nn + 255) / 256 * 256) + ct_radix_pass_workspace_size();
+}
+
+int ct_spatial_order(const double* queries, int64_t n, int32_t kind, const double* bbox_host4, int32_t* order,
+                     void* ws, size_t ws_bytes, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (n < 0 || n > INT32_MAX || (kind != 0 && kind != 1) || !bbox_host4)
+        return ct_fail(CT_ERR_ARG, "bad spatial-order arguments");
+    if (!ws || ws_bytes < ct_spatial_order_workspace_size(n)) return ct_fail(CT_ERR_WORKSPACE, "workspace too small");
+    if (n == 0) return CT_OK;
+    const size_t part = (4 * (size_t)n + 255) / 256 * 256;
+    unsigned* kin = (unsigned*)ws;
+    unsigned* kout = (unsigned*)((char*)ws + part);
+    int* iout = (int*)((char*)ws + 2 * part);
+    void* rws = (char*)ws + 3 * part;
+    const double ex = bbox_host4[1] - bbox_host4[0], ey = bbox_host4[3] - bbox_host4[2];
+    const float sx = ex > 0.0 ? (float)(256.0 / ex) : 0.0f, sy = ey > 0.0 ? (float)(256.0 / ey) : 0.0f;
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 152 * 16);
+    k_spatial_keys<<<blocks, 256, 0, st>>>((const double4*)queries, n, kind, bbox_host4[0], bbox_host4[2], sx, sy,
+                                           kin);
+    CT_CHECK_LAUNCH("spatial keys");
+    int s = ct_radix_pass(kin, nullptr, n, 0, kout, iout, rws, ws_bytes - 3 * part, stream);
+    if (s) return s;
+    return ct_radix_pass(kout, iout, n, 8, kin, order, rws, ws_bytes - 3 * part, stream);
+}
+
+int ct_gather_rows(const double* queries, const int32_t* order, int64_t n, double* out, void* stream) {
+    if (n <= 0) return CT_OK;
+    k_gather_rows<<<(unsigned)std::min<int64_t>((n + 255) / 256, 152 * 16), 256, 0, (cudaStream_t)stream>>>(
+        (const double4*)queries, order, n, (double4*)out);
+    CT_CHECK_LAUNCH("gather rows");
+    return CT_OK;
+}
+
+int ct_test_edge_candidates_u8(const ct_tree* t, int32_t mode, const double* segs, const int32_t* cand_seg,
+                               const int32_t* cand_pos, int64_t n_cand, uint8_t* keep, double* xy, void* stream) {
+    int s = check_tree(t);
+    if (s) return s;
+    if (n_cand == 0) return CT_OK;
+    if (mode != 0 && mode != 1) return ct_fail(CT_ERR_ARG, "mode must be 0 or 1");
+    cudaStream_t st = (cudaStream_t)stream;
+    TreeQ T = make_q(t);
+    unsigned g = (unsigned)std::min<int64_t>(grid_of(n_cand, 128), 152 * 64);
+    if (mode == 0)
+        k_edge_test<0, uint8_t><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep,
+                                                   (double4*)xy);
+    else
+        k_edge_test<1, uint8_t><<<g, 128, 0, st>>>(T, (const double4*)segs, cand_seg, cand_pos, n_cand, keep,
+                                                   (double4*)xy);
+    CT_CHECK_LAUNCH("test_edge_candidates");
+    return CT_OK;
+}
+
+size_t ct_edge_hit_counts_workspace_size(int64_t n) { return ct_scan_workspace_size(n) + 256; }
+
+int ct_edge_hit_counts(const uint8_t* keep, const int64_t* cand_off, const int64_t* cand_cnt, const int32_t* order,
+                       int64_t n, int64_t* counts, int64_t* offsets, void* ws, size_t ws_bytes, int64_t* total_host,
+                       int64_t* longest_host, void* stream) {
+    if (n < 0) return ct_fail(CT_ERR_ARG, "negative length");
+    if (!ws || ws_bytes < ct_edge_hit_counts_workspace_size(n)) return ct_fail(CT_ERR_WORKSPACE, "workspace too small");
+    if (!total_host || !longest_host) return ct_fail(CT_ERR_ARG, "no host results");
+    cudaStream_t st = (cudaStream_t)stream;
+    // block sums, the total behind them, and the longest behind that: one copy
+    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+    int64_t* sums = (int64_t*)ws;
+    CT_CUDA(cudaMemsetAsync(sums + nb, 0, 2 * sizeof(int64_t), st));
+    if (n > 0) {
+        k_hit_counts<<<(unsigned)std::min<int64_t>(grid_of(n, 8), 152 * 16), 256, 0, st>>>(
+            keep, cand_off, cand_cnt, order, n, counts, (unsigned long long*)(sums + nb + 1));
+        k_scan_reduce<<<(unsigned)nb, SCAN_T, 0, st>>>(counts, n, sums);
+        k_scan_sums<<<1, SCAN_T, 0, st>>>(sums, nb);
+        k_scan_down<<<(unsigned)nb, SCAN_T, 0, st>>>(counts, n, sums, offsets);
+    }
+    CT_CHECK_LAUNCH("edge_hit_counts");
+    int64_t got[2] = {0, 0};
+    CT_CUDA(cudaMemcpyAsync(got, sums + nb, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    CT_CUDA(cudaStreamSynchronize(st));
+    *total_host = got[0];
+    *longest_host = got[1];
+    return CT_OK;
+}
+
+size_t ct_finish_edge_hits_workspace_size(int64_t total, int64_t longest) {
+    const size_t t = (size_t)(total > 0 ? total : 1);
+    const size_t lists = ((t / (WARP_SORT_MAX + 1) + 2) * sizeof(int) + 256 + 255) / 256 * 256;
+    return lists + (longest > FIN_SMEM ? t * 2 * (sizeof(unsigned long long) + sizeof(unsigned)) + 256 : 0);
+}
+
+int ct_finish_edge_hits(const ct_tree* t, const double* segs, const int32_t* order, const uint8_t* keep,
+                        const int32_t* cand_pos, const double* xy_cand, const int64_t* cand_off,
+                        const int64_t* cand_cnt, int64_t n, const int64_t* counts, const int64_t* offsets,
+                        int64_t total, int64_t longest, int64_t* ii, int64_t* jj, double* xy, void* ws,
+                        size_t ws_bytes, void* stream) {
+    if (!t) return ct_fail(CT_ERR_ARG, "tree is null");
+    if (n < 0 || n > INT32_MAX) return ct_fail(CT_ERR_ARG, "at most 2^31 - 1 segments");
+    if (total == 0 || n == 0) return CT_OK;
+    if (!ws || ws_bytes < ct_finish_edge_hits_workspace_size(total, longest))
+        return ct_fail(CT_ERR_WORKSPACE, "finish workspace too small");
+    cudaStream_t st = (cudaStream_t)stream;
+    unsigned long long* nlist = (unsigned long long*)ws;
+    int* list = (int*)(nlist + 1);
+    const size_t lists = (((size_t)total / (WARP_SORT_MAX + 1) + 2) * sizeof(int) + 256 + 255) / 256 * 256;
+    unsigned long long* gk = (unsigned long long*)((char*)ws + lists);
+    unsigned* gx = (unsigned*)(gk + 2 * total);
+    const HitSort H{(const double4*)segs, order, keep, cand_pos, t->bb_indices, (const double4*)xy_cand, cand_off,
+                    cand_cnt, counts, offsets, ii, jj, (double4*)xy};
+    CT_CUDA(cudaMemsetAsync(nlist, 0, sizeof(unsigned long long), st));
+    k_finish_warp<<<(unsigned)std::min<int64_t>(grid_of(n, 8), 152 * 32), 256, 0, st>>>(H, n, list, nlist);
+    if (longest > WARP_SORT_MAX) k_finish_block<<<152 * 8, FIN_T, 0, st>>>(H, list, nlist, total, gk, gx);
+    CT_CHECK_LAUNCH("finish_edge_hits");
     return CT_OK;
 }
 
