@@ -1210,6 +1210,54 @@ __device__ __forceinline__ int edge_face_fast(const TreeQ& T, dpt a, dpt b, int 
     return X.x > x0 + mg && X.x < x1 - mg && X.y > y0 + mg && X.y < y1 - mg ? 1 : -1;
 }
 
+__device__ __noinline__ bool edge_edge_general(dpt a, dpt b, dpt p, dpt q, dpt* c) {
+    return lines_intersect(a, b, p, q, &c->x, &c->y);
+}
+
+// lines_intersect (geometry_utils.py:318-418) of a -> b and p -> q when its
+// decisions are certain in float32: 1 a crossing at c, 0 none, -1 unsure.
+// With U = q - p, V = b - a, D = a - p (float64 differences truncated to
+// float, 2 u of each) the four left_of tests are the signs of U x D,
+// U x (D + V), V x D and V x (U - D) (upstream's rounded products are off by
+// 2^-53 of theirs).  If both pairs differ the segments cross properly, so
+// upstream's overlap tests hold; it then only asks whether they are parallel
+// within its tolerance.  Otherwise it returns false unless p and q both lie
+// within the tolerance of a -> b's line.  The crossing itself is computed as
+// upstream does, products and quotient on the integer pipes.  The float64
+// unit bounded the plain form (60 instructions of 20 cycles per warp): 2.5M
+// candidates of 100k cross-sections of a network 272 -> 95 us.
+__device__ __forceinline__ int edge_edge_fast(dpt a, dpt b, dpt p, dpt q, dpt* c) {
+    const float u24 = 5.9604644775390625e-08f;
+    const dpt U = vsub(q, p), V = vsub(b, a), D = vsub(a, p);
+    const float2 u = make_float2(cl_float(U.x), cl_float(U.y)), v = make_float2(cl_float(V.x), cl_float(V.y));
+    const float2 d = make_float2(cl_float(D.x), cl_float(D.y));
+    const float mu = fabsf(u.x) + fabsf(u.y), mv = fabsf(v.x) + fabsf(v.y), md = fabsf(d.x) + fabsf(d.y);
+    if (!(mu < 1e15f && mv < 1e15f && md < 1e15f)) return -1;
+    const float2 e = make_float2(d.x + v.x, d.y + v.y), g = make_float2(u.x - d.x, u.y - d.y);
+    const float c1 = __fmaf_rn(u.x, d.y, -(u.y * d.x)), c2 = __fmaf_rn(u.x, e.y, -(u.y * e.x));
+    const float c3 = __fmaf_rn(v.x, d.y, -(v.y * d.x)), c4 = __fmaf_rn(v.x, g.y, -(v.y * g.x));
+    const float den = __fmaf_rn(v.x, u.y, -(v.y * u.x));
+    const float tu = 12.0f * u24 * mu + 2.4e-38f, tv = 12.0f * u24 * mv + 2.4e-38f, f = 1e-36f;
+    // tolerance 1e-12 of U's larger component, at least 1e-15; times |V|
+    const float tol = 1.02f * fmaxf(1e-15f, 1e-12f * (fmaxf(fabsf(u.x), fabsf(u.y)) + 2.4e-38f)) * (mv + 2.4e-38f);
+    const bool s12 = fabsf(c1) > tu * md + f * mu + f && fabsf(c2) > tu * (md + mv) + f * mu + f;
+    const bool s34 = fabsf(c3) > tv * md + tol + f * mv + f && fabsf(c4) > tv * (mu + md) + tol + f * mv + f;
+    // the pair known to lie on one side settles a miss, if p or q is clear of
+    // the tolerance as well
+    const bool clear = fabsf(c3) > tv * md + tol + f * mv + f || fabsf(c4) > tv * (mu + md) + tol + f * mv + f;
+    if (clear && s12 && (c1 > 0.0f) == (c2 > 0.0f)) return 0;
+    if (s34 && (c3 < 0.0f) == (c4 > 0.0f)) return 0;
+    if (!(s12 && s34) || !(fabsf(den) > tv * mu + tol + f * mv + f)) return -1;
+    bool bad = false;
+    const dpt R = mkp(sf_value(sf_bits(D.x) ^ 0x8000000000000000ull), sf_value(sf_bits(D.y) ^ 0x8000000000000000ull));
+    const double denom = sf_mul(V.x, U.y, &bad) - sf_mul(V.y, U.x, &bad);
+    const double t = sf_div(sf_mul(R.x, U.y, &bad) - sf_mul(R.y, U.x, &bad), denom, &bad);
+    const double x = sf_mul(t, V.x, &bad), y = sf_mul(t, V.y, &bad);
+    if (bad) return -1;
+    *c = mkp(a.x + x, a.y + y);
+    return 1;
+}
+
 // The cell test of every candidate (compute_edge_face_intersect
 // query.py:309-328 / compute_edge_edge_intersect 292-306).
 template <int MODE, typename KeepT>
@@ -1224,9 +1272,10 @@ __global__ void __launch_bounds__(128) k_edge_test(TreeQ T, const double4* __res
         bool hit;
         if (MODE == 0) {
             double2 p0 = T.poly[(size_t)j * 2], p1 = T.poly[(size_t)j * 2 + 1];
-            double x, y;
-            hit = lines_intersect(a, b, mkp(p0.x, p0.y), mkp(p1.x, p1.y), &x, &y);
-            c = mkp(x, y);
+            const dpt p = mkp(p0.x, p0.y), q = mkp(p1.x, p1.y);
+            c = mkp(dnan(), dnan());
+            const int r = edge_edge_fast(a, b, p, q, &c);
+            hit = r < 0 ? edge_edge_general(a, b, p, q, &c) : r == 1;
             d = c;
         } else {
             int r = -1;
