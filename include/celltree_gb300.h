@@ -498,6 +498,10 @@ int ct_write_boxes_ws(const ct_tree* tree, const double* boxes, int64_t n, const
  * ct_count_boxes + ct_write_boxes. */
 int ct_count_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
                         int32_t* spec, int32_t spec_cap, void* stream);
+/* The same counts and scratch by one thread per box: faster for boxes of about
+ * a cell that come in mesh order (query faces). */
+int ct_count_small_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
+                              int64_t* counts, int32_t* spec, int32_t spec_cap, void* stream);
 int ct_write_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
                         const int64_t* counts, const int64_t* offsets, const int32_t* spec, int32_t spec_cap,
                         int64_t total_pairs, int32_t min_job_cells, int64_t* ii, int64_t* jj, void* workspace,

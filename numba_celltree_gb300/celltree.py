@@ -365,7 +365,9 @@ class CellTree2d(CellTree2dBase):
         _lib.check(lib.ct_counter_clockwise(_device.ptr(v_d), _device.ptr(f_d), n, K, st), "counter_clockwise")
         bb = _device.empty((n, 4), torch.float64, t.device)
         _lib.check(lib.ct_face_bboxes(_device.ptr(v_d), _device.ptr(f_d), n, K, _device.ptr(bb), st), "face_bboxes")
-        si, sj = t.locate_boxes(bb)
+        # as many faces as a quarter of the tree's cells and enough threads:
+        # the boxes are a few cells each
+        si, sj = t.locate_boxes(bb, small=n >= t.WORK_ORDER_MIN and 4 * n >= t.n)
         m = int(si.shape[0])
         flag = _device.empty((m,), torch.uint8, t.device)
         _lib.check(

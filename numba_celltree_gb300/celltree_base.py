@@ -419,26 +419,9 @@ class _GpuTree:
         )
         return offsets, int(total.value)
 
-    # queries per batch from which box / segment queries run in work order
-    # (below it the ordering's fixed cost outweighs the better warp balance)
+    # queries per batch from which box / segment queries may run in spatial
+    # order (below it the ordering's fixed cost outweighs what it saves)
     WORK_ORDER_MIN = 65536
-
-    def work_order(self, q_d, kind: int, force=None):
-        """Permutation grouping box (kind 0) / segment (kind 1) queries of
-        similar size, or None for small batches (`force` True / False
-        overrides the size rule)."""
-        n = int(q_d.shape[0])
-        if force is False or (force is None and n < self.WORK_ORDER_MIN):
-            return None
-        torch = _device.torch()
-        lib = _lib.load()
-        nbytes = int(lib.ct_work_order_workspace_size(n))
-        ws = _device.empty((nbytes,), torch.uint8, self.device)
-        order = _device.empty((n,), torch.int32, self.device)
-        cell = max(self.max_diagonal, 1e-300)
-        _lib.check(lib.ct_work_order(_device.ptr(q_d), n, kind, cell, _device.ptr(order), _device.ptr(ws), nbytes,
-                                     _device.stream()), "work order")
-        return order
 
     def ensure_box_index(self):
         """Build the box index of the multi-result queries on first use (cell
@@ -606,15 +589,15 @@ class _GpuTree:
     SPEC_CAP_LARGE = 16
     SPEC_MAX_BYTES = 1 << 30
 
-    def locate_boxes(self, boxes_d, config=None, budget=None):
+    def locate_boxes(self, boxes_d, config=None, budget=None, small=False):
         """Pairs (box, cell) of every box query, box-major in upstream order;
         with `budget`, returns None instead when the pairs would exceed it
-        (the per-box counts are left in self.last_counts)."""
+        (the per-box counts are left in self.last_counts).  `small`: the boxes
+        are about a cell each and come in mesh order (counted by a thread
+        each)."""
         n = int(boxes_d.shape[0])
         if config is None:
-            m = min(n, autotune.SAMPLE_MAX["boxes"])
-            step = max(1, n // max(m, 1))
-            config = self.maybe_tune("boxes", n, lambda c: self.locate_boxes(boxes_d[::step][:m].contiguous(), c), m)
+            config = self.cached("boxes", n)
         torch = _device.torch()
         lib = _lib.load()
         st = _device.stream()
@@ -622,14 +605,17 @@ class _GpuTree:
         self.reset_error()
         self.ensure_box_index()
         self._apply("boxes", config)
-        order = self.work_order(boxes_d, 0, config.get("work_order"))
+        order = None
+        if not small and self.in_spatial_order(n, config):
+            order = self.spatial_order(boxes_d, 0)[0]
         spec = None
         cap = self.SPEC_CAP if n <= self.SPEC_MAX_BOXES else self.SPEC_CAP_LARGE
         if self.SPEC_MAX_BOXES > 0 and 0 < n and n * cap * 4 <= self.SPEC_MAX_BYTES:
             # one traversal: the counting pass also keeps each box's first pairs
             spec = _device.empty((n, cap), torch.int32, self.device)
-            _lib.check(lib.ct_count_boxes_spec(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
-                                               _device.ptr(counts), _device.ptr(spec), cap, st),
+            count = lib.ct_count_small_boxes_spec if small else lib.ct_count_boxes_spec
+            _lib.check(count(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
+                             _device.ptr(counts), _device.ptr(spec), cap, st),
                        "locate_boxes")
         else:
             _lib.check(lib.ct_count_boxes(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
@@ -673,6 +659,17 @@ class _GpuTree:
         )
         return ii, jj
 
+    # cells from which a tree's node and cell records (about 130 bytes a cell)
+    # outgrow the 129 MB of L2, so that the order of the queries matters: 1M
+    # segments on 5M cells 15.6 -> 9.9 ms with the spatial order, 100k on a
+    # network of 501k edges 0.60 -> 0.56 ms without it
+    ORDER_MIN_CELLS = 1 << 20
+
+    def in_spatial_order(self, n: int, config: dict) -> bool:
+        """Whether a batch of n boxes / segments runs in spatial order."""
+        return n > 0 and (bool(config.get("work_order")) or
+                          (n >= self.WORK_ORDER_MIN and self.n >= self.ORDER_MIN_CELLS))
+
     def spatial_order(self, q_d, kind: int):
         """Permutation of box (kind 0) / segment (kind 1) queries by a 256 x
         256 Morton grid over the tree, and the queries in that order."""
@@ -696,10 +693,10 @@ class _GpuTree:
         With `budget`, returns None instead when the candidates would exceed
         it (the per-segment candidate counts are left in self.last_counts).
 
-        Batches of WORK_ORDER_MIN segments run in spatial order (results stay
-        in segment order): the traversal and the cell test read nodes and
-        cells that the segments before have brought into L2.  1M short
-        segments on 5M cells read 19 KB of DRAM each in their own order."""
+        Large batches run in spatial order (results stay in segment order):
+        the traversal and the cell test read nodes and cells that the segments
+        before have brought into L2.  1M short segments on 5M cells read 19 KB
+        of DRAM each in their own order."""
         n = int(segs_d.shape[0])
         if config is None:
             config = self.cached("segments", n)
@@ -710,7 +707,7 @@ class _GpuTree:
         self.ensure_box_index()
         self._apply("segments", config)
         order = None
-        if n >= self.WORK_ORDER_MIN or (n > 0 and config.get("work_order")):
+        if self.in_spatial_order(n, config):
             order, segs_d = self.spatial_order(segs_d, 1)
         P = _device.ptr
         coff, ccnt, nc, items = self.edge_candidate_ranges(segs_d, mode, None, self.edge_cut(config, n), keep=True)

@@ -103,6 +103,10 @@ struct BoxJob {
 };
 constexpr int BOX_JOB_MIN = 8;  // default: smaller subtrees are written in line
 
+// One thread per box: boxes of about a cell each that come in mesh order (the
+// query faces of locate_faces), whose neighbouring lanes take the same path --
+// 1M faces on 500k cells 0.38 ms, by warps (below) 0.6 ms -- and, with DEEP,
+// trees deeper than the warps' walk takes.
 template <bool WRITE, bool DEEP>
 __global__ void __launch_bounds__(256) k_boxes(TreeQ T, const double4* __restrict__ boxes, int64_t n,
                                                const int* __restrict__ order, int64_t* __restrict__ cnt_or_off,
@@ -290,6 +294,218 @@ __global__ void __launch_bounds__(256) k_boxes(TreeQ T, const double4* __restric
         }
     }
     if (!WRITE) cnt_or_off[i] = count;
+}
+
+// ---------------------------------------------------------------------------
+// Box queries by warps (ct_walk.cuh): counts, with `spec` the first spec_cap
+// cells of every box (in output order) as well, or with WRITE the pairs at
+// the boxes' offsets.  The tests of a node and of a cell are those of
+// k_boxes, whose comments give the reasons.  A terminal node is a leaf
+// or a subtree wholly inside the box; the outputs of 32 of them are numbered
+// through and shared out over the lanes, so pairs are written coalesced
+// however they are spread over nodes.
+//
+// A thread per box was bound by its chain of node loads and by the largest
+// box of its warp (9 of 32 lanes active).  250k boxes of 0.1 to 50 m on 5M
+// cells: counting 4.6 -> 2.6 ms, writing 6.8 -> 4.6 ms; 10k small boxes on 80k
+// cells 117 -> 37 us.
+// ---------------------------------------------------------------------------
+struct WalkBox {  // 88 bytes: an odd number of 8-byte words, so lanes of different queries hit different banks
+    unsigned long long kx0, kx1, ky0, ky1;
+    float qx0, qx1, qy0, qy1;  // the box in the float32 frame, rounded inward
+    float ox0, ox1, oy0, oy1;  // and outward
+    int64_t base;
+    int id;
+    bool keys, idx;
+    int64_t pad;
+};
+
+template <bool WRITE>
+struct BoxWalk {
+    const TreeQ& T;
+    const double4* boxes;
+    const WalkBox* Q;
+    int64_t* emitted;
+    int lane;
+    int64_t *ii, *jj;
+    int* spec;
+    int spcap;
+
+    __device__ __forceinline__ int visit(int v, int qi, int, int* first, int* second) const {
+        const WalkBox& S = Q[qi];
+        const float4 q = T.nf[v];
+        const double2 d = T.nd[v];
+        if (S.idx) {
+            const float4 b = *reinterpret_cast<const float4*>(T.nbx + v);  // xmin, xmax, ymin, ymax
+            if (b.y < S.ox0 || b.x > S.ox1 || b.w < S.oy0 || b.z > S.oy1) return WALK_DROP;
+            if (S.qx0 < b.x && b.y < S.qx1 && S.qy0 < b.z && b.w < S.qy1) return WALK_ALL;
+        }
+        if (nb(q) >= 0) return WALK_LEAF;
+        const int dim = -1 - nb(q);
+        bool left, right;
+        if (S.keys) {
+            left = (dim ? S.ky0 : S.kx0) <= fkey(d.x);
+            right = (dim ? S.ky1 : S.kx1) >= fkey(d.y);
+        } else {
+            const double4 b = boxes[S.id];
+            left = (dim ? b.z : b.x) <= d.x;
+            right = (dim ? b.w : b.y) >= d.y;
+        }
+        // the right child is visited first
+        const int child = na(q);
+        *first = right ? child + 1 : (left ? child : -1);
+        *second = (left && right) ? child : -1;
+        return *first >= 0 ? WALK_OPEN : WALK_DROP;
+    }
+
+    // boxes_intersect geometry_utils.py:292-300
+    __device__ __forceinline__ bool overlaps(const WalkBox& S, int j) const {
+        const dbox b = leaf_box(T, j);
+        return S.keys ? (S.kx0 < fkey(b.xmax) && fkey(b.xmin) < S.kx1 && S.ky0 < fkey(b.ymax) && fkey(b.ymin) < S.ky1)
+                      : boxes_intersect(load_box(reinterpret_cast<const double*>(boxes + S.id)), b);
+    }
+
+    __device__ __forceinline__ void put(int64_t at, int64_t id, int64_t rank, int j) const {
+        if (WRITE) {
+            ii[at + rank] = id;
+            jj[at + rank] = T.bbi[j];
+        } else if (rank < spcap) {
+            spec[at + rank] = (int)T.bbi[j];
+        }
+    }
+
+    __device__ __forceinline__ void emit(int v, unsigned meta, bool have) const {
+        const unsigned FULL = 0xffffffffu;
+        const int qi = have ? (int)(meta & WALK_QMASK) : -1;
+        const WalkBox& S = Q[have ? qi : 0];
+        const bool all = have && (meta & WALK_WHOLE) != 0;
+        int ptr = 0, size = 0;
+        unsigned hit = 0;  // the overlapping ones of a leaf's first 32 cells
+        int64_t c = 0;
+        if (all) {
+            const int4 r = reinterpret_cast<const int4*>(T.nbx + v)[1];
+            ptr = r.x;
+            size = r.y;
+            c = size;
+        } else if (have) {
+            const float4 q = T.nf[v];
+            ptr = na(q);
+            size = nb(q);
+            for (int k = 0; k < size; k++)
+                if (overlaps(S, ptr + k)) {
+                    if (k < 32) hit |= 1u << k;
+                    c++;
+                }
+        }
+        const int64_t rank = walk_rank<int64_t>(qi, c, have, lane, emitted);
+        if (!WRITE && !spec) return;
+        const int64_t at = have ? S.base : 0;
+        const int id = have ? S.id : 0;
+        int64_t share = WRITE ? c : min(c, max((int64_t)0, (int64_t)spcap - rank));
+        if (!all && size > 32) {  // a large leaf: its own lane
+            int64_t r = rank;
+            for (int k = 0; k < size && share > 0; k++)
+                if (overlaps(S, ptr + k)) put(at, id, r++, ptr + k);
+            share = 0;
+        }
+        int64_t incl = share;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int64_t excl = incl - share, total = __shfl_sync(FULL, incl, 31);
+        for (int64_t t0 = 0; t0 < total; t0 += 32) {
+            const int64_t t = t0 + lane;
+            int k = 0;  // the node of output t: the last one that starts at or before it
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(FULL, excl, k + o) <= t) k += o;
+            const int64_t o = t - __shfl_sync(FULL, excl, k);
+            const int kp = __shfl_sync(FULL, ptr, k), ks = __shfl_sync(FULL, size, k);
+            unsigned kh = __shfl_sync(FULL, hit, k);
+            const int64_t kr = __shfl_sync(FULL, rank, k), ka = __shfl_sync(FULL, at, k);
+            const int ki = __shfl_sync(FULL, id, k);
+            const bool kall = __shfl_sync(FULL, (int)all, k) != 0;
+            if (t >= total) continue;
+            int j;
+            if (kall) {
+                // output o of a whole subtree, leaves by decreasing
+                // position, each leaf's cells by increasing position
+                const int end = kp + ks, q = end - 1 - (int)o;
+                const int s0 = T.lstart[q];
+                if (s0 < kp || s0 > q) {  // corrupt index: leave the slot, report
+                    set_error(T.err, CT_DEVERR_LOOP);
+                    continue;
+                }
+                int e = q + 1;
+                while (e < end && T.lstart[e] == s0) e++;
+                j = s0 + (e - 1 - q);
+            } else {
+                for (int z = (int)o; z > 0; z--) kh &= kh - 1u;
+                j = kp + __ffs(kh) - 1;
+            }
+            put(ka, ki, kr + o, j);
+        }
+    }
+};
+
+template <bool WRITE>
+__global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const double4* __restrict__ boxes, int64_t n,
+                                                              const int* __restrict__ order, int per_warp,
+                                                              int64_t* __restrict__ cnt_or_off,
+                                                              int64_t* __restrict__ ii, int64_t* __restrict__ jj,
+                                                              int* __restrict__ spec, int spcap,
+                                                              const int64_t* __restrict__ spec_cnt) {
+    __shared__ WalkBuf bufs[WALK_WARPS];
+    __shared__ WalkBox qs[WALK_WARPS][WALK_Q];
+    __shared__ int64_t counts[WALK_WARPS][WALK_Q];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    const int64_t t0 = ((int64_t)blockIdx.x * WALK_WARPS + wi) * per_warp;
+    if (t0 >= n) return;
+    const bool valid = lane < per_warp && t0 + lane < n;
+    int64_t i = 0;
+    bool start = false;
+    if (valid) {
+        i = order ? (int64_t)order[t0 + lane] : t0 + lane;
+        // writing after a count with scratch: boxes whose pairs all fit it
+        // were written from it (k_boxes_spec_emit)
+        if (!(WRITE && spec_cnt && spec_cnt[i] <= spcap)) {
+            const double4 q4 = boxes[i];
+            dbox b;
+            b.xmin = q4.x;
+            b.xmax = q4.y;
+            b.ymin = q4.z;
+            b.ymax = q4.w;
+            start = boxes_intersect(b, T.bbox);
+            if (start) {
+                WalkBox& S = qs[wi][lane];
+                S.keys = T.finite && not_nan(b.xmin) && not_nan(b.xmax) && not_nan(b.ymin) && not_nan(b.ymax);
+                S.kx0 = fkey(b.xmin);
+                S.kx1 = fkey(b.xmax);
+                S.ky0 = fkey(b.ymin);
+                S.ky1 = fkey(b.ymax);
+                S.idx = S.keys && T.nbx != nullptr;
+                const double x0 = b.xmin - T.ox, x1 = b.xmax - T.ox, y0 = b.ymin - T.oy, y1 = b.ymax - T.oy;
+                S.qx0 = __double2float_ru(x0);
+                S.qx1 = __double2float_rd(x1);
+                S.qy0 = __double2float_ru(y0);
+                S.qy1 = __double2float_rd(y1);
+                S.ox0 = __double2float_rd(x0);
+                S.ox1 = __double2float_ru(x1);
+                S.oy0 = __double2float_rd(y0);
+                S.oy1 = __double2float_ru(y1);
+                S.id = (int)i;
+                S.base = WRITE ? cnt_or_off[i] : i * (int64_t)spcap;
+            }
+        }
+    }
+    if (lane < WALK_Q) counts[wi][lane] = 0;
+    const int nq = walk_begin(bufs[wi], start ? 0 : -1, lane);
+    BoxWalk<WRITE> pol{T, boxes, qs[wi], counts[wi], lane, ii, jj, spec, spcap};
+    walk(pol, bufs[wi], nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
+    __syncwarp();
+    if (!WRITE && valid) cnt_or_off[i] = counts[wi][lane];
 }
 
 // The cells of each deferred subtree, one warp per subtree, in upstream's
@@ -542,24 +758,25 @@ __device__ __forceinline__ EdgeKeys edge_keys(const TreeQ& T, dpt a, dpt b) {
 // are the traversal's.  Counts per task, or with WRITE the candidates (nodes)
 // at their offsets.
 //
-// Bound by reading the nodes (90 B each) in no order; 8 tasks per warp fill
-// the rounds of short segments, fewer when there are few tasks.  The two cut
+// Bound by reading the nodes (90 B each) where the segments come in no order;
+// 8 tasks per warp fill the rounds of short segments.  The two cut
 // passes and the two item passes of 1000 segments across a mesh of 5M cells:
 // 1.73 -> 0.72 ms; 1M short segments uncut: 7.0 ms as with one thread per
 // segment.
 // ---------------------------------------------------------------------------
-struct WalkSeg {
-    double ax, ay, bx, by;
+struct WalkSeg {  // 88 bytes, as WalkBox
     unsigned long long kax, kay, kbx, kby;
     LineF lf;
-    int64_t base;
     int seg;
+    int64_t base;
     bool keys, posx, posy;
+    int64_t pad;
 };
 
 template <int MODE, bool ITEMS, bool WRITE>
 struct SegWalk {
     const TreeQ& T;
+    const double4* segs;
     const WalkSeg* Q;
     int* emitted;
     int lane, cut;
@@ -585,7 +802,8 @@ struct SegWalk {
             *first = right ? child + 1 : (left ? child : -1);
             *second = (left && right) ? child : -1;
         } else {
-            const dpt a = mkp(S.ax, S.ay), b = mkp(S.bx, S.by);
+            const double4 s4 = segs[S.seg];
+            const dpt a = mkp(s4.x, s4.y), b = mkp(s4.z, s4.w);
             edge_children(T, nd, q, a, b, vsub(b, a), false, 0, 0, 0, 0, first, second);
         }
         return *first >= 0 ? WALK_OPEN : WALK_DROP;
@@ -604,7 +822,8 @@ struct SegWalk {
             const unsigned long long x0 = fkey(bx.xmin), x1 = fkey(bx.xmax), y0 = fkey(bx.ymin), y1 = fkey(bx.ymax);
             return (cs_code_keys(S.kax, S.kay, x0, x1, y0, y1) & cs_code_keys(S.kbx, S.kby, x0, x1, y0, y1)) == 0;
         }
-        return (cs_code(mkp(S.ax, S.ay), bx) & cs_code(mkp(S.bx, S.by), bx)) == 0;
+        const double4 s4 = segs[S.seg];
+        return (cs_code(mkp(s4.x, s4.y), bx) & cs_code(mkp(s4.z, s4.w), bx)) == 0;
     }
 
     __device__ __forceinline__ void put(const WalkSeg& S, int rank, int val) const {
@@ -616,34 +835,31 @@ struct SegWalk {
         }
     }
 
-    __device__ __forceinline__ void emit(const int* node, const unsigned short* meta, int m) const {
-        for (int base = 0; base < m; base += 32) {
-            const bool have = base + lane < m;
-            const int v = have ? node[base + lane] : -1, qi = have ? (int)(meta[base + lane] & WALK_QMASK) : -1;
-            const WalkSeg& S = Q[have ? qi : 0];
-            int ptr = 0, size = 0, c = have ? 1 : 0;
-            unsigned hit = 0;  // the first 32 cells of the leaf
-            if (!ITEMS) {
-                c = 0;
-                if (have) {
-                    const float4 q = T.nf[v];
-                    ptr = na(q);
-                    size = nb(q);
+    __device__ __forceinline__ void emit(int v, unsigned meta, bool have) const {
+        const int qi = have ? (int)(meta & WALK_QMASK) : -1;
+        const WalkSeg& S = Q[have ? qi : 0];
+        int ptr = 0, size = 0, c = have ? 1 : 0;
+        unsigned hit = 0;  // the first 32 cells of the leaf
+        if (!ITEMS) {
+            c = 0;
+            if (have) {
+                const float4 q = T.nf[v];
+                ptr = na(q);
+                size = nb(q);
+            }
+            for (int k = 0; k < size; k++)
+                if (candidate(S, ptr + k)) {
+                    if (k < 32) hit |= 1u << k;
+                    c++;
                 }
-                for (int k = 0; k < size; k++)
-                    if (candidate(S, ptr + k)) {
-                        if (k < 32) hit |= 1u << k;
-                        c++;
-                    }
-            }
-            int r = walk_rank(qi, c, have, lane, emitted);
-            if (ITEMS) {
-                if (have) put(S, r, v);
-            } else if (c > 0 && (WRITE || spcap > 0)) {
-                for (unsigned h = hit; h; h &= h - 1u) put(S, r++, ptr + __ffs(h) - 1);
-                for (int k = 32; k < size; k++)
-                    if (candidate(S, ptr + k)) put(S, r++, ptr + k);
-            }
+        }
+        int r = walk_rank<int>(qi, c, have, lane, emitted);
+        if (ITEMS) {
+            if (have) put(S, r, v);
+        } else if (c > 0 && (WRITE || spcap > 0)) {
+            for (unsigned h = hit; h; h &= h - 1u) put(S, r++, ptr + __ffs(h) - 1);
+            for (int k = 32; k < size; k++)
+                if (candidate(S, ptr + k)) put(S, r++, ptr + k);
         }
     }
 };
@@ -683,10 +899,6 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_edge_walk(
                 const dpt V = vsub(b, a);
                 const EdgeKeys K = edge_keys(T, a, b);
                 WalkSeg& S = qs[wi][lane];
-                S.ax = a.x;
-                S.ay = a.y;
-                S.bx = b.x;
-                S.by = b.y;
                 S.kax = K.kax;
                 S.kay = K.kay;
                 S.kbx = K.kbx;
@@ -701,16 +913,9 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_edge_walk(
         }
     }
     if (lane < WALK_Q) counts[wi][lane] = 0;
-    WalkBuf& B = bufs[wi];
-    const unsigned b = __ballot_sync(0xffffffffu, start >= 0);
-    if (start >= 0) {
-        const int p = __popc(b & ((1u << lane) - 1u));
-        B.node[0][p] = start;
-        B.meta[0][p] = (unsigned short)lane;
-    }
-    __syncwarp();
-    SegWalk<MODE, ITEMS, WRITE> pol{T, qs[wi], counts[wi], lane, cut, out_seg, out_val, spcap};
-    walk(pol, B, __popc(b), lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
+    const int nq = walk_begin(bufs[wi], start, lane);
+    SegWalk<MODE, ITEMS, WRITE> pol{T, segs, qs[wi], counts[wi], lane, cut, out_seg, out_val, spcap};
+    walk(pol, bufs[wi], nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
     __syncwarp();
     if (!WRITE && valid) cnt_or_off[row] = counts[wi][lane];
 }
@@ -2523,12 +2728,26 @@ using namespace ctm;
 
 // Tasks per warp: one while they do not fill the resident warps (152 SMs x
 // 32), up to 8 beyond, so that a round's 32 lanes find nodes at every level.
+static int walk_tasks(int64_t n) {
+    int per_warp = 1;
+    while (per_warp < WALK_Q && n / (2 * per_warp) >= 152 * 32) per_warp *= 2;
+    return per_warp;
+}
+
+template <bool WRITE>
+static void launch_box_walk(const TreeQ& T, const double4* boxes, int64_t n, const int* order, int64_t* cnt_or_off,
+                            int64_t* ii, int64_t* jj, int* spec, int spcap, const int64_t* spec_cnt,
+                            cudaStream_t st) {
+    const int per_warp = walk_tasks(n);
+    k_box_walk<WRITE><<<grid_of((n + per_warp - 1) / per_warp, WALK_WARPS), 32 * WALK_WARPS, 0, st>>>(
+        T, boxes, n, order, per_warp, cnt_or_off, ii, jj, spec, spcap, spec_cnt);
+}
+
 template <bool ITEMS, bool WRITE>
 static void launch_edge_walk(int mode, const TreeQ& T, const double4* segs, int64_t n, const int* order,
                              const int* item_seg, const int* item_node, int cut, int64_t* cnt_or_off, int* out_seg,
                              int* out_val, int spcap, const int64_t* spec_cnt, cudaStream_t st) {
-    int per_warp = 1;
-    while (per_warp < WALK_Q && n / (2 * per_warp) >= 152 * 32) per_warp *= 2;
+    const int per_warp = walk_tasks(n);
     const unsigned g = grid_of((n + per_warp - 1) / per_warp, WALK_WARPS);
     if (mode == 0)
         k_edge_walk<0, ITEMS, WRITE><<<g, 32 * WALK_WARPS, 0, st>>>(T, segs, n, order, item_seg, item_node, cut,
@@ -2658,10 +2877,10 @@ int ct_count_boxes(const ct_tree* t, const double* boxes, int64_t n, const int32
     const int bt = box_threads(t);
     if (deep_tree(t))
         k_boxes<false, true><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(make_q(t), (const double4*)boxes, n,
-                                                                              order, counts, nullptr, nullptr);
+                                                                             order, counts, nullptr, nullptr);
     else
-        k_boxes<false, false><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(make_q(t), (const double4*)boxes, n,
-                                                                               order, counts, nullptr, nullptr);
+        launch_box_walk<false>(make_q(t), (const double4*)boxes, n, order, counts, nullptr, nullptr, nullptr, 0,
+                               nullptr, (cudaStream_t)stream);
     CT_CHECK_LAUNCH("count_boxes");
     return CT_OK;
 }
@@ -2674,10 +2893,10 @@ int ct_write_boxes(const ct_tree* t, const double* boxes, int64_t n, const int32
     const int bt = box_threads(t);
     if (deep_tree(t))
         k_boxes<true, true><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(make_q(t), (const double4*)boxes, n,
-                                                                             order, (int64_t*)offsets, ii, jj);
+                                                                            order, (int64_t*)offsets, ii, jj);
     else
-        k_boxes<true, false><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(make_q(t), (const double4*)boxes, n,
-                                                                              order, (int64_t*)offsets, ii, jj);
+        launch_box_walk<true>(make_q(t), (const double4*)boxes, n, order, (int64_t*)offsets, ii, jj, nullptr, 0,
+                              nullptr, (cudaStream_t)stream);
     CT_CHECK_LAUNCH("write_boxes");
     return CT_OK;
 }
@@ -2700,19 +2919,16 @@ int ct_write_boxes_ws(const ct_tree* t, const double* boxes, int64_t n, const in
         return ct_fail(CT_ERR_WORKSPACE, "write_boxes workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     TreeQ T = make_q(t);
-    if (!T.nbx) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);  // no box index: no subtrees
+    // no box index: no subtrees; the warps' walk writes them by itself
+    if (!T.nbx || !deep_tree(t)) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);
     const int jm = box_job_min(min_job_cells);
     unsigned long long* njobs = (unsigned long long*)ws;
     BoxJob* jobs = (BoxJob*)((char*)ws + 256);
     const int64_t cap = (total_pairs > 0 ? total_pairs : 0) / jm + 1;
     CT_CUDA(cudaMemsetAsync(njobs, 0, sizeof(unsigned long long), st));
     const int bt = box_threads(t);
-    if (deep_tree(t))
-        k_boxes<true, true><<<grid_of(n, bt), bt, 0, st>>>(T, (const double4*)boxes, n, order, (int64_t*)offsets,
-                                                           ii, jj, jobs, njobs, cap, jm);
-    else
-        k_boxes<true, false><<<grid_of(n, bt), bt, 0, st>>>(T, (const double4*)boxes, n, order, (int64_t*)offsets,
-                                                            ii, jj, jobs, njobs, cap, jm);
+    k_boxes<true, true><<<grid_of(n, bt), bt, 0, st>>>(T, (const double4*)boxes, n, order, (int64_t*)offsets, ii, jj,
+                                                      jobs, njobs, cap, jm);
     k_box_jobs<<<152 * 8, 256, 0, st>>>(jobs, njobs, cap, T.lstart, T.bbi, ii, jj, T.err);
     CT_CHECK_LAUNCH("write_boxes");
     return CT_OK;
@@ -2731,11 +2947,25 @@ int ct_count_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const 
     const double4* B = (const double4*)boxes;
     if (deep_tree(t))
         k_boxes<false, true><<<grid_of(n, bt), bt, 0, st>>>(T, B, n, order, counts, nullptr, nullptr, nullptr, nullptr,
-                                                            0, BOX_JOB_MIN, spec, spec_cap, nullptr);
+                                                           0, BOX_JOB_MIN, spec, spec_cap, nullptr);
     else
-        k_boxes<false, false><<<grid_of(n, bt), bt, 0, st>>>(T, B, n, order, counts, nullptr, nullptr, nullptr,
-                                                             nullptr, 0, BOX_JOB_MIN, spec, spec_cap, nullptr);
+        launch_box_walk<false>(T, B, n, order, counts, nullptr, nullptr, spec, spec_cap, nullptr, st);
     CT_CHECK_LAUNCH("count_boxes_spec");
+    return CT_OK;
+}
+
+int ct_count_small_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
+                              int32_t* spec, int32_t spec_cap, void* stream) {
+    int s = check_tree(t);
+    if (s) return s;
+    if (n == 0 || deep_tree(t)) return ct_count_boxes_spec(t, boxes, n, order, counts, spec, spec_cap, stream);
+    if (!spec || spec_cap < 1 || spec_cap > 4096) return ct_fail(CT_ERR_ARG, "spec_cap must be in [1, 4096]");
+    if (t->n_elements >= INT32_MAX) return ct_fail(CT_ERR_ARG, "tree size out of range");
+    const int bt = box_threads(t);
+    k_boxes<false, false><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(
+        make_q(t), (const double4*)boxes, n, order, counts, nullptr, nullptr, nullptr, nullptr, 0, BOX_JOB_MIN, spec,
+        spec_cap, nullptr);
+    CT_CHECK_LAUNCH("count_small_boxes_spec");
     return CT_OK;
 }
 
@@ -2754,20 +2984,21 @@ int ct_write_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const 
     const TreeQ T = make_q(t);
     k_boxes_spec_emit<<<(unsigned)std::min<int64_t>(grid_of(n * (int64_t)spec_cap, 256), 152 * 16), 256, 0, st>>>(
         counts, offsets, n, spec, spec_cap, ii, jj);
+    int64_t* off = (int64_t*)offsets;
+    const double4* B = (const double4*)boxes;
+    if (!deep_tree(t)) {
+        launch_box_walk<true>(T, B, n, order, off, ii, jj, nullptr, spec_cap, counts, st);
+        CT_CHECK_LAUNCH("write_boxes_spec");
+        return CT_OK;
+    }
     const int jm = box_job_min(min_job_cells);
     unsigned long long* njobs = (unsigned long long*)ws;
     BoxJob* jobs = T.nbx ? (BoxJob*)((char*)ws + 256) : nullptr;
     const int64_t cap = (total_pairs > 0 ? total_pairs : 0) / jm + 1;
     CT_CUDA(cudaMemsetAsync(njobs, 0, sizeof(unsigned long long), st));
     const int bt = box_threads(t);
-    const double4* B = (const double4*)boxes;
-    int64_t* off = (int64_t*)offsets;
-    if (deep_tree(t))
-        k_boxes<true, true><<<grid_of(n, bt), bt, 0, st>>>(T, B, n, order, off, ii, jj, jobs, njobs, cap, jm,
-                                                           nullptr, spec_cap, counts);
-    else
-        k_boxes<true, false><<<grid_of(n, bt), bt, 0, st>>>(T, B, n, order, off, ii, jj, jobs, njobs, cap, jm,
-                                                            nullptr, spec_cap, counts);
+    k_boxes<true, true><<<grid_of(n, bt), bt, 0, st>>>(T, B, n, order, off, ii, jj, jobs, njobs, cap, jm, nullptr,
+                                                      spec_cap, counts);
     if (jobs) k_box_jobs<<<152 * 8, 256, 0, st>>>(jobs, njobs, cap, T.lstart, T.bbi, ii, jj, T.err);
     CT_CHECK_LAUNCH("write_boxes_spec");
     return CT_OK;

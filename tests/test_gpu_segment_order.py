@@ -39,11 +39,13 @@ def test_hits_per_segment(oracle, cells, work_order):
 
 
 @pytest.mark.parametrize("n", [65535, 65536, 70001])
-def test_spatial_order_of_large_batches(oracle, n):
+def test_spatial_order_of_large_batches(oracle, n, monkeypatch):
     import torch
 
     from numba_celltree_gb300 import CellTree2d, EdgeCellTree2d
+    from numba_celltree_gb300.celltree_base import _GpuTree
 
+    monkeypatch.setattr(_GpuTree, "ORDER_MIN_CELLS", 0)
     xy, f = syn.mixed_mesh(60, seed=5, extent=(60.0, 60.0))
     rng = np.random.default_rng(n)
     a = rng.uniform(-3.0, 63.0, (n, 2))
