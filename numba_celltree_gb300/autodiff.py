@@ -36,6 +36,29 @@ def _check_vertices(v, n_vertices: int, name: str):
     return v
 
 
+def _area_grad(ctx, g):
+    """Gradients to both meshes' vertices of the areas of the saved pairs."""
+    torch = _torch()
+    va, vb, fa, fb, ia, ib = ctx.saved_tensors
+    err = ctx.err
+    err.zero_()
+    gva = torch.zeros_like(va)
+    gvb = torch.zeros_like(vb)
+    g = g.detach().to(torch.float64).contiguous()
+    _lib.check(
+        _lib.load().ct_area_of_intersection_grad(
+            _device.ptr(va), _device.ptr(fa), int(fa.shape[1]), _device.ptr(vb), _device.ptr(fb),
+            int(fb.shape[1]), _device.ptr(ia), _device.ptr(ib), int(ia.shape[0]), _device.ptr(g),
+            _device.ptr(gva), _device.ptr(gvb), _device.ptr(err), _device.stream(),
+        ),
+        "area_of_intersection_grad",
+    )
+    if int(err.item()):
+        raise _lib.CellTreeError("area_of_intersection_grad: clip polygon scratch overflow")
+    return (gva if ctx.needs_input_grad[0] else None, gvb if ctx.needs_input_grad[1] else None,
+            None, None, None, None, None)
+
+
 def _make_functions():
     torch = _torch()
 
@@ -61,24 +84,39 @@ def _make_functions():
 
         @staticmethod
         def backward(ctx, g):
-            va, vb, fa, fb, ia, ib = ctx.saved_tensors
-            err = ctx.err
-            err.zero_()
-            gva = torch.zeros_like(va)
-            gvb = torch.zeros_like(vb)
-            g = g.detach().to(torch.float64).contiguous()
+            return _area_grad(ctx, g)
+
+    class KeptArea(torch.autograd.Function):
+        """The pairs of (ia, ib) that overlap, and their areas.  The pairs
+        dropped have area zero and no gradient, so the backward pass runs over
+        the kept ones alone (an indexing of the areas by a mask would sort
+        them on the way back)."""
+
+        @staticmethod
+        def forward(ctx, va, vb, fa, fb, ia, ib, tree):
+            n = int(ia.shape[0])
+            area = torch.empty((n,), dtype=torch.float64, device=va.device)
+            va_c, vb_c = va.detach().contiguous(), vb.detach().contiguous()
             _lib.check(
-                _lib.load().ct_area_of_intersection_grad(
-                    _device.ptr(va), _device.ptr(fa), int(fa.shape[1]), _device.ptr(vb), _device.ptr(fb),
-                    int(fb.shape[1]), _device.ptr(ia), _device.ptr(ib), int(ia.shape[0]), _device.ptr(g),
-                    _device.ptr(gva), _device.ptr(gvb), _device.ptr(err), _device.stream(),
+                _lib.load().ct_area_of_intersection(
+                    _device.ptr(va_c), _device.ptr(fa), int(fa.shape[1]), _device.ptr(vb_c), _device.ptr(fb),
+                    int(fb.shape[1]), _device.ptr(ia), _device.ptr(ib), n, _device.ptr(area),
+                    _device.ptr(tree.error_word), _device.stream(),
                 ),
-                "area_of_intersection_grad",
+                "area_of_intersection",
             )
-            if int(err.item()):
-                raise _lib.CellTreeError("area_of_intersection_grad: clip polygon scratch overflow")
-            return (gva if ctx.needs_input_grad[0] else None, gvb if ctx.needs_input_grad[1] else None,
-                    None, None, None, None, None)
+            tree.stage_error()
+            i, j, kept = (x.clone() for x in tree.compact(ia, ib, area=area))  # synchronises (pair count)
+            tree.raise_on_staged_error()
+            ctx.mark_non_differentiable(i, j)
+            ctx.set_materialize_grads(False)  # no zeros for the index outputs
+            ctx.save_for_backward(va_c, vb_c, fa, fb, i, j)
+            ctx.err = tree.error_word
+            return i, j, kept
+
+        @staticmethod
+        def backward(ctx, gi, gj, g):
+            return (None,) * 7 if g is None else _area_grad(ctx, g)
 
     class BarycentricWeights(torch.autograd.Function):
         """weights[i] of point i in tree face face_index[i] (zero row for -1)."""
@@ -125,7 +163,7 @@ def _make_functions():
             return (gp if ctx.needs_input_grad[0] else None, gv if ctx.needs_input_grad[1] else None,
                     None, None, None)
 
-    return ClipArea, BarycentricWeights
+    return ClipArea, BarycentricWeights, KeptArea
 
 
 _FUNCS = None
@@ -148,24 +186,23 @@ def intersect_faces(tree, vertices, faces, fill_value: int = -1, tree_vertices=N
     ``vertices`` and ``tree_vertices`` (indices held fixed).
     """
     torch = _torch()
-    ClipArea, _ = _functions()
+    KeptArea = _functions()[2]
     t = tree._tree
     tv = t.vertices if tree_vertices is None else _check_vertices(tree_vertices, int(t.vertices.shape[0]),
                                                                       "tree_vertices")
     if not (isinstance(vertices, torch.Tensor) and vertices.is_cuda):
         vertices = torch.as_tensor(cast_vertices(vertices), device=t.device)
     v = _check_vertices(vertices, int(vertices.shape[0]), "vertices")
-    f = cast_faces(faces.detach().cpu().numpy() if isinstance(faces, torch.Tensor) else faces, fill_value)
+    if isinstance(faces, torch.Tensor) and not faces.is_cuda:
+        faces = faces.detach().numpy()
+    f = cast_faces(faces, fill_value)
     v_d, f_d = tree._faces_on_device(v.detach(), f)
     if f_d.shape[0] == 0:
         e = torch.empty((0,), dtype=torch.int64, device=t.device)
         return e, e, torch.empty((0,), dtype=torch.float64, device=t.device)
     i, j = tree._locate_faces_dev(v_d, f_d)  # orients f_d counter-clockwise in place, as upstream
     t.reset_error()
-    area = ClipArea.apply(v, tv, f_d, t.elements, i, j, t.error_word)
-    t.raise_on_device_error()
-    keep = area.detach() > 0
-    return i[keep], j[keep], area[keep]
+    return KeptArea.apply(v, tv, f_d, t.elements, i, j, t)
 
 
 def compute_barycentric_weights(tree, points, tolerance: Optional[float] = None, tree_vertices=None):
@@ -176,7 +213,7 @@ def compute_barycentric_weights(tree, points, tolerance: Optional[float] = None,
     fixed).
     """
     torch = _torch()
-    _, BarycentricWeights = _functions()
+    BarycentricWeights = _functions()[1]
     t = tree._tree
     tol = tree._tolerance(tolerance)
     tv = t.vertices if tree_vertices is None else _check_vertices(tree_vertices, int(t.vertices.shape[0]),

@@ -16,6 +16,7 @@
 // line, |cross| = 0) take the subgradient that treats sign(0) as 0.
 #include <cstdint>
 
+#include "ct_clip.cuh"
 #include "ct_common.cuh"
 #include "ct_geom.cuh"
 #include "ct_internal.h"
@@ -113,21 +114,14 @@ __device__ int clip_taped(Clip& C, const dpt* subj, int la, const dpt* clip, int
     return nn;
 }
 
-// Gradient of the area of intersection of every pair (ia[t], ib[t]) with
-// upstream gradient g[t]; accumulated into gva (subject mesh) and gvb
-// (clipper / tree mesh).
-__global__ void k_clip_area_grad(const double* __restrict__ va, const int64_t* __restrict__ fa, int Ka,
-                                 const double* __restrict__ vb, const int64_t* __restrict__ fb, int Kb,
-                                 const int64_t* __restrict__ ia, const int64_t* __restrict__ ib, int64_t n,
-                                 const double* __restrict__ g, double* __restrict__ gva, double* __restrict__ gvb,
-                                 unsigned int* __restrict__ err) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const double G = g[t];
-    if (G == 0.0) return;
+// Gradient of the area of intersection of one pair with upstream gradient G,
+// by the tape; accumulated into gva (subject mesh) and gvb (clipper / tree
+// mesh).
+__device__ __noinline__ void clip_grad_taped(const double* __restrict__ va, const int64_t* __restrict__ face_a, int Ka,
+                                             const double* __restrict__ vb, const int64_t* __restrict__ face_b,
+                                             int Kb, double G, double* __restrict__ gva, double* __restrict__ gvb,
+                                             unsigned int* __restrict__ err) {
     dpt a[CT_MAX_N_VERTEX], b[CT_MAX_N_VERTEX];
-    const int64_t* face_a = fa + ia[t] * Ka;
-    const int64_t* face_b = fb + ib[t] * Kb;
     int la = gather_polygon(va, face_a, Ka, a);
     int lb = gather_polygon(vb, face_b, Kb, b);
     if (la < 1 || lb < 1) return;
@@ -197,6 +191,101 @@ __global__ void k_clip_area_grad(const double* __restrict__ va, const int64_t* _
         int64_t vi = face_b[k];
         if (cadj[k].x != 0.0) atomicAdd(&gvb[2 * vi], cadj[k].x);
         if (cadj[k].y != 0.0) atomicAdd(&gvb[2 * vi + 1], cadj[k].y);
+    }
+}
+
+// Gradients of every pair (ia[t], ib[t]) with upstream gradient g[t].
+__global__ void k_clip_area_grad(const double* __restrict__ va, const int64_t* __restrict__ fa, int Ka,
+                                 const double* __restrict__ vb, const int64_t* __restrict__ fb, int Kb,
+                                 const int64_t* __restrict__ ia, const int64_t* __restrict__ ib, int64_t n,
+                                 const double* __restrict__ g, double* __restrict__ gva, double* __restrict__ gvb,
+                                 unsigned int* __restrict__ err) {
+    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n || g[t] == 0.0) return;
+    clip_grad_taped(va, fa + ia[t] * Ka, Ka, vb, fb + ib[t] * Kb, Kb, g[t], gva, gvb, err);
+}
+
+__device__ __forceinline__ void add_grad(double* __restrict__ g, int64_t v, double x, double y) {
+    if (x != 0.0) atomicAdd(&g[2 * v], x);
+    if (y != 0.0) atomicAdd(&g[2 * v + 1], y);
+}
+
+// The same for polygons of up to 8 vertices: the clip of ct_clip.cuh with each
+// edge of the clipped polygon known to lie on an edge p -> q of the subject or
+// the clipper.  When p and q move, the edge moves with them, and the area
+// changes by the flux through it: for a counter-clockwise polygon and its edge
+// P -> Q with normal n = (dy, -dx), d area = n . ((1 - t) dp + t dq), t the
+// parameter of the edge's middle on p -> q.  That is the derivative of the fan
+// area the tape replays whenever the fan's triangles all turn one way; a
+// triangle whose turn float32 does not settle (vertices in line, slivers), a
+// pair the small clip does not handle and a clipper edge of no length take
+// the tape.
+// The tape kept 8 KB per thread in local memory and a chain of up to six
+// adjoint steps; this is 20 float64 instructions per edge after the clip.
+// 860k (triangle, quad) pairs: 1.90 -> 0.51 ms.
+template <int KT>
+__global__ void __launch_bounds__(CL_THREADS) k_clip_area_grad_small(
+    const double2* __restrict__ va, const int64_t* __restrict__ fa, int Ka, const double2* __restrict__ vb,
+    const int64_t* __restrict__ fb, int Kb, const int64_t* __restrict__ ia, const int64_t* __restrict__ ib, int64_t n,
+    const double* __restrict__ g, double* __restrict__ gva, double* __restrict__ gvb, unsigned int* __restrict__ err) {
+    __shared__ ClipCols<KT> S;
+    const float u24 = 5.9604644775390625e-08f;
+    const int tid = threadIdx.x;
+    const int64_t t = (int64_t)blockIdx.x * CL_THREADS + tid;
+    if (t >= n) return;
+    const double G = g[t];
+    if (G == 0.0) return;
+    const int64_t *face_a = fa + ia[t] * Ka, *face_b = fb + ib[t] * Kb;
+    const int la = polygon_length(face_a, Ka), lb = polygon_length(face_b, Kb);
+    for (int k = 0; k < la; k++) S.v[k][tid] = va[face_a[k]];
+    for (int k = 0; k < lb; k++) S.c[k][tid] = vb[face_b[k]];
+    ClipPoly C;
+    bool ok = clip_small<KT, false, true>(S, tid, la, lb, &C);
+    if (ok && C.L == 0) return;  // area 0: zero gradient
+    // the turn of every fan triangle
+    bool left = false, right = false;
+    if (ok) {
+        const float2 f0 = S.f[C.list & 7u][tid];
+        float2 u = S.f[(C.list >> 4) & 7u][tid];
+        u = make_float2(u.x - f0.x, u.y - f0.y);
+        for (int k = 2; k < C.L; k++) {
+            float2 w = S.f[(C.list >> (4 * k)) & 7u][tid];
+            w = make_float2(w.x - f0.x, w.y - f0.y);
+            const float p = u.x * w.y, q = u.y * w.x, c = p - q;
+            const float thr = 16.0f * u24 * (fabsf(p) + fabsf(q)) +
+                              2.2f * C.ed * (fabsf(u.x) + fabsf(u.y) + fabsf(w.x) + fabsf(w.y) + 2.0f * C.ed) + 1e-37f;
+            left = left || c > thr;
+            right = right || c < -thr;
+            ok = ok && fabsf(c) > thr;
+            u = w;
+        }
+    }
+    if (!ok || left == right) {
+        clip_grad_taped((const double*)va, face_a, Ka, (const double*)vb, face_b, Kb, G, gva, gvb, err);
+        return;
+    }
+    const double s = left ? G : -G;
+    for (int k = 0; k < C.L; k++) {
+        const double2 P = S.v[(C.list >> (4 * k)) & 7u][tid];
+        const double2 Q = S.v[(C.list >> (k + 1 < C.L ? 4 * k + 4 : 0)) & 7u][tid];
+        const uint32_t e = (C.own >> (4 * k)) & 15u;
+        const bool clip = e >= 8u;
+        // the edge's two vertices
+        const int i1 = clip ? (int)e - 8 : ((int)e + 1 < la ? (int)e + 1 : 0);
+        const int i0 = clip ? (i1 > 0 ? i1 - 1 : lb - 1) : (int)e;
+        const int64_t v0 = clip ? face_b[i0] : face_a[i0], v1 = clip ? face_b[i1] : face_a[i1];
+        const double2 p = clip ? S.c[i0][tid] : va[v0], q = clip ? S.c[i1][tid] : va[v1];
+        const double ex = q.x - p.x, ey = q.y - p.y;
+        const double mx = (P.x - p.x) + (Q.x - p.x), my = (P.y - p.y) + (Q.y - p.y);
+        const double num = __fma_rn(mx, ex, my * ey), den = 2.0 * __fma_rn(ex, ex, ey * ey);
+        bool bad = false;
+        double m = sf_div(num, den, &bad);
+        if (bad) m = num / den;
+        const double nx = s * (Q.y - P.y), ny = s * (P.x - Q.x);
+        const double gx = nx * m, gy = ny * m;
+        double* grad = clip ? gvb : gva;
+        add_grad(grad, v1, gx, gy);
+        add_grad(grad, v0, nx - gx, ny - gy);
     }
 }
 
@@ -343,8 +432,17 @@ int ct_area_of_intersection_grad(const double* va, const int64_t* fa, int32_t Ka
     if (!va || !fa || !vb || !fb || !ia || !ib || !grad_area || !grad_va || !grad_vb)
         return ct_fail(CT_ERR_ARG, "null argument");
     unsigned grid = (unsigned)((n + 127) / 128);
-    k_clip_area_grad<<<grid, 128, 0, (cudaStream_t)stream>>>(va, fa, Ka, vb, fb, Kb, ia, ib, n, grad_area, grad_va,
-                                                             grad_vb, error_word);
+    cudaStream_t st = (cudaStream_t)stream;
+    const double2 *a = (const double2*)va, *b = (const double2*)vb;
+    if (Ka < 3 || Ka > CL_SLOTS || Kb < 3 || Kb > 8 || (((uintptr_t)va | (uintptr_t)vb) & 15))
+        k_clip_area_grad<<<grid, 128, 0, st>>>(va, fa, Ka, vb, fb, Kb, ia, ib, n, grad_area, grad_va, grad_vb,
+                                               error_word);
+    else if (Kb <= 4)
+        k_clip_area_grad_small<4><<<grid, CL_THREADS, 0, st>>>(a, fa, Ka, b, fb, Kb, ia, ib, n, grad_area, grad_va,
+                                                               grad_vb, error_word);
+    else
+        k_clip_area_grad_small<8><<<grid, CL_THREADS, 0, st>>>(a, fa, Ka, b, fb, Kb, ia, ib, n, grad_area, grad_va,
+                                                               grad_vb, error_word);
     CT_CHECK_LAUNCH("area_of_intersection_grad");
     return CT_OK;
 }

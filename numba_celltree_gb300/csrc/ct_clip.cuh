@@ -98,10 +98,21 @@ __device__ __forceinline__ ClipCross cl_cross(double2 a2, double2 b2, float2 fa,
     return c;
 }
 
+// The clipped polygon: slots of its L (0: nothing left) vertices in order,
+// with OWN the edge each vertex's outgoing edge lies on (subject edge k, from
+// its vertex k, or 8 + i, the clipper's edge to its vertex i), and the error
+// of its float32 coordinates.
+struct ClipPoly {
+    uint32_t list, own;
+    int L;
+    float ed;
+};
+
 // The subject's n_poly (<= CL_SLOTS) vertices in S.v and the clipper's n_clip
-// in S.c (column of the thread).  False: not handled here.
-template <int KT, bool BOX>
-__device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_poly, int n_clip, double* area) {
+// in S.c (column of the thread).  False: not handled here (with OWN also
+// clippers with an edge of no length).
+template <int KT, bool BOX, bool OWN>
+__device__ __forceinline__ bool clip_small(ClipCols<KT>& S, int tid, int n_poly, int n_clip, ClipPoly* C) {
     const float u24 = 5.9604644775390625e-08f;
     const double2 O = S.c[0][tid];
     float mx = 0.0f;
@@ -133,12 +144,17 @@ __device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_
     uint32_t list = 0x76543210u;
     int L = n_poly;
     if (L < CL_SLOTS) list &= (1u << (4 * L)) - 1u;
+    uint32_t own = list;
+    C->L = 0;
     for (int k = 0, p = n_poly - 1; k < n_poly; p = k, k++)
         if (cl_equal(S.f[k][tid], S.f[p][tid], ed, S.v[k][tid], S.v[p][tid])) return false;
     for (int i = 0; i < n_clip; i++) {
         const double2 s = S.c[i][tid];
         const dpt U = mkp(s.x - r.x, s.y - r.y);
-        if (g_zero(U.x) && g_zero(U.y)) continue;
+        if (g_zero(U.x) && g_zero(U.y)) {
+            if (OWN) return false;
+            continue;
+        }
         const float2 uf = make_float2(cl_float(U.x), cl_float(U.y));
         if (!(cl_max2(uf) < 1e15f && cl_max2(fr) < 1e15f)) return false;
         // Inside test U.x (b.y - r.y) > U.y (b.x - r.x) in float32: with W =
@@ -166,10 +182,7 @@ __device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_
             in = (in & ~(1u << j)) | ((lhs > rhs ? 1u : 0u) << j);
         }
         const uint32_t full = (1u << L) - 1u;
-        if (in == 0u) {
-            *area = 0.0;
-            return true;
-        }
+        if (in == 0u) return true;
         if (in != full) {
             const uint32_t prev = ((in << 1) | (in >> (L - 1))) & full;
             const uint32_t enter = in & ~prev, leave = prev & ~in;
@@ -198,11 +211,15 @@ __device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_
             // the walk's output order: a run of kept vertices je .. between
             // its two crossings, or, when the last vertex is kept, those up
             // to jl, the two crossings, those from je
-            if ((in >> (L - 1)) & 1u)
-                list = (list & ((1u << (4 * jl)) - 1u)) | (s1 << (4 * jl)) | (s0 << (4 * jl + 4)) |
-                       ((list >> (4 * je)) << (4 * jl + 8));
-            else
-                list = s0 | (((list >> (4 * je)) & ((1u << (4 * kept)) - 1u)) << 4) | (s1 << (4 * kept + 4));
+            const uint32_t oe = (own >> (4 * je0)) & 15u, ol = 8u + (uint32_t)i;
+            auto next = [&](uint32_t x, uint32_t e, uint32_t l) -> uint32_t {
+                if ((in >> (L - 1)) & 1u)
+                    return (x & ((1u << (4 * jl)) - 1u)) | (l << (4 * jl)) | (e << (4 * jl + 4)) |
+                           ((x >> (4 * je)) << (4 * jl + 8));
+                return e | (((x >> (4 * je)) & ((1u << (4 * kept)) - 1u)) << 4) | (l << (4 * kept + 4));
+            };
+            list = next(list, s0, s1);
+            if (OWN) own = next(own, oe, ol);
             L = kept + 2;
         }
         // fs = fr + U: one rounding, and the errors of both
@@ -210,16 +227,26 @@ __device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_
         fr = make_float2(fr.x + uf.x, fr.y + uf.y);
         er += eU + u24 * cl_max2(fr);
     }
-    if (L < 3) {
-        *area = 0.0;
-        return true;
-    }
+    C->list = list;
+    C->own = own;
+    C->L = L < 3 ? 0 : L;
+    C->ed = ed;
+    return true;
+}
+
+template <int KT, bool BOX>
+__device__ __forceinline__ bool clip_area_small(ClipCols<KT>& S, int tid, int n_poly, int n_clip, double* area) {
+    ClipPoly C;
+    if (!clip_small<KT, BOX, false>(S, tid, n_poly, n_clip, &C)) return false;
+    const uint32_t list = C.list;
+    *area = 0.0;
+    if (C.L == 0) return true;
     // polygon_area geometry_utils.py:82-95
     const double2 a = S.v[list & 7u][tid], b = S.v[(list >> 4) & 7u][tid];
     dpt U = mkp(b.x - a.x, b.y - a.y);
     double sum = 0.0;
     bool bad = false;
-    for (int j = 2; j < L; j++) {
+    for (int j = 2; j < C.L; j++) {
         const double2 c = S.v[(list >> (4 * j)) & 7u][tid];
         const dpt V = mkp(a.x - c.x, a.y - c.y);
         double p = sf_mul(U.x, V.y, &bad), q = sf_mul(U.y, V.x, &bad);
