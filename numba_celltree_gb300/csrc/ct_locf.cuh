@@ -131,6 +131,33 @@ __device__ __forceinline__ int leaf_filter_delta(float dx, float dy, float errd,
     return parity ? LF_INSIDE : LF_OUTSIDE;
 }
 
+// The same decision without leaving the loop early: a caller whose lanes differ
+// in whether they ask comes back together (an exit inside a branch makes the
+// compiler rejoin the lanes only at the caller's end).
+__device__ __forceinline__ int leaf_filter_joined(float dx, float dy, float errd, float dabs, float tolf,
+                                                  const float2* __restrict__ rel, int len) {
+    const float u = 5.9604644775390625e-08f;
+    const float dmax = fmaxf(fabsf(dx), fabsf(dy));
+    const float2 rl = rel[len - 2];
+    float ux = rl.x - dx, uy = rl.y - dy;
+    int parity = 0;
+    bool unsure = false;
+    for (int k = 0; k < len; k++) {
+        const float2 r = k ? rel[k - 1] : make_float2(0.0f, 0.0f);
+        const float vx = r.x - dx, vy = r.y - dy;
+        const float A = ux * vy - uy * vx;
+        const float m = fmaxf(fmaxf(fabsf(ux), fabsf(uy)), fmaxf(fabsf(vx), fabsf(vy)));
+        const float e = errd + 1.1920928955078125e-07f * (m + dmax) + dabs;
+        const float thr = 2.0f * (8.0f * u * m * m + 4.0f * m * e + 6.0f * e * e) +
+                          tolf * (fabsf(vx - ux) + fabsf(vy - uy) + 2.0f * e) * 1.000001f + 1e-30f;
+        unsure = unsure || !(fabsf(A) > thr);
+        if ((uy > 0.0f) != (vy > 0.0f)) parity ^= (int)((vy > uy) ? (A > 0.0f) : (A < 0.0f));
+        ux = vx;
+        uy = vy;
+    }
+    return unsure ? LF_UNSURE : parity ? LF_INSIDE : LF_OUTSIDE;
+}
+
 template <int KT>
 __device__ __forceinline__ int leaf_filter_local(const PtSplit& P, float dabs, float tolf,
                                                  const float4* __restrict__ cell, int len) {
