@@ -809,12 +809,12 @@ def main():
     # kernels per batched step: radix sort (key+hist, scan x3, scatter for the
     # first 8-bit digit; hist, scan x3, scatter for each further digit),
     # candidate lists (+ the two-pass bucketed scatter of their results when
-    # the queries are sorted) + open-query traversal, pair tests, resolve,
-    # overflow
+    # the queries are sorted) + open queries, overflow; without lists a
+    # traversal of every query, pair tests, resolve, overflow
     passes = bins // 8
     lists = t.cand_idx is not None and tol <= float(t.desc.cand_tol)
-    stage2 = (4 if bins and n > (1 << 23) else 2) if lists else 1
-    launches_per_step = (5 * passes if bins else 0) + stage2 + 3
+    stage2 = (5 if bins and n > (1 << 23) else 3) if lists else 4
+    launches_per_step = (5 * passes if bins else 0) + stage2
     value = ws * n / (ms32 * 1e-3) / 1e6
     value64 = ws * n / (ms64 * 1e-3) / 1e6
 

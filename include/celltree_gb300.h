@@ -105,7 +105,8 @@ typedef struct ct_tree {
                                  float32 frame, leaf order */
     int64_t cand_n;           /* host: entries of cand_idx */
     double cand_tol;          /* host: largest query tolerance the lists cover */
-    int32_t bounds_finite;    /* host (ct_pack_tree): every node bound and bb_coords value is finite */
+    int32_t bounds_finite;    /* host (ct_pack_tree): 1: every node bound and bb_coords value is finite; 3: and
+                               * every inner node's positions are its left child's, then its right child's */
     /* box index of the multi-result queries (filled by ct_pack_box_index;
      * all three NULL disables it) */
     void* bb_leaf;            /* device: n_elements x 4 doubles, bb_coords in leaf (bb_indices) order */

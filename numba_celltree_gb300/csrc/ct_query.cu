@@ -529,6 +529,13 @@ __global__ void k_pack_nodes(int64_t n_nodes, const int64_t* __restrict__ child,
         parent[c + 1] = (int)v;
     }
     if (c == -1 && (ptr[v] < 0 || size[v] < 0 || ptr[v] + size[v] > n_elem)) atomicOr(bad, 1u);
+    // a node's positions are its left child's, then its right one's: the order
+    // of two cells in a walk can be had from their positions
+    if (v == 0 && (ptr[0] != 0 || size[0] != n_elem)) atomicOr(bad, 4u);
+    if (c > v && c + 1 < n_nodes &&
+        (ptr[c] != ptr[v] || size[c] < 0 || size[c + 1] < 0 || ptr[c + 1] != ptr[v] + size[c] ||
+         size[v] != size[c] + size[c + 1]))
+        atomicOr(bad, 4u);
     double L = Lmax[v], R = Rmin[v];
     if (!isfinite(L) || !isfinite(R)) atomicOr(bad, 2u);  // not an error: queries keep the literal float64 path
     nd[v] = make_double2(L, R);
@@ -737,7 +744,7 @@ int ct_pack_tree(ct_tree* t, void* stream) {
     CT_CUDA(cudaMemcpyAsync(hv, red, sizeof(hv), cudaMemcpyDeviceToHost, st));
     CT_CUDA(cudaStreamSynchronize(st));
     if (hv[1] & 1u) return ct_fail(CT_ERR_DEVICE, "tree structure check failed (child or leaf range out of order)");
-    t->bounds_finite = (hv[1] & 2u) ? 0 : 1;
+    t->bounds_finite = (hv[1] & 2u) ? 0 : (hv[1] & 4u) ? 1 : 3;
     t->vmax = 0.0f;  // unused by the local-frame float32 cells
     // float64 rounding of absolute vertex coordinates (the float64 predicate
     // rounds relative to them): 2^-50 * max |coordinate|
