@@ -43,7 +43,7 @@ constexpr int NBMAX = 32;          // maximum n_buckets
 constexpr int STATS_THREADS = 256; // threads of the stats / scatter CTAs
 constexpr int TILE_MIN = 2048;     // minimum cells per tile
 constexpr int MAX_TILES = 512;     // maximum tiles per node
-constexpr int SUB_WARPS = 2;       // warps per CTA in the subtree kernel (8.1 KB of shared memory each)
+constexpr int SUB_WARPS = 2;       // warps per CTA in the subtree kernel (10.5 KB of shared memory each)
 
 enum : int { K_PENDING = 0, K_SPLIT = 1, K_LEAF = 2, K_SUBTREE = 3 };
 
@@ -231,6 +231,7 @@ struct Decision {
     int kind;     // 0: all cells in one bucket, 1: split, -1: error
     int nleft;    // cells in the left child
     int rbucket;  // first bucket of the right child
+    int lbucket, rbest;  // buckets whose bounds are Lmax and Rmin
     double Lmax, Rmin;
 };
 
@@ -246,7 +247,7 @@ __device__ Decision warp_decide(const int* cnt, const double* bRmin, const doubl
     Decision D;
     D.kind = -1;
     D.nleft = 0;
-    D.rbucket = -1;
+    D.rbucket = D.lbucket = D.rbest = -1;
     D.Lmax = -1.0;
     D.Rmin = -1.0;
     bool ne = lane < NB && cnt[lane] > 0;
@@ -328,6 +329,8 @@ __device__ Decision warp_decide(const int* cnt, const double* bRmin, const doubl
     group_min_kp(FULL, kr, (unsigned)lane, &ko, &pr);
     int bl_w = __shfl_sync(FULL, bk, (int)pl);
     int br_w = __shfl_sync(FULL, bk, (int)pr);
+    D.lbucket = bl_w;
+    D.rbest = br_w;
     D.Lmax = bLmax[bl_w];
     D.Rmin = bRmin[br_w];
     D.nleft = __shfl_sync(FULL, pre, plane - 1);
@@ -818,52 +821,120 @@ __global__ void __launch_bounds__(STATS_THREADS) k_scatter(WS ws, int parity, in
 
 // ------------------------------------------------------------------------
 // phase B: one warp builds a subtree of <= SMALL cells in shared memory
+//
+// Nodes of more than SUB_TINY cells take the whole warp, one after another;
+// smaller ones a lane each, a level of the subtree at a time.  Most nodes of a
+// subtree are small (of 128 cells: 3 inner nodes above 32 cells, about 75
+// below), and a node costs the warp the same instructions whether 4 lanes have
+// a cell or 32 lanes have a node.  A tree of 16M cells: all nodes by the whole
+// warp 10.5 ms (700 instructions a node), lanes from 16 cells 4.3 ms, with the
+// centroids and order keys computed once a cell 3.6, lanes from 12 / 24 / 32
+// cells 5.0 / 3.7 / 3.2 ms.  What bounds it now: issue at 20 warps per SM, a
+// level's longest node.
+//
+// A split is known by the gap it makes: the last position of its left child.
+// Gaps are distinct, and the splits before one in upstream's (pre-order)
+// numbering are those with a gap before its first position and its ancestors
+// that it lies left of.  So nodes can be processed in any order and are
+// numbered at the end.
 // ------------------------------------------------------------------------
+constexpr int SUB_TINY = 32;  // cells of a node that one lane processes (4 buckets)
+static_assert(SUB_TINY <= 32, "a node's bucket numbers are held in 64 bits");
 
-// Per-warp shared memory of a subtree: the four box fields of its cells
-// (the centroids are recomputed from them with the expression that produced
-// them, so the same bits), and the node stack as packed arrays.  8.1 KB, so
-// that more warps are resident (the kernel is bound by issue latency).
+// Per-warp shared memory of a subtree: order keys of its cells' four box
+// fields (complemented for the maxima, so that every extreme is a minimum) and
+// of their centroids, the open nodes and the splits, by gap.
 struct SubSmem {
-    double F[4][SMALL];
+    unsigned long long F[4][SMALL];
+    unsigned long long C[2][SMALL];
     unsigned long long K[NBMAX + 1];
     double bRmin[NBMAX];
     double bLmax[NBMAX];
-    int gid[SMALL];
-    int stk_v[SMALL + 2];      // node
-    int stk_depth[SMALL + 2];  // depth
+    unsigned long long big[SMALL / 2];      // open nodes (sub_node)
+    unsigned long long tiny[2][SMALL / 2];  // those of a lane each, this level and the next
     int cnt[NBMAX];
     int bstart[NBMAX];
     int brun[NBMAX];
-    unsigned short perm[SMALL];
-    unsigned short tmp[SMALL];
-    unsigned short stk_p[SMALL + 2];  // local ptr
-    unsigned short stk_n[SMALL + 2];  // size
-    unsigned char bkt[SMALL];         // bucket of each position before the partition
-    unsigned char nbkt[SMALL];        // bucket of each position after it
-    signed char stk_flag[SMALL + 2];  // dim, or dim - 2 after an all-in-one-bucket flip
+    unsigned char perm[SMALL];
+    unsigned char tmp[SMALL];
+    unsigned char bkt[SMALL];   // bucket of each position before the partition
+    unsigned char nbkt[SMALL];  // bucket of each position after it
+    // the split at gap g: first position, size (0: no split), ancestors it is
+    // left of, parent's gap (SUB_ROOT: none), cells whose bounds are Lmax and
+    // Rmin, flags: bit 0 the dimension, bit 1 a right child
+    unsigned char gp[SMALL], gn[SMALL], gleft[SMALL], gpar[SMALL], gmax[SMALL], gmin[SMALL], gflag[SMALL];
+    unsigned char gchild[2][SMALL];  // its children: SUB_LEAF, SUB_SPLIT, SUB_TURNED
+    int root;                        // the same for the subtree's root
 };
-static_assert(SMALL <= 65535, "subtree positions are 16-bit");
+static_assert(SMALL <= 128, "positions and sizes are bytes");
+constexpr int SUB_ROOT = 255;
+enum { SUB_LEAF = 0, SUB_SPLIT = 1, SUB_TURNED = 2 };  // TURNED: a leaf after its dimension was changed
 
-__device__ __forceinline__ void sub_push(SubSmem& S, int sp, int v, int p, int n, int flag, int depth) {
-    S.stk_v[sp] = v;
-    S.stk_p[sp] = (unsigned short)p;
-    S.stk_n[sp] = (unsigned short)n;
-    S.stk_flag[sp] = (signed char)flag;
-    S.stk_depth[sp] = depth;
+// An open node: first position, size, dimension, whether that was changed,
+// right child, parent's gap, ancestors it lies left of, depth below the root.
+struct SubNode {
+    int p, n, d, turned, side, par, left, depth;
+};
+__device__ __forceinline__ unsigned long long sub_pack(const SubNode& v) {
+    return (unsigned long long)((unsigned)v.p | (unsigned)v.n << 8 | (unsigned)v.d << 16 | (unsigned)v.turned << 17 |
+                                (unsigned)v.side << 18) |
+           (unsigned long long)((unsigned)v.par | (unsigned)v.left << 8 | (unsigned)v.depth << 16) << 32;
+}
+__device__ __forceinline__ SubNode sub_unpack(unsigned long long w) {
+    const unsigned a = (unsigned)w, b = (unsigned)(w >> 32);
+    SubNode v;
+    v.p = a & 255u;
+    v.n = (a >> 8) & 255u;
+    v.d = (a >> 16) & 1u;
+    v.turned = (a >> 17) & 1u;
+    v.side = (a >> 18) & 1u;
+    v.par = b & 255u;
+    v.left = (b >> 8) & 255u;
+    v.depth = b >> 16;
+    return v;
+}
+__device__ __forceinline__ void sub_state(SubSmem& S, const SubNode& v, int state) {
+    if (v.par == SUB_ROOT) S.root = state;
+    else S.gchild[v.side][v.par] = (unsigned char)state;
+}
+// The split of v into its first nl cells and the others.
+__device__ __forceinline__ void sub_split(SubSmem& S, const SubNode& v, int nl, int cmax, int cmin) {
+    const int g = v.p + nl - 1;
+    S.gp[g] = (unsigned char)v.p;
+    S.gn[g] = (unsigned char)v.n;
+    S.gleft[g] = (unsigned char)v.left;
+    S.gpar[g] = (unsigned char)v.par;
+    S.gmax[g] = (unsigned char)cmax;
+    S.gmin[g] = (unsigned char)cmin;
+    S.gflag[g] = (unsigned char)(v.d | v.side << 1);
+    S.gchild[0][g] = S.gchild[1][g] = SUB_LEAF;
+    sub_state(S, v, SUB_SPLIT);
+}
+__device__ __forceinline__ SubNode sub_child(const SubNode& v, int nl, int side) {
+    SubNode c;
+    c.p = side ? v.p + nl : v.p;
+    c.n = side ? v.n - nl : nl;
+    c.d = 1 - v.d;
+    c.turned = 0;
+    c.side = side;
+    c.par = v.p + nl - 1;
+    c.left = v.left + (side ? 0 : 1);
+    c.depth = v.depth + 1;
+    return c;
 }
 
+// The bound whose key in S.F[f] is k (zeros as +0.0).
+__device__ __forceinline__ double sub_value(int f, unsigned long long k) { return fkey_inv((f & 1) ? ~k : k); }
 
-// First-occurrence min over perm[p .. p+n) of field f (min-form key: maxima
-// complemented when `is_max`); returns the exact value.  All lanes call.
-__device__ __forceinline__ double warp_range_extreme(const SubSmem& S, int f, bool is_max, int p, int n) {
+// First-occurrence extreme of field f over perm[p .. p+n): its cell.  All
+// lanes call.
+__device__ __forceinline__ int warp_range_extreme(const SubSmem& S, int f, int p, int n) {
     const unsigned FULL = 0xffffffffu;
     int lane = threadIdx.x & 31;
     unsigned long long best = ~0ull;
     unsigned bpos = 0;  // always a valid position, even for NaN-only ranges
     for (int i = lane; i < n; i += 32) {
-        unsigned long long k = fkey(S.F[f][S.perm[p + i]]);
-        if (is_max) k = ~k;
+        const unsigned long long k = S.F[f][S.perm[p + i]];
         if (k < best) {
             best = k;
             bpos = (unsigned)i;
@@ -872,11 +943,278 @@ __device__ __forceinline__ double warp_range_extreme(const SubSmem& S, int f, bo
     unsigned long long ko;
     unsigned po;
     group_min_kp(FULL, best, bpos, &ko, &po);
-    return S.F[f][S.perm[p + (int)po]];
+    return S.perm[p + (int)po];
+}
+
+// One node by the whole warp.  Returns the cells of its left child, 0: a leaf
+// (all cells in one bucket), -1: the same in this dimension, the other is
+// next, -2: cells outside the buckets (upstream indexes past its buckets).
+__device__ int sub_node_warp(SubSmem& S, const SubNode& v, int NB, long long cpl, int* cmax, int* cmin) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, p = v.p, n = v.n, d = v.d;
+    // get_bounds of the node (creation.py:271-277)
+    const int eR = warp_range_extreme(S, 2 * d, p, n), eL = warp_range_extreme(S, 2 * d + 1, p, n);
+    const double R = sub_value(0, S.F[2 * d][eR]), Lr = sub_value(1, S.F[2 * d + 1][eL]);
+    double bl = bucket_len(Lr, R, NB);
+    for (int j = lane; j <= NB; j += 32) S.K[j] = fkey(bucket_edge(j, bl, R));  // NB + 1 edges
+    if (lane < NB) {
+        S.cnt[lane] = 0;
+        S.brun[lane] = 0;
+    }
+    __syncwarp();
+    bool lbad = false;
+    for (int i = lane; i < n; i += 32) {
+        const int e = S.perm[p + i];
+        int b = find_bucket(S.K, NB, S.C[d][e]);
+        if (b < 0) {
+            lbad = true;
+            b = 0;
+        }
+        S.bkt[i] = (unsigned char)b;
+        atomicAdd(&S.cnt[b], 1);
+    }
+    if (__any_sync(FULL, lbad)) return -2;
+    __syncwarp();
+    {
+        int c = lane < NB ? S.cnt[lane] : 0;
+        int incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            int t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane < NB) S.bstart[lane] = incl - c;
+    }
+    __syncwarp();
+    // stable partition (stable_partition / sort_bbox_indices creation.py:54-150)
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        int i = c0 + lane;
+        int b = i < n ? (int)S.bkt[i] : 255;
+        unsigned grp = __match_any_sync(FULL, b);
+        int rank = __popc(grp & lanemask_lt());
+        if (i < n) {
+            const int dst = S.bstart[b] + S.brun[b] + rank;
+            S.tmp[dst] = S.perm[p + i];
+            S.nbkt[dst] = (unsigned char)b;
+        }
+        __syncwarp();
+        if (i < n && (int)(__ffs(grp) - 1) == lane) S.brun[b] += __popc(grp);
+        __syncwarp();
+    }
+    for (int i = lane; i < n; i += 32) S.perm[p + i] = S.tmp[i];
+    __syncwarp();
+    if (cpl == 1 && n == 2) {  // special case creation.py:311-320
+        *cmax = eL;
+        *cmin = eR;
+        return 1;
+    }
+    // per-bucket bounds (creation.py:300-306): the first-occurrence
+    // minimum of Rmin and maximum of Lmax of every bucket in one pass over
+    // the node's positions (after the partition bucket b is a contiguous
+    // run).  The lanes of one bucket reduce (key, position) together and
+    // their first lane folds the result into the bucket's running minimum
+    // (a later chunk never wins a tie: first occurrence).  Keys and
+    // positions use scratch the partition is done with: S.K (Rmin keys),
+    // S.bLmax viewed as keys (Lmax), S.brun / S.bstart (positions).
+    unsigned long long* kR = S.K;
+    unsigned long long* kL = reinterpret_cast<unsigned long long*>(S.bLmax);
+    if (lane < NB) {
+        kR[lane] = ~0ull;
+        kL[lane] = ~0ull;
+        S.brun[lane] = S.bstart[lane];  // positions when every key of the bucket ties at ~0
+    }
+    __syncwarp();
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int i = c0 + lane;
+        int b = -1;
+        unsigned long long kr = ~0ull, kl = ~0ull;
+        if (i < n) {
+            b = S.nbkt[i];
+            const int e = S.perm[p + i];
+            kr = S.F[2 * d][e];
+            kl = S.F[2 * d + 1][e];
+        }
+        const unsigned grp = __match_any_sync(FULL, b);
+        unsigned long long mr, ml;
+        unsigned pr, pl;
+        group_min_kp(grp, kr, (unsigned)i, &mr, &pr);
+        group_min_kp(grp, kl, (unsigned)i, &ml, &pl);
+        if (b >= 0 && lane == (int)(__ffs(grp) - 1)) {
+            if (mr < kR[b]) {
+                kR[b] = mr;
+                S.brun[b] = (int)pr;
+            }
+            if (ml < kL[b]) {
+                kL[b] = ml;
+                S.bstart[b] = (int)pl;
+            }
+        }
+        __syncwarp();
+    }
+    if (lane < NB) {
+        const bool any = S.cnt[lane] > 0;
+        const double rmin = any ? sub_value(0, S.F[2 * d][S.perm[p + S.brun[lane]]]) : DBL_MAX;
+        const double lmax = any ? sub_value(1, S.F[2 * d + 1][S.perm[p + S.bstart[lane]]]) : -DBL_MAX;
+        S.bRmin[lane] = rmin;
+        S.bLmax[lane] = lmax;  // replaces this bucket's key
+    }
+    __syncwarp();
+    const Decision D = warp_decide(S.cnt, S.bRmin, S.bLmax, NB, n, R, Lr, bl);
+    if (D.kind == 0) return v.turned ? 0 : -1;  // all cells in one bucket (creation.py:345-358)
+    if (D.kind < 0) return -2;
+    *cmax = S.perm[p + S.bstart[D.lbucket]];
+    *cmin = S.perm[p + S.brun[D.rbest]];
+    return D.nleft;
+}
+
+__device__ __forceinline__ int byte_of(unsigned w, int k) { return (int)((w >> (8 * k)) & 255u); }
+
+// The same for a node of at most SUB_TINY cells and 4 buckets, by one lane.
+__device__ __forceinline__ int sub_node_lane(SubSmem& S, const SubNode& v, long long cpl, int* cmax, int* cmin) {
+    const int p = v.p, n = v.n;
+    const unsigned long long* Flo = S.F[2 * v.d];
+    const unsigned long long* Fhi = S.F[2 * v.d + 1];
+    const unsigned long long* C = S.C[v.d];
+    unsigned long long kR = ~0ull, kL = ~0ull;
+    int eR = S.perm[p], eL = eR;
+    for (int i = 0; i < n; i++) {
+        const int e = S.perm[p + i];
+        const unsigned long long a = Flo[e], b = Fhi[e];
+        if (a < kR) {
+            kR = a;
+            eR = e;
+        }
+        if (b < kL) {
+            kL = b;
+            eL = e;
+        }
+    }
+    const double R = sub_value(0, Flo[eR]), Lr = sub_value(1, Fhi[eL]);
+    const double bl = bucket_len(Lr, R, 4);
+    const unsigned long long K0 = fkey(bucket_edge(0, bl, R)), K1 = fkey(bucket_edge(1, bl, R)),
+                             K2 = fkey(bucket_edge(2, bl, R)), K3 = fkey(bucket_edge(3, bl, R)),
+                             K4 = fkey(bucket_edge(4, bl, R));
+    // bucket of every cell (2 bits each), cells and, in order of first
+    // occurrence, cells of the extreme bounds of every bucket (a byte each)
+    unsigned long long codes = 0;
+    unsigned count = 0, cR = 0, cL = 0;
+    bool bad = false;
+    for (int i = 0; i < n; i++) {
+        const int e = S.perm[p + i];
+        const unsigned long long kc = C[e];
+        bad = bad || kc < K0 || kc >= K4;
+        const int q = K2 <= kc ? (K3 <= kc ? 3 : 2) : (K1 <= kc ? 1 : 0);  // find_bucket
+        codes |= (unsigned long long)q << (2 * i);
+        const unsigned m = 255u << (8 * q), at = (unsigned)e << (8 * q);
+        const bool fresh = (count & m) == 0u;
+        count += 1u << (8 * q);
+        if (fresh || Flo[e] < Flo[byte_of(cR, q)]) cR = (cR & ~m) | at;
+        if (fresh || Fhi[e] < Fhi[byte_of(cL, q)]) cL = (cL & ~m) | at;
+    }
+    int res = -2;
+    if (!bad) {
+        // stable partition
+        unsigned off = (count << 8) + (count << 16) + (count << 24);  // cells of the buckets before, a byte each
+        const unsigned before = off;
+        const int m = (byte_of(count, 0) > 0) + (byte_of(count, 1) > 0) + (byte_of(count, 2) > 0) +
+                      (byte_of(count, 3) > 0);
+        if (m > 1) {
+            for (int i = 0; i < n; i++) {
+                const int q = (int)((codes >> (2 * i)) & 3u);
+                S.tmp[p + byte_of(off, q)] = S.perm[p + i];
+                off += 1u << (8 * q);
+            }
+            for (int i = 0; i < n; i++) S.perm[p + i] = S.tmp[p + i];
+        }
+        if (cpl == 1 && n == 2) {
+            *cmax = eL;
+            *cmin = eR;
+            res = 1;
+        } else if (m == 1) {
+            res = v.turned ? 0 : -1;
+        } else {
+            // split_plane as in warp_decide: float32 costs, float64 ones where
+            // two are too close
+            int plane = -1, prev = -1, near = 0;
+            bool ok = true;
+            float c32[4], cmin32 = FLT_MAX;
+            const float fbl = (float)bl;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                c32[k] = FLT_MAX;
+                if (byte_of(count, k) > 0) {
+                    if (prev >= 0 && m == 2) plane = k;
+                    if (prev >= 0 && m > 2) {
+                        const double dl = sub_value(1, Fhi[byte_of(cL, prev)]) - R, dr = Lr - sub_value(0, Flo[byte_of(cR, k)]);
+                        const float fl = (float)dl, fr = (float)dr;
+                        const float vl = fl / fbl, vr = fr / fbl;
+                        const bool z = fbl > 1e-30f && fbl < 1e30f && (dl == 0.0 || (fl >= 1e-30f && vl >= 1e-30f)) &&
+                                       (dr == 0.0 || (fr >= 1e-30f && vr >= 1e-30f));
+                        const int nL = byte_of(before, k);
+                        c32[k] = vl * (float)nL + vr * (float)(n - nL);
+                        ok = ok && z && c32[k] < 1e30f;
+                        cmin32 = fminf(cmin32, c32[k]);
+                    }
+                    prev = k;
+                }
+            }
+            if (m > 2 && ok) {
+                const float u = 5.9604644775390625e-08f;
+                int last = -1;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (c32[k] < FLT_MAX && c32[k] <= cmin32 * (1.0f + 32.0f * u) + 1e-37f) {
+                        last = k;
+                        near++;
+                    }
+                if (near == 1) plane = last;
+            }
+            if (plane < 0) {
+                unsigned long long kmin = ~0ull;
+                prev = -1;
+                for (int k = 0; k < 4; k++) {
+                    if (byte_of(count, k) > 0) {
+                        if (prev >= 0) {
+                            const int nL = byte_of(before, k);
+                            const double left_volume = (sub_value(1, Fhi[byte_of(cL, prev)]) - R) / bl;
+                            const double right_volume = (Lr - sub_value(0, Flo[byte_of(cR, k)])) / bl;
+                            const double cost = left_volume * exact_i2d(nL) + right_volume * exact_i2d(n - nL);
+                            if (!is_nan_bits(cost) && fkey(cost) < fkey(DBL_MAX) && fkey(cost) < kmin) {
+                                kmin = fkey(cost);
+                                plane = k;
+                            }
+                        }
+                        prev = k;
+                    }
+                }
+            }
+            if (plane >= 0) {
+                int bl_c = -1, br_c = -1;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (byte_of(count, k) > 0) {
+                        const int el = byte_of(cL, k), er = byte_of(cR, k);
+                        if (k < plane && (bl_c < 0 || Fhi[el] < Fhi[bl_c])) bl_c = el;
+                        if (k >= plane && (br_c < 0 || Flo[er] < Flo[br_c])) br_c = er;
+                    }
+                }
+                *cmax = bl_c;
+                *cmin = br_c;
+                res = byte_of(before, plane);
+            }
+        }
+    }
+    return res;
+}
+
+// Appends the lanes' nodes (`have`) of more than cpl cells to the list.
+__device__ __forceinline__ void sub_append(unsigned long long* list, int* n, bool have, const SubNode& v) {
+    const unsigned b = __ballot_sync(0xffffffffu, have);
+    if (have) list[*n + __popc(b & lanemask_lt())] = sub_pack(v);
+    *n += __popc(b);
 }
 
 template <bool LOOP>
-__global__ void __launch_bounds__(SUB_WARPS * 32) k_subtree(WS ws, int NB, long long cpl) {
+__global__ void __launch_bounds__(SUB_WARPS * 32, 10) k_subtree(WS ws, int NB, long long cpl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const unsigned FULL = 0xffffffffu;
     int lane = threadIdx.x & 31;
@@ -884,220 +1222,155 @@ __global__ void __launch_bounds__(SUB_WARPS * 32) k_subtree(WS ws, int NB, long 
     SubSmem& S = reinterpret_cast<SubSmem*>(smem_raw)[w];
     const int nsmall = ws.cnt->small_count;
     const int step = LOOP ? (int)gridDim.x * SUB_WARPS : INT32_MAX / 2;
+    const int tiny = NB == 4 ? SUB_TINY : 0;
     for (int sidx = blockIdx.x * SUB_WARPS + w; sidx < nsmall; sidx += step) {
-    __syncwarp();
-    int r = ws.small_list[sidx];
-    ARec* RR = &ws.recs[r];
-    int p0 = RR->ptr, s = RR->size, par = RR->parity, d0 = RR->dim, lvl = RR->level;
-    for (int i = lane; i < s; i += 32) {
-        for (int k = 0; k < 4; k++) S.F[k][i] = ws.f[par][k][p0 + i];
-        S.gid[i] = ws.idx[par][p0 + i];
-        S.perm[i] = (unsigned short)i;
-    }
-    LRec* L = ws.lrec + 2 * (size_t)p0;
-    if (lane == 0) {
-        LRec z;
-        z.Lmax = -1.0;
-        z.Rmin = -1.0;
-        z.child = -1;
-        z.ptr = p0;
-        z.size = s;
-        z.dim = d0;
-        L[0] = z;
-        sub_push(S, 0, 0, 0, s, d0, lvl);
-    }
-    __syncwarp();
-    int sp = 1, nloc = 1, maxd = lvl;
-    bool err = false;
-    while (sp > 0) {
-        sp--;
-        int v = S.stk_v[sp], p = S.stk_p[sp], n = S.stk_n[sp], flag = S.stk_flag[sp], depth = S.stk_depth[sp];
         __syncwarp();
-        int d = flag < 0 ? flag + 2 : flag;
-        if ((long long)n <= cpl) continue;
-        // get_bounds of the node (creation.py:271-277)
-        double R = warp_range_extreme(S, 2 * d, false, p, n);
-        double Lr = warp_range_extreme(S, 2 * d + 1, true, p, n);
-        double bl = bucket_len(Lr, R, NB);
-        for (int j = lane; j <= NB; j += 32) S.K[j] = fkey(bucket_edge(j, bl, R));  // NB + 1 edges
-        if (lane < NB) {
-            S.cnt[lane] = 0;
-            S.brun[lane] = 0;
-        }
-        __syncwarp();
-        bool lbad = false;
-        for (int i = lane; i < n; i += 32) {
-            const int e = S.perm[p + i];
-            int b = find_bucket(S.K, NB, fkey(centroid_of(S.F[2 * d][e], S.F[2 * d + 1][e])));
-            if (b < 0) {
-                lbad = true;
-                b = 0;
+        ARec* RR = &ws.recs[ws.small_list[sidx]];
+        const int p0 = RR->ptr, s = RR->size, par = RR->parity, d0 = RR->dim, lvl = RR->level;
+        for (int i = lane; i < s; i += 32) {
+#pragma unroll
+            for (int d = 0; d < 2; d++) {
+                const double lo = ws.f[par][2 * d][p0 + i], hi = ws.f[par][2 * d + 1][p0 + i];
+                S.F[2 * d][i] = fkey(lo);
+                S.F[2 * d + 1][i] = ~fkey(hi);
+                S.C[d][i] = fkey(centroid_of(lo, hi));
             }
-            S.bkt[i] = (unsigned char)b;
-            atomicAdd(&S.cnt[b], 1);
+            S.perm[i] = (unsigned char)i;
         }
-        if (__any_sync(FULL, lbad)) {
-            err = true;
-            continue;  // upstream indexes past its buckets; keep a leaf
-        }
-        __syncwarp();
-        if (lane < 32) {
-            int c = lane < NB ? S.cnt[lane] : 0;
-            int incl = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += t;
+        for (int i = lane; i < SMALL; i += 32) S.gn[i] = 0;
+        SubNode v = {0, s, d0, 0, 0, SUB_ROOT, 0, 0};
+        int nbig = 0, cur = 0, ncur = 0, nnext = 0, deepest = 0;
+        bool err = false;
+        if (lane == 0) S.root = SUB_LEAF;
+        if ((long long)s > cpl) {
+            if (s > tiny) {
+                if (lane == 0) S.big[0] = sub_pack(v);
+                nbig = 1;
+            } else {
+                if (lane == 0) S.tiny[0][0] = sub_pack(v);
+                ncur = 1;
             }
-            if (lane < NB) S.bstart[lane] = incl - c;
         }
         __syncwarp();
-        // stable partition (stable_partition / sort_bbox_indices creation.py:54-150)
-        for (int c0 = 0; c0 < n; c0 += 32) {
-            int i = c0 + lane;
-            int b = i < n ? (int)S.bkt[i] : 255;
-            unsigned grp = __match_any_sync(FULL, b);
-            int rank = __popc(grp & lanemask_lt());
-            if (i < n) {
-                const int dst = S.bstart[b] + S.brun[b] + rank;
-                S.tmp[dst] = S.perm[p + i];
-                S.nbkt[dst] = (unsigned char)b;
+        while (nbig > 0) {
+            v = sub_unpack(S.big[--nbig]);
+            __syncwarp();
+            int cmax = 0, cmin = 0;
+            const int nl = sub_node_warp(S, v, NB, cpl, &cmax, &cmin);
+            if (nl == -2) err = true;
+            if (nl == -1) {  // once more, in the other dimension
+                v.d = 1 - v.d;
+                v.turned = 1;
+                if (lane == 0) S.big[nbig] = sub_pack(v);
+                nbig++;
+            }
+            if (lane == 0 && nl > 0) sub_split(S, v, nl, cmax, cmin);
+            if (lane == 0 && nl <= 0 && v.turned) sub_state(S, v, SUB_TURNED);
+            if (nl > 0) {
+                deepest = max(deepest, v.depth + 1);
+                const SubNode c = sub_child(v, nl, lane & 1);
+                const bool open = lane < 2 && (long long)c.n > cpl;
+                sub_append(S.big, &nbig, open && c.n > tiny, c);
+                sub_append(S.tiny[0], &ncur, open && c.n <= tiny, c);
             }
             __syncwarp();
-            if (i < n && (int)(__ffs(grp) - 1) == lane) S.brun[b] += __popc(grp);
-            __syncwarp();
         }
-        for (int i = lane; i < n; i += 32) S.perm[p + i] = S.tmp[i];
-        __syncwarp();
-        // special case creation.py:311-320
-        if (cpl == 1 && n == 2) {
-            if (lane == 0) {
-                L[v].Lmax = Lr;
-                L[v].Rmin = R;
-                L[v].child = nloc;
-                LRec a;
-                a.Lmax = -1.0;
-                a.Rmin = -1.0;
-                a.child = -1;
-                a.size = 1;
-                a.dim = 1 - d;
-                a.ptr = p0 + p;
-                L[nloc] = a;
-                a.ptr = p0 + p + 1;
-                L[nloc + 1] = a;
-            }
-            nloc += 2;
-            maxd = max(maxd, depth + 1);
-            __syncwarp();
-            continue;
-        }
-        // per-bucket bounds (creation.py:300-306): the first-occurrence
-        // minimum of Rmin and maximum of Lmax of every bucket in one pass over
-        // the node's positions (after the partition bucket b is a contiguous
-        // run).  The lanes of one bucket reduce (key, position) together and
-        // their first lane folds the result into the bucket's running minimum
-        // (a later chunk never wins a tie: first occurrence).  Keys and
-        // positions use scratch the partition is done with: S.K (Rmin keys),
-        // S.bLmax viewed as keys (Lmax), S.brun / S.bstart (positions).
-        {
-            unsigned long long* kR = S.K;
-            unsigned long long* kL = reinterpret_cast<unsigned long long*>(S.bLmax);
-            if (lane < NB) {
-                kR[lane] = ~0ull;
-                kL[lane] = ~0ull;
-                S.brun[lane] = S.bstart[lane];  // positions when every key of the bucket ties at ~0
-            }
-            __syncwarp();
-            for (int c0 = 0; c0 < n; c0 += 32) {
-                const int i = c0 + lane;
-                int b = -1;
-                unsigned long long kr = ~0ull, kl = ~0ull;
-                if (i < n) {
-                    b = S.nbkt[i];
-                    const int e = S.perm[p + i];
-                    kr = fkey(S.F[2 * d][e]);
-                    kl = ~fkey(S.F[2 * d + 1][e]);
-                }
-                const unsigned grp = __match_any_sync(FULL, b);
-                unsigned long long mr, ml;
-                unsigned pr, pl;
-                group_min_kp(grp, kr, (unsigned)i, &mr, &pr);
-                group_min_kp(grp, kl, (unsigned)i, &ml, &pl);
-                if (b >= 0 && lane == (int)(__ffs(grp) - 1)) {
-                    if (mr < kR[b]) {
-                        kR[b] = mr;
-                        S.brun[b] = (int)pr;
-                    }
-                    if (ml < kL[b]) {
-                        kL[b] = ml;
-                        S.bstart[b] = (int)pl;
+        while (ncur > 0) {
+            nnext = 0;
+            for (int base = 0; base < ncur; base += 32) {
+                const bool have = base + lane < ncur;
+                int nl = 0, cmax = 0, cmin = 0;
+                v = sub_unpack(have ? S.tiny[cur][base + lane] : 0ull);
+                if (have) {
+                    nl = sub_node_lane(S, v, cpl, &cmax, &cmin);
+                    if (nl == -2) err = true;
+                    if (nl > 0) {
+                        sub_split(S, v, nl, cmax, cmin);
+                        deepest = max(deepest, v.depth + 1);
+                    } else if (nl != -1 && v.turned) {
+                        sub_state(S, v, SUB_TURNED);
                     }
                 }
                 __syncwarp();
-            }
-            if (lane < NB) {
-                const bool any = S.cnt[lane] > 0;
-                const double rmin = any ? S.F[2 * d][S.perm[p + S.brun[lane]]] : DBL_MAX;
-                const double lmax = any ? S.F[2 * d + 1][S.perm[p + S.bstart[lane]]] : -DBL_MAX;
-                S.bRmin[lane] = rmin;
-                S.bLmax[lane] = lmax;  // replaces this bucket's key
-            }
-            __syncwarp();
-        }
-        Decision D = warp_decide(S.cnt, S.bRmin, S.bLmax, NB, n, R, Lr, bl);
-        if (D.kind == 0) {
-            // all cells in one bucket (creation.py:345-358)
-            if (flag >= 0) {
-                if (lane == 0) {
-                    L[v].dim = 1 - L[v].dim;
-                    sub_push(S, sp, v, p, n, (1 - d) - 2, depth);
+                const SubNode l = sub_child(v, nl, 0), r = sub_child(v, nl, 1);
+                if (nl == -1) {
+                    v.d = 1 - v.d;
+                    v.turned = 1;
                 }
-                sp++;
-            } else if (lane == 0) {
-                L[v].Lmax = -1.0;
-                L[v].Rmin = -1.0;
+                sub_append(S.tiny[cur ^ 1], &nnext, nl == -1 || (nl > 0 && (long long)l.n > cpl), nl == -1 ? v : l);
+                sub_append(S.tiny[cur ^ 1], &nnext, nl > 0 && (long long)r.n > cpl, r);
             }
             __syncwarp();
-            continue;
+            cur ^= 1;
+            ncur = nnext;
         }
-        if (D.kind < 0) {
-            err = true;
-            continue;
-        }
-        int nl = D.nleft;
-        if (lane == 0) {
-            L[v].Lmax = D.Lmax;
-            L[v].Rmin = D.Rmin;
-            L[v].child = nloc;
-            LRec a;
-            a.Lmax = -1.0;
-            a.Rmin = -1.0;
-            a.child = -1;
-            a.dim = 1 - d;
-            a.ptr = p0 + p;
-            a.size = nl;
-            L[nloc] = a;
-            a.ptr = p0 + p + nl;
-            a.size = n - nl;
-            L[nloc + 1] = a;
-            // push right, then left (creation.py:378-379)
-            sub_push(S, sp, nloc + 1, p + nl, n - nl, 1 - d, depth + 1);
-            sub_push(S, sp + 1, nloc, p, nl, 1 - d, depth + 1);
-        }
-        sp += 2;
-        nloc += 2;
-        maxd = max(maxd, depth + 1);
         __syncwarp();
-    }
-    __syncwarp();
-    for (int i = lane; i < s; i += 32) ws.final_idx[p0 + i] = S.gid[S.perm[i]];
-    if (lane == 0) {
-        RR->splits = (nloc - 1) / 2;
-        RR->nlocal = nloc;
-        RR->err = err ? 1 : 0;
-        atomicMax(&ws.cnt->max_depth, maxd);
-        atomicMax(&ws.tree_depth[RR->tree], maxd);
-        if (err) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
-    }
+        // numbering: the splits as bits by gap
+        unsigned act[SMALL / 32];
+        int splits = 0;
+#pragma unroll
+        for (int k = 0; k < SMALL / 32; k++) {
+            act[k] = __ballot_sync(FULL, S.gn[k * 32 + lane] != 0);
+            splits += __popc(act[k]);
+        }
+        auto child_of = [&](int g) -> int {  // local number of the left child
+            const int p = S.gp[g];
+            int c = S.gleft[g];
+#pragma unroll
+            for (int k = 0; k < SMALL / 32; k++) {
+                const int b = p - 32 * k;
+                c += __popc(b >= 32 ? act[k] : b > 0 ? act[k] & ((1u << b) - 1u) : 0u);
+            }
+            return 1 + 2 * c;
+        };
+        LRec* L = ws.lrec + 2 * (size_t)p0;
+        if (lane == 0 && S.root != SUB_SPLIT) {
+            LRec z;
+            z.Lmax = -1.0;
+            z.Rmin = -1.0;
+            z.child = -1;
+            z.ptr = p0;
+            z.size = s;
+            z.dim = S.root == SUB_TURNED ? 1 - d0 : d0;
+            L[0] = z;
+        }
+        for (int g = lane; g < s; g += 32) {
+            if (S.gn[g] != 0) {
+                const int p = S.gp[g], n = S.gn[g], d = S.gflag[g] & 1, side = S.gflag[g] >> 1, gpar = S.gpar[g];
+                const int c = child_of(g);
+                LRec z;
+                z.Lmax = ws.f[par][2 * d + 1][p0 + S.gmax[g]];  // (the keys don't hold the sign of a zero)
+                z.Rmin = ws.f[par][2 * d][p0 + S.gmin[g]];
+                z.child = c;
+                z.ptr = p0 + p;
+                z.size = n;
+                z.dim = d;
+                L[gpar == SUB_ROOT ? 0 : child_of(gpar) + side] = z;
+                z.Lmax = -1.0;
+                z.Rmin = -1.0;
+                z.child = -1;
+                for (int k = 0; k < 2; k++) {
+                    const int state = S.gchild[k][g];
+                    if (state != SUB_SPLIT) {
+                        z.ptr = p0 + (k ? g + 1 : p);
+                        z.size = k ? p + n - 1 - g : g + 1 - p;
+                        z.dim = state == SUB_TURNED ? d : 1 - d;
+                        L[c + k] = z;
+                    }
+                }
+            }
+        }
+        for (int i = lane; i < s; i += 32) ws.final_idx[p0 + i] = ws.idx[par][p0 + S.perm[i]];
+        deepest = __reduce_max_sync(FULL, deepest);
+        err = __any_sync(FULL, err);
+        if (lane == 0) {
+            RR->splits = splits;
+            RR->nlocal = 1 + 2 * splits;
+            RR->err = err ? 1 : 0;
+            atomicMax(&ws.cnt->max_depth, lvl + deepest);
+            atomicMax(&ws.tree_depth[RR->tree], lvl + deepest);
+            if (err) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
+        }
     }
 }
 
