@@ -40,12 +40,15 @@ namespace ct {
 
 constexpr int SMALL = 128;         // subtree size handled by one warp
 constexpr int NBMAX = 32;          // maximum n_buckets
-constexpr int STATS_THREADS = 256; // threads of the stats / scatter CTAs
+constexpr int STATS_THREADS = 256; // threads of the stats CTAs
+constexpr int SCAT_THREADS = 128;  // threads of the scatter CTAs
+constexpr int STATS4_THREADS = 64; // threads of the stats CTAs for 4 buckets
 constexpr int TILE_MIN = 2048;     // minimum cells per tile
-constexpr int MAX_TILES = 512;     // maximum tiles per node
+constexpr int MAX_TILES = 2048;    // maximum tiles per node
 constexpr int SUB_WARPS = 2;       // warps per CTA in the subtree kernel (10.5 KB of shared memory each)
 
-enum : int { K_PENDING = 0, K_SPLIT = 1, K_LEAF = 2, K_SUBTREE = 3 };
+// K_TURN: all cells in one bucket of the node's dimension, the other is next
+enum : int { K_PENDING = 0, K_SPLIT = 1, K_LEAF = 2, K_SUBTREE = 3, K_TURN = 4 };
 
 // Phase-A node record.
 struct ARec {
@@ -81,6 +84,7 @@ struct Counters {
     int root_zp[4];
     int done;    // device-driven level loop: no pending record left (or an error)
     int nlev;    // device-driven level loop: phase-A levels recorded in lvl_b / lvl_e
+    int turned;  // a node of this level needs its other dimension
 };
 
 // most phase-A levels the device-driven level loop runs (a balanced tree of
@@ -437,16 +441,19 @@ __global__ void k_root_resolve(WS ws, int n) {
 // phase A
 // ------------------------------------------------------------------------
 
-__device__ __forceinline__ int tile_len_for(int size) {
+// Cells per tile: TILE_MIN, fewer where a level has too few tiles for the GPU
+// (80k cells, 40 tiles of 2048 -> 160 of 512: stats and scatter 22 -> 15 us a
+// level).
+__device__ __forceinline__ int tile_len_for(int size, int n) {
     int t = (size + MAX_TILES - 1) / MAX_TILES;
-    if (t < TILE_MIN) t = TILE_MIN;
+    t = max(t, min(TILE_MIN, max(512, n / (152 * 8))));
     t = (t + STATS_THREADS - 1) / STATS_THREADS * STATS_THREADS;
     return t;
 }
 
 // One warp per record of the current level: make tiles for pending nodes and
 // reset their stats slots.
-__global__ void k_make_tiles(WS ws, int NB) {
+__global__ void k_make_tiles(WS ws, int NB, int n) {
     if (ws.cnt->done) return;
     int lb = ws.cnt->lb, le = ws.cnt->le;
     int lane = threadIdx.x & 31;
@@ -456,7 +463,7 @@ __global__ void k_make_tiles(WS ws, int NB) {
         ARec* R = &ws.recs[r];
         if (R->kind != K_PENDING) continue;
         int size = R->size;
-        int tl = tile_len_for(size);
+        int tl = tile_len_for(size, n);
         int nt = (size + tl - 1) / tl;
         int t0 = 0;
         if (lane == 0) t0 = atomicAdd(&ws.cnt->tile_count, nt);
@@ -483,102 +490,167 @@ __global__ void k_make_tiles(WS ws, int NB) {
     }
 }
 
-// Per tile: bucket membership in both dimensions; per (dim, bucket): count,
-// first-occurrence min of lo_x / lo_y and max of hi_x / hi_y (as min-form
-// keys) and the first position of a zero value.
+// Per tile: bucket membership in the dimensions asked for; per (dim, bucket):
+// count, first-occurrence min of lo_x / lo_y and max of hi_x / hi_y (as
+// min-form keys) and the first position of a zero value.
 // LOOP: the device-driven level loop's form -- a fixed grid walks the tiles
 // whose count the make-tiles pass left on the device.
-template <bool LOOP>
-__global__ void __launch_bounds__(STATS_THREADS) k_stats(WS ws, int parity, int NB) {
+// The dimensions: BOTH (the forest builds, whose levels are launched without
+// knowing whether a node needs its other one), the node's OWN, or the OTHER
+// one of the nodes that need it (K_TURN), in a second pass that finds none on
+// nearly every mesh.
+// NB4 (4 buckets, one dimension): each thread keeps the 16 extremes of its
+// cells in registers, combined once per tile; otherwise the lanes of a bucket
+// combine theirs for every 32 cells.  Both dimensions and a combination per
+// 32 cells took 424 instructions and 200 cycles of the float64 unit per 32
+// cells, 0.32 ms a level of 16M cells; now 0.15 to 0.19 (CTAs of 128 / 256
+// threads, fewer for the small nodes of the last levels: 0.19 / 0.23).
+enum { DIM_BOTH = 0, DIM_OWN = 1, DIM_OTHER = 2 };
+
+template <bool LOOP, int DIMS, bool NB4>
+__global__ void __launch_bounds__(NB4 ? STATS4_THREADS : STATS_THREADS, NB4 ? 12 : 1) k_stats(WS ws, int parity, int NB) {
     __shared__ unsigned long long K[2][NBMAX + 1];
     __shared__ unsigned int cnt[2][NBMAX];
     __shared__ unsigned long long key[2][NBMAX][4];
     __shared__ int zp[2][NBMAX][4];
     const unsigned FULL = 0xffffffffu;
+    const unsigned long long KZ = 0x8000000000000000ull;  // fkey(0)
+    if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
     const int nt = LOOP ? (ws.cnt->done ? 0 : ws.cnt->tile_count) : (int)gridDim.x;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-    if (LOOP) __syncthreads();  // the previous tile's readers are done with the shared arrays
-    int r = ws.tile_rec[t];
-    int s = ws.tile_start[t], e = ws.tile_end[t];
-    int lb = ws.cnt->lb;
-    const ARec* R = &ws.recs[r];
-    int tid = threadIdx.x;
-    for (int j = tid; j < 2 * NBMAX; j += blockDim.x) (&cnt[0][0])[j] = 0u;
-    for (int j = tid; j < 2 * NBMAX * 4; j += blockDim.x) {
-        (&key[0][0][0])[j] = ~0ull;
-        (&zp[0][0][0])[j] = INT32_MAX;
-    }
-    if (tid < 2 * (NB + 1)) {
-        int d = tid / (NB + 1), j = tid % (NB + 1);
-        double Rd = R->bnd[2 * d], Ld = R->bnd[2 * d + 1];
-        K[d][j] = fkey(bucket_edge(j, bucket_len(Ld, Rd, NB), Rd));
-    }
-    __syncthreads();
-    const double* F0 = ws.f[parity][0];
-    const double* F1 = ws.f[parity][1];
-    const double* F2 = ws.f[parity][2];
-    const double* F3 = ws.f[parity][3];
-    for (int base = s; base < e; base += blockDim.x) {
-        int i = base + tid;
-        bool valid = i < e;
-        double v0 = 0, v1 = 0, v2 = 0, v3 = 0, c0 = 0, c1 = 0;
-        if (valid) {
-            v0 = F0[i];
-            v1 = F1[i];
-            v2 = F2[i];
-            v3 = F3[i];
-            c0 = centroid_of(v0, v1);
-            c1 = centroid_of(v2, v3);
+        if (LOOP) __syncthreads();  // the previous tile's readers are done with the shared arrays
+        const int r = ws.tile_rec[t];
+        const int s = ws.tile_start[t], e = ws.tile_end[t];
+        const int lb = ws.cnt->lb;
+        const ARec* R = &ws.recs[r];
+        if (DIMS == DIM_OTHER && R->kind != K_TURN) continue;
+        const int d0 = DIMS == DIM_BOTH ? 0 : DIMS == DIM_OWN ? R->dim : 1 - R->dim;
+        const int d1 = DIMS == DIM_BOTH ? 2 : d0 + 1;
+        const int tid = threadIdx.x;
+        for (int j = tid; j < 2 * NBMAX; j += blockDim.x) (&cnt[0][0])[j] = 0u;
+        for (int j = tid; j < 2 * NBMAX * 4; j += blockDim.x) {
+            (&key[0][0][0])[j] = ~0ull;
+            (&zp[0][0][0])[j] = INT32_MAX;
         }
-        unsigned long long k0 = fkey(v0), k1 = ~fkey(v1), k2 = fkey(v2), k3 = ~fkey(v3);
+        if (tid < 2 * (NB + 1)) {
+            int d = tid / (NB + 1), j = tid % (NB + 1);
+            double Rd = R->bnd[2 * d], Ld = R->bnd[2 * d + 1];
+            K[d][j] = fkey(bucket_edge(j, bucket_len(Ld, Rd, NB), Rd));
+        }
+        __syncthreads();
+        const double* F0 = ws.f[parity][0];
+        const double* F1 = ws.f[parity][1];
+        const double* F2 = ws.f[parity][2];
+        const double* F3 = ws.f[parity][3];
+        if (NB4) {
+            const unsigned long long E0 = K[d0][0], E1 = K[d0][1], E2 = K[d0][2], E3 = K[d0][3], E4 = K[d0][4];
+            unsigned long long m[4][4], count = 0;  // count: 16 bits a bucket (a thread has at most 2^15 cells)
 #pragma unroll
-        for (int d = 0; d < 2; d++) {
-            int b = -2;
-            if (valid) {
-                b = find_bucket(K[d], NB, fkey(d ? c1 : c0));
-                if (b < 0) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
+            for (int b = 0; b < 4; b++)
+#pragma unroll
+                for (int f = 0; f < 4; f++) m[b][f] = ~0ull;
+            double n0 = 0, n1 = 0, n2 = 0, n3 = 0;  // the next cell's, loaded while this one is counted
+            if (s + tid < e) {
+                n0 = F0[s + tid];
+                n1 = F1[s + tid];
+                n2 = F2[s + tid];
+                n3 = F3[s + tid];
             }
-            unsigned grp = __match_any_sync(FULL, b);
-            if (b >= 0) {
-                unsigned long long m0 = group_min_k(grp, k0);
-                unsigned long long m1 = group_min_k(grp, k1);
-                unsigned long long m2 = group_min_k(grp, k2);
-                unsigned long long m3 = group_min_k(grp, k3);
-                if ((int)(__ffs(grp) - 1) == (tid & 31)) {
-                    atomicAdd(&cnt[d][b], (unsigned)__popc(grp));
-                    atomicMin(&key[d][b][0], m0);
-                    atomicMin(&key[d][b][1], m1);
-                    atomicMin(&key[d][b][2], m2);
-                    atomicMin(&key[d][b][3], m3);
+            for (int i = s + tid; i < e; i += STATS4_THREADS) {
+                const double v0 = n0, v1 = n1, v2 = n2, v3 = n3;
+                const int j = i + STATS4_THREADS;
+                if (j < e) {
+                    n0 = F0[j];
+                    n1 = F1[j];
+                    n2 = F2[j];
+                    n3 = F3[j];
                 }
-                if (is_zero(v0)) atomicMin(&zp[d][b][0], i);
-                if (is_zero(v1)) atomicMin(&zp[d][b][1], i);
-                if (is_zero(v2)) atomicMin(&zp[d][b][2], i);
-                if (is_zero(v3)) atomicMin(&zp[d][b][3], i);
+                const unsigned long long kc = fkey(d0 ? centroid_of(v2, v3) : centroid_of(v0, v1));
+                const unsigned long long k[4] = {fkey(v0), ~fkey(v1), fkey(v2), ~fkey(v3)};
+                const bool in = kc >= E0 && kc < E4;
+                const int b = E2 <= kc ? (E3 <= kc ? 3 : 2) : (E1 <= kc ? 1 : 0);  // find_bucket
+                if (!in) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
+                count += in ? 1ull << (16 * b) : 0ull;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+#pragma unroll
+                    for (int f = 0; f < 4; f++) m[q][f] = (in && b == q && k[f] < m[q][f]) ? k[f] : m[q][f];
+                }
+                if (in && (k[0] == KZ || k[1] == ~KZ || k[2] == KZ || k[3] == ~KZ)) {
+#pragma unroll
+                    for (int f = 0; f < 4; f++)
+                        if (k[f] == ((f & 1) ? ~KZ : KZ)) atomicMin(&zp[d0][b][f], i);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const unsigned c = __reduce_add_sync(FULL, (unsigned)((count >> (16 * b)) & 0xffffull));
+                if (c) {
+                    if ((tid & 31) == 0) atomicAdd(&cnt[d0][b], c);
+#pragma unroll
+                    for (int f = 0; f < 4; f++) {
+                        const unsigned long long x = group_min_k(FULL, m[b][f]);
+                        if ((tid & 31) == f) atomicMin(&key[d0][b][f], x);
+                    }
+                }
+            }
+        } else {
+            for (int base = s; base < e; base += blockDim.x) {
+                int i = base + tid;
+                bool valid = i < e;
+                double v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+                if (valid) {
+                    v0 = F0[i];
+                    v1 = F1[i];
+                    v2 = F2[i];
+                    v3 = F3[i];
+                }
+                const unsigned long long k[4] = {fkey(v0), ~fkey(v1), fkey(v2), ~fkey(v3)};
+                for (int d = d0; d < d1; d++) {
+                    int b = -2;
+                    if (valid) {
+                        b = find_bucket(K[d], NB, fkey(d ? centroid_of(v2, v3) : centroid_of(v0, v1)));
+                        if (b < 0) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
+                    }
+                    unsigned grp = __match_any_sync(FULL, b);
+                    if (b >= 0) {
+                        unsigned long long m[4];
+#pragma unroll
+                        for (int f = 0; f < 4; f++) m[f] = group_min_k(grp, k[f]);
+                        if ((int)(__ffs(grp) - 1) == (tid & 31)) {
+                            atomicAdd(&cnt[d][b], (unsigned)__popc(grp));
+#pragma unroll
+                            for (int f = 0; f < 4; f++) atomicMin(&key[d][b][f], m[f]);
+                        }
+#pragma unroll
+                        for (int f = 0; f < 4; f++)
+                            if (k[f] == ((f & 1) ? ~KZ : KZ)) atomicMin(&zp[d][b][f], i);
+                    }
+                }
             }
         }
-    }
-    __syncthreads();
-    size_t sidx = (size_t)(r - lb);
-    for (int j = tid; j < 2 * NB; j += blockDim.x) {
-        int d = j / NB, b = j % NB;
-        unsigned c = cnt[d][b];
-        ws.tile_cnt[(size_t)t * 2 * NB + j] = c;
-        if (c) atomicAdd(&ws.st_cnt[sidx * 2 * NB + j], c);
-    }
-    for (int j = tid; j < 2 * NB * 4; j += blockDim.x) {
-        int d = j / (NB * 4), b = (j / 4) % NB, f = j % 4;
-        if (cnt[d][b]) {
-            atomicMin(&ws.st_key[sidx * 2 * NB * 4 + j], key[d][b][f]);
-            if (zp[d][b][f] != INT32_MAX) atomicMin(&ws.st_zp[sidx * 2 * NB * 4 + j], zp[d][b][f]);
+        __syncthreads();
+        size_t sidx = (size_t)(r - lb);
+        for (int j = d0 * NB + tid; j < d1 * NB; j += blockDim.x) {
+            int d = j / NB, b = j % NB;
+            unsigned c = cnt[d][b];
+            ws.tile_cnt[(size_t)t * 2 * NB + j] = c;
+            if (c) atomicAdd(&ws.st_cnt[sidx * 2 * NB + j], c);
         }
-    }
+        for (int j = d0 * NB * 4 + tid; j < d1 * NB * 4; j += blockDim.x) {
+            int d = j / (NB * 4), b = (j / 4) % NB, f = j % 4;
+            if (cnt[d][b]) {
+                atomicMin(&ws.st_key[sidx * 2 * NB * 4 + j], key[d][b][f]);
+                if (zp[d][b][f] != INT32_MAX) atomicMin(&ws.st_zp[sidx * 2 * NB * 4 + j], zp[d][b][f]);
+            }
+        }
     }
 }
 
 // One warp per record of the current level: the upstream split decision for
-// pending nodes, children records, bucket bases and tile prefixes.
-template <bool LOOP>
+// pending nodes, children records, bucket bases and tile prefixes.  DIMS: the
+// dimensions k_stats has looked at.
+template <bool LOOP, int DIMS>
 __global__ void k_decide(WS ws, int NB, long long cpl) {
     __shared__ int s_cnt[4][2][NBMAX];
     __shared__ double s_Rmin[4][2][NBMAX];
@@ -587,17 +659,20 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     int lane = threadIdx.x & 31;
     int w = threadIdx.x >> 5;  // blockDim = 128
     if (LOOP && ws.cnt->done) return;
+    if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
     int lb = ws.cnt->lb, le = ws.cnt->le;
     const int step = LOOP ? (int)gridDim.x * 4 : INT32_MAX / 2;
     for (int r = lb + blockIdx.x * 4 + w; r < le; r += step) {
     __syncwarp();
     ARec* R = &ws.recs[r];
-    if (R->kind != K_PENDING) continue;
+    if (R->kind != (DIMS == DIM_OTHER ? K_TURN : K_PENDING)) continue;
     int parity = R->parity;
     size_t sidx = (size_t)(r - lb);
     int size = R->size, ptr = R->ptr;
-    // resolve per-bucket bounds of both dimensions
-    for (int j = lane; j < 2 * NB; j += 32) {
+    int d0 = R->dim;
+    // resolve the per-bucket bounds
+    const int dj = DIMS == DIM_BOTH ? 0 : DIMS == DIM_OWN ? d0 : 1 - d0;
+    for (int j = dj * NB + lane; j < (DIMS == DIM_BOTH ? 2 : dj + 1) * NB; j += 32) {
         int d = j / NB, b = j % NB;
         int c = (int)ws.st_cnt[sidx * 2 * NB + j];
         s_cnt[w][d][b] = c;
@@ -612,7 +687,6 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
         s_Lmax[w][d][b] = lmax;
     }
     __syncwarp();
-    int d0 = R->dim;
     int stored_dim = d0;
     int ds = -1;
     Decision D;
@@ -621,7 +695,8 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     if ((long long)size <= cpl) {
         D.kind = 2;  // leaf (creation.py:267)
     } else {
-        for (int attempt = 0; attempt < 2; attempt++) {
+        for (int attempt = DIMS == DIM_OTHER ? 1 : 0; attempt < 2; attempt++) {
+            if (attempt == 1) stored_dim = 1 - d0;
             int d = attempt == 0 ? d0 : 1 - d0;
             int tot = 0;
             for (int b = 0; b < NB; b++) tot += s_cnt[w][d][b];
@@ -641,9 +716,16 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
                 break;
             }
             // all cells in one bucket: flip the stored dim once, then give up
-            if (attempt == 0) stored_dim = 1 - d0;
-            else D.kind = 2;
+            if (attempt == 1) D.kind = 2;
+            if (DIMS == DIM_OWN) break;
         }
+    }
+    if (DIMS == DIM_OWN && !bad && D.kind == 0) {
+        if (lane == 0) {
+            R->kind = K_TURN;
+            ws.cnt->turned = 1;
+        }
+        continue;
     }
     if (bad) {
         if (lane == 0) atomicOr(&ws.cnt->err, CT_DEVERR_BUCKET);
@@ -674,24 +756,25 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     int rb = D.rbucket;
     // child bounds: first occurrence over the child's buckets in order
     size_t kb0 = sidx * 2 * NB * 4 + (size_t)ds * NB * 4;
-    double cb[2][4];
-    for (int f = 0; f < 4; f++) {
-        for (int side = 0; side < 2; side++) {
-            int b0 = side ? rb : 0, b1 = side ? NB : rb;
-            unsigned long long best = ~0ull;
-            int bb = -1;
-            for (int b = b0; b < b1; b++) {
-                if (s_cnt[w][ds][b] == 0) continue;
-                unsigned long long k = ws.st_key[kb0 + (size_t)b * 4 + f];
-                if (k < best) {
-                    best = k;
-                    bb = b;
-                }
+    double cb = 0.0;  // of lane f + 4 * side
+    if (lane < 8) {
+        const int f = lane & 3, side = lane >> 2;
+        int b0 = side ? rb : 0, b1 = side ? NB : rb;
+        unsigned long long best = ~0ull;
+        int bb = -1;
+        for (int b = b0; b < b1; b++) {
+            const unsigned long long k = ws.st_key[kb0 + (size_t)b * 4 + f];
+            if (s_cnt[w][ds][b] != 0 && k < best) {
+                best = k;
+                bb = b;
             }
-            cb[side][f] = (bb < 0) ? ((f & 1) ? -DBL_MAX : DBL_MAX)
-                                   : resolve_key(best, f, ws.st_zp[kb0 + (size_t)bb * 4 + f], ws.f[parity][f]);
         }
+        cb = (bb < 0) ? ((f & 1) ? -DBL_MAX : DBL_MAX)
+                      : resolve_key(best, f, ws.st_zp[kb0 + (size_t)bb * 4 + f], ws.f[parity][f]);
     }
+    double cbnd[4];
+#pragma unroll
+    for (int f = 0; f < 4; f++) cbnd[f] = __shfl_sync(FULL, cb, f + 4 * (lane & 1));
     int child_dim = 1 - ds;
     if (lane < 2) {
         ARec ch;
@@ -706,7 +789,7 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
         ch.split_dim = -1;
         ch.Lmax = -1.0;
         ch.Rmin = -1.0;
-        for (int f = 0; f < 4; f++) ch.bnd[f] = cb[lane][f];
+        for (int f = 0; f < 4; f++) ch.bnd[f] = cbnd[f];
         ch.kind = (ch.size > SMALL) ? K_PENDING : K_SUBTREE;
         ws.recs[c + lane] = ch;
         if (ch.kind == K_SUBTREE) {
@@ -736,6 +819,38 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     int nt = t1 - t0;
     int per = (nt + 31) / 32;
     int my0 = t0 + lane * per, my1 = min(t0 + (lane + 1) * per, t1);
+    if (NB == 4) {  // the four buckets at once
+        const int4* in = reinterpret_cast<const int4*>(ws.tile_cnt) + ds;
+        int4* out = reinterpret_cast<int4*>(ws.tile_pref);
+        int a[4] = {0, 0, 0, 0};
+#pragma unroll 4
+        for (int t = my0; t < my1; t++) {
+            const int4 c = in[2 * (size_t)t];
+            a[0] += c.x;
+            a[1] += c.y;
+            a[2] += c.z;
+            a[3] += c.w;
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            int incl = a[b];
+            for (int o = 1; o < 32; o <<= 1) {
+                int v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += v;
+            }
+            a[b] = incl - a[b];
+        }
+#pragma unroll 4
+        for (int t = my0; t < my1; t++) {
+            const int4 c = in[2 * (size_t)t];
+            out[t] = make_int4(a[0], a[1], a[2], a[3]);
+            a[0] += c.x;
+            a[1] += c.y;
+            a[2] += c.z;
+            a[3] += c.w;
+        }
+        continue;
+    }
     for (int b = 0; b < NB; b++) {
         int sum = 0;
         for (int t = my0; t < my1; t++) sum += (int)ws.tile_cnt[(size_t)t * 2 * NB + ds * NB + b];
@@ -754,68 +869,101 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
 }
 
 // Per tile: stable partition of split nodes into the other buffer; leaf cells
-// go straight to their final position.
+// go straight to their final position.  A round takes SCAT_IPT cells per
+// thread: their loads are in flight together, and the warps' bucket counts are
+// scanned once for all.  One cell per thread and round, 3 barriers per 256
+// cells: 250 us a level of 16M cells; now 180 (CTAs of 64 / 256 threads 187 /
+// 195, and twice that on the last levels of 256), 170 at the copy rate.
+constexpr int SCAT_IPT = 4;
+
 template <bool LOOP>
-__global__ void __launch_bounds__(STATS_THREADS) k_scatter(WS ws, int parity, int NB) {
+__global__ void __launch_bounds__(SCAT_THREADS) k_scatter(WS ws, int parity, int NB) {
     __shared__ unsigned long long K[NBMAX + 1];
     __shared__ int base[NBMAX];
-    __shared__ int run[NBMAX];
-    __shared__ int wcnt[STATS_THREADS / 32][NBMAX];
+    constexpr int SCAT_WARPS = SCAT_THREADS / 32, ROWS = SCAT_IPT * SCAT_WARPS;
+    static_assert(ROWS <= 32, "a lane per (round's part, warp)");
+    __shared__ int first[ROWS][NBMAX];  // cells of (part, warp) per bucket, then where the first goes
     const unsigned FULL = 0xffffffffu;
     const int nt = LOOP ? (ws.cnt->done ? 0 : ws.cnt->tile_count) : (int)gridDim.x;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-    if (LOOP) __syncthreads();
-    int r = ws.tile_rec[t];
-    int s = ws.tile_start[t], e = ws.tile_end[t];
-    int lb = ws.cnt->lb;
-    const ARec* R = &ws.recs[r];
-    int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int* idx_in = ws.idx[parity];
-    if (R->kind != K_SPLIT) {
-        for (int i = s + tid; i < e; i += blockDim.x) ws.final_idx[i] = idx_in[i];
-        continue;
-    }
-    int ds = R->split_dim;
-    size_t sidx = (size_t)(r - lb);
-    if (tid <= NB) {
-        double Rd = R->bnd[2 * ds], Ld = R->bnd[2 * ds + 1];
-        K[tid] = fkey(bucket_edge(tid, bucket_len(Ld, Rd, NB), Rd));
-    }
-    if (tid < NB) {
-        base[tid] = ws.nb_base[sidx * NB + tid] + ws.tile_pref[(size_t)t * NB + tid];
-        run[tid] = 0;
-    }
-    __syncthreads();
-    const double* Lo = ws.f[parity][2 * ds];
-    const double* Hi = ws.f[parity][2 * ds + 1];
-    for (int b0 = s; b0 < e; b0 += blockDim.x) {
-        int i = b0 + tid;
-        bool valid = i < e;
-        int b = valid ? find_bucket(K, NB, fkey(centroid_of(Lo[i], Hi[i]))) : -2;
-        if (valid && b < 0) b = -1;  // counted nowhere: flagged by k_stats
-        unsigned grp = __match_any_sync(FULL, b);
-        int rank = __popc(grp & lanemask_lt());
-        for (int j = tid; j < (STATS_THREADS / 32) * NBMAX; j += blockDim.x) (&wcnt[0][0])[j] = 0;
+        if (LOOP) __syncthreads();
+        int r = ws.tile_rec[t];
+        int s = ws.tile_start[t], e = ws.tile_end[t];
+        int lb = ws.cnt->lb;
+        const ARec* R = &ws.recs[r];
+        const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+        const int* idx_in = ws.idx[parity];
+        if (R->kind != K_SPLIT) {
+            for (int i = s + tid; i < e; i += blockDim.x) ws.final_idx[i] = idx_in[i];
+            continue;
+        }
+        const int ds = R->split_dim, op = 1 - parity;
+        size_t sidx = (size_t)(r - lb);
+        for (int j = tid; j <= NB; j += SCAT_THREADS) {
+            double Rd = R->bnd[2 * ds], Ld = R->bnd[2 * ds + 1];
+            K[j] = fkey(bucket_edge(j, bucket_len(Ld, Rd, NB), Rd));
+        }
+        if (tid < NB) base[tid] = ws.nb_base[sidx * NB + tid] + ws.tile_pref[(size_t)t * NB + tid];
         __syncthreads();
-        if (b >= 0 && (int)(__ffs(grp) - 1) == lane) wcnt[w][b] = __popc(grp);
-        __syncthreads();
-        int off = 0;
-        if (b >= 0) {
-            for (int ww = 0; ww < w; ww++) off += wcnt[ww][b];
-            int dst = base[b] + run[b] + off + rank;
-            int op = 1 - parity;
+        const double* Lo = ws.f[parity][2 * ds];
+        const double* Hi = ws.f[parity][2 * ds + 1];
+        const double* Lo2 = ws.f[parity][2 - 2 * ds];
+        const double* Hi2 = ws.f[parity][3 - 2 * ds];
+        for (int b0 = s; b0 < e; b0 += SCAT_THREADS * SCAT_IPT) {
+            double lo[SCAT_IPT], hi[SCAT_IPT], lo2[SCAT_IPT], hi2[SCAT_IPT];
+            int id[SCAT_IPT], b[SCAT_IPT], rank[SCAT_IPT];
 #pragma unroll
-            for (int k = 0; k < 4; k++) ws.f[op][k][dst] = ws.f[parity][k][i];
-            ws.idx[op][dst] = idx_in[i];
+            for (int k = 0; k < SCAT_IPT; k++) {
+                const int i = b0 + k * SCAT_THREADS + tid;
+                lo[k] = hi[k] = lo2[k] = hi2[k] = 0.0;
+                id[k] = 0;
+                if (i < e) {
+                    lo[k] = Lo[i];
+                    hi[k] = Hi[i];
+                    lo2[k] = Lo2[i];
+                    hi2[k] = Hi2[i];
+                    id[k] = idx_in[i];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < SCAT_IPT; k++) {
+                const bool valid = b0 + k * SCAT_THREADS + tid < e;
+                b[k] = valid ? find_bucket(K, NB, fkey(centroid_of(lo[k], hi[k]))) : -2;
+                if (valid && b[k] < 0) b[k] = -1;  // counted nowhere: flagged by k_stats
+                const unsigned grp = __match_any_sync(FULL, b[k]);
+                rank[k] = __popc(grp & lanemask_lt());
+                int* row = first[k * SCAT_WARPS + w];
+                if (lane < NB) row[lane] = 0;
+                __syncwarp();
+                if (b[k] >= 0 && rank[k] == 0) row[b[k]] = __popc(grp);
+            }
+            __syncthreads();
+            for (int q = w; q < NB; q += SCAT_WARPS) {
+                const int c = lane < ROWS ? first[lane][q] : 0;
+                int incl = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int at = base[q];
+                __syncwarp();
+                if (lane < ROWS) first[lane][q] = at + incl - c;
+                if (lane == 31) base[q] = at + incl;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < SCAT_IPT; k++) {
+                if (b[k] >= 0) {
+                    const int dst = first[k * SCAT_WARPS + w][b[k]] + rank[k];
+                    ws.f[op][2 * ds][dst] = lo[k];
+                    ws.f[op][2 * ds + 1][dst] = hi[k];
+                    ws.f[op][2 - 2 * ds][dst] = lo2[k];
+                    ws.f[op][3 - 2 * ds][dst] = hi2[k];
+                    ws.idx[op][dst] = id[k];
+                }
+            }
+            __syncwarp();  // a warp's rows are its own until the next barrier
         }
-        __syncthreads();
-        if (tid < NB) {
-            int tot = 0;
-            for (int ww = 0; ww < STATS_THREADS / 32; ww++) tot += wcnt[ww][tid];
-            run[tid] += tot;
-        }
-        __syncthreads();
-    }
     }
 }
 
@@ -1746,7 +1894,7 @@ namespace ct {
 // Phases A, B and C over the root records already in place (one per tree).
 // Returns the record count through *nrec_out; one host synchronisation per
 // phase-A level.
-static int build_levels(WS& ws, cudaStream_t st, int NB, int64_t cpl, bool run_phase_a, int n_roots,
+static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, bool run_phase_a, int n_roots,
                         Counters* hc_out) {
     // a function attribute belongs to the current device (and context): set
     // it on every call rather than once per process
@@ -1763,17 +1911,22 @@ static int build_levels(WS& ws, cudaStream_t st, int NB, int64_t cpl, bool run_p
             int width = le - lb;
             // tiles for pending nodes of this level
             cudaMemsetAsync(&ws.cnt->tile_count, 0, sizeof(int), st);
+            cudaMemsetAsync(&ws.cnt->turned, 0, sizeof(int), st);
             int g = std::max(1, std::min((width + 3) / 4, 4096));
-            k_make_tiles<<<g, 128, 0, st>>>(ws, NB);
+            k_make_tiles<<<g, 128, 0, st>>>(ws, NB, n);
             CT_CHECK_LAUNCH("make_tiles");
             CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
             CT_CUDA(cudaStreamSynchronize(st));
             if (hc.err & 0x80000000u) return ct_fail(CT_ERR_WORKSPACE, "builder tile capacity exceeded");
             int ntiles = hc.tile_count;
             if (ntiles == 0) break;
-            k_stats<false><<<ntiles, STATS_THREADS, 0, st>>>(ws, parity, NB);
-            k_decide<false><<<(width + 3) / 4, 128, 0, st>>>(ws, NB, (long long)cpl);
-            k_scatter<false><<<ntiles, STATS_THREADS, 0, st>>>(ws, parity, NB);
+            const int gd = (width + 3) / 4;
+            if (NB == 4) k_stats<false, DIM_OWN, true><<<ntiles, STATS4_THREADS, 0, st>>>(ws, parity, NB);
+            else k_stats<false, DIM_OWN, false><<<ntiles, STATS_THREADS, 0, st>>>(ws, parity, NB);
+            k_decide<false, DIM_OWN><<<gd, 128, 0, st>>>(ws, NB, (long long)cpl);
+            k_stats<true, DIM_OTHER, false><<<std::min(ntiles, 152 * 8), STATS_THREADS, 0, st>>>(ws, parity, NB);
+            k_decide<true, DIM_OTHER><<<std::min(gd, 152 * 8), 128, 0, st>>>(ws, NB, (long long)cpl);
+            k_scatter<false><<<ntiles, SCAT_THREADS, 0, st>>>(ws, parity, NB);
             CT_CHECK_LAUNCH("phase A level");
             CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
             CT_CUDA(cudaStreamSynchronize(st));
@@ -1868,7 +2021,7 @@ int ct_build_tree(const double* bb, int64_t n, int32_t NB, int64_t cpl, int32_t 
     }
     CT_CHECK_LAUNCH("build init");
     Counters hc;
-    int s = build_levels(ws, st, NB, cpl, ni > SMALL, 1, &hc);
+    int s = build_levels(ws, st, ni, NB, cpl, ni > SMALL, 1, &hc);
     if (s) return s;
     long long root_splits = 0;
     CT_CUDA(cudaMemcpyAsync(&root_splits, &ws.recs[0].splits, sizeof(long long), cudaMemcpyDeviceToHost, st));
@@ -1930,7 +2083,7 @@ int ct_build_forest(const double* bb, int64_t n_total, const int64_t* tree_off_h
     k_forest_root_resolve<<<gt, 256, 0, st>>>(ws);
     CT_CHECK_LAUNCH("forest init");
     Counters hc;
-    int s = build_levels(ws, st, NB, cpl, any_large, n_trees, &hc);
+    int s = build_levels(ws, st, ni, NB, cpl, any_large, n_trees, &hc);
     if (s) return s;
     std::vector<ARec> roots(n_trees);
     std::vector<int> depth(n_trees);
@@ -1998,10 +2151,10 @@ int ct_build_forest_async(const double* bb, int64_t n_total, const int64_t* tree
         for (int L = 0; L < DEV_MAX_LEVELS; L++) {
             const int parity = L & 1;
             k_level_start<<<1, 32, 0, st>>>(ws);
-            k_make_tiles<<<G, 128, 0, st>>>(ws, NB);
-            k_stats<true><<<G, STATS_THREADS, 0, st>>>(ws, parity, NB);
-            k_decide<true><<<G, 128, 0, st>>>(ws, NB, (long long)cpl);
-            k_scatter<true><<<G, STATS_THREADS, 0, st>>>(ws, parity, NB);
+            k_make_tiles<<<G, 128, 0, st>>>(ws, NB, ni);
+            k_stats<true, DIM_BOTH, false><<<G, STATS_THREADS, 0, st>>>(ws, parity, NB);
+            k_decide<true, DIM_BOTH><<<G, 128, 0, st>>>(ws, NB, (long long)cpl);
+            k_scatter<true><<<G, SCAT_THREADS, 0, st>>>(ws, parity, NB);
             k_level_next<<<1, 32, 0, st>>>(ws, L);
         }
     }
