@@ -79,7 +79,7 @@ struct Counters {
     unsigned int err;
     int max_depth;
     int lb, le;  // current level record range
-    int pad;
+    long long splits0;  // (host) splits of the first tree
     unsigned long long root_key[4];
     int root_zp[4];
     int done;    // device-driven level loop: no pending record left (or an error)
@@ -369,6 +369,7 @@ __global__ void k_reset(WS ws, int n, int cpl_small_root, int root_dim) {
     Counters* c = ws.cnt;
     c->rec_count = 1;
     c->tile_count = 0;
+    c->turned = 0;
     c->small_count = 0;
     c->err = 0;
     c->max_depth = 0;
@@ -393,6 +394,8 @@ __global__ void k_reset(WS ws, int n, int cpl_small_root, int root_dim) {
     r.Lmax = -1.0;
     r.Rmin = -1.0;
     ws.recs[0] = r;
+    ws.lvl_b[0] = 0;
+    ws.lvl_e[0] = 1;
     ws.tree_depth[0] = 0;
     if (n <= SMALL) {
         ws.small_list[0] = 0;
@@ -493,8 +496,7 @@ __global__ void k_make_tiles(WS ws, int NB, int n) {
 // Per tile: bucket membership in the dimensions asked for; per (dim, bucket):
 // count, first-occurrence min of lo_x / lo_y and max of hi_x / hi_y (as
 // min-form keys) and the first position of a zero value.
-// LOOP: the device-driven level loop's form -- a fixed grid walks the tiles
-// whose count the make-tiles pass left on the device.
+// A grid walks the tiles whose count the make-tiles pass left on the device.
 // The dimensions: BOTH (the forest builds, whose levels are launched without
 // knowing whether a node needs its other one), the node's OWN, or the OTHER
 // one of the nodes that need it (K_TURN), in a second pass that finds none on
@@ -507,7 +509,7 @@ __global__ void k_make_tiles(WS ws, int NB, int n) {
 // threads, fewer for the small nodes of the last levels: 0.19 / 0.23).
 enum { DIM_BOTH = 0, DIM_OWN = 1, DIM_OTHER = 2 };
 
-template <bool LOOP, int DIMS, bool NB4>
+template <int DIMS, bool NB4>
 __global__ void __launch_bounds__(NB4 ? STATS4_THREADS : STATS_THREADS, NB4 ? 12 : 1) k_stats(WS ws, int parity, int NB) {
     __shared__ unsigned long long K[2][NBMAX + 1];
     __shared__ unsigned int cnt[2][NBMAX];
@@ -516,9 +518,9 @@ __global__ void __launch_bounds__(NB4 ? STATS4_THREADS : STATS_THREADS, NB4 ? 12
     const unsigned FULL = 0xffffffffu;
     const unsigned long long KZ = 0x8000000000000000ull;  // fkey(0)
     if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
-    const int nt = LOOP ? (ws.cnt->done ? 0 : ws.cnt->tile_count) : (int)gridDim.x;
+    const int nt = ws.cnt->done ? 0 : ws.cnt->tile_count;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        if (LOOP) __syncthreads();  // the previous tile's readers are done with the shared arrays
+        __syncthreads();  // the previous tile's readers are done with the shared arrays
         const int r = ws.tile_rec[t];
         const int s = ws.tile_start[t], e = ws.tile_end[t];
         const int lb = ws.cnt->lb;
@@ -650,7 +652,7 @@ __global__ void __launch_bounds__(NB4 ? STATS4_THREADS : STATS_THREADS, NB4 ? 12
 // One warp per record of the current level: the upstream split decision for
 // pending nodes, children records, bucket bases and tile prefixes.  DIMS: the
 // dimensions k_stats has looked at.
-template <bool LOOP, int DIMS>
+template <int DIMS>
 __global__ void k_decide(WS ws, int NB, long long cpl) {
     __shared__ int s_cnt[4][2][NBMAX];
     __shared__ double s_Rmin[4][2][NBMAX];
@@ -658,10 +660,10 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     const unsigned FULL = 0xffffffffu;
     int lane = threadIdx.x & 31;
     int w = threadIdx.x >> 5;  // blockDim = 128
-    if (LOOP && ws.cnt->done) return;
+    if (ws.cnt->done) return;
     if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
     int lb = ws.cnt->lb, le = ws.cnt->le;
-    const int step = LOOP ? (int)gridDim.x * 4 : INT32_MAX / 2;
+    const int step = (int)gridDim.x * 4;
     for (int r = lb + blockIdx.x * 4 + w; r < le; r += step) {
     __syncwarp();
     ARec* R = &ws.recs[r];
@@ -876,7 +878,6 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
 // 195, and twice that on the last levels of 256), 170 at the copy rate.
 constexpr int SCAT_IPT = 4;
 
-template <bool LOOP>
 __global__ void __launch_bounds__(SCAT_THREADS) k_scatter(WS ws, int parity, int NB) {
     __shared__ unsigned long long K[NBMAX + 1];
     __shared__ int base[NBMAX];
@@ -884,9 +885,9 @@ __global__ void __launch_bounds__(SCAT_THREADS) k_scatter(WS ws, int parity, int
     static_assert(ROWS <= 32, "a lane per (round's part, warp)");
     __shared__ int first[ROWS][NBMAX];  // cells of (part, warp) per bucket, then where the first goes
     const unsigned FULL = 0xffffffffu;
-    const int nt = LOOP ? (ws.cnt->done ? 0 : ws.cnt->tile_count) : (int)gridDim.x;
+    const int nt = ws.cnt->done ? 0 : ws.cnt->tile_count;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        if (LOOP) __syncthreads();
+        __syncthreads();
         int r = ws.tile_rec[t];
         int s = ws.tile_start[t], e = ws.tile_end[t];
         int lb = ws.cnt->lb;
@@ -1526,10 +1527,8 @@ __global__ void __launch_bounds__(SUB_WARPS * 32, 10) k_subtree(WS ws, int NB, l
 // phase C: numbering and emission
 // ------------------------------------------------------------------------
 
-// ---- the device-driven level loop: per-level bookkeeping on the device ----
-__global__ void k_level_start(WS ws) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && !ws.cnt->done) ws.cnt->tile_count = 0;
-}
+// The levels after those of the last run.
+__global__ void k_levels_again(WS ws) { ws.cnt->nlev = 1; }
 
 // After a level's scatter: the records it created are the next level; none
 // (or a capacity error) ends the loop.
@@ -1549,39 +1548,46 @@ __global__ void k_level_next(WS ws, int L) {
     }
     c->lb = nb;
     c->le = ne;
+    c->tile_count = 0;
+    c->turned = 0;
     ws.lvl_b[L + 1] = nb;
     ws.lvl_e[L + 1] = ne;
     c->nlev = L + 2;
 }
 
+__device__ __forceinline__ void count_up(const WS& ws, int r) {
+    ARec* R = &ws.recs[r];
+    if (R->kind == K_SPLIT) R->splits = 1 + ws.recs[R->child].splits + ws.recs[R->child + 1].splits;
+    else if (R->kind == K_LEAF) R->splits = 0;
+    // K_SUBTREE: set by k_subtree
+}
+
+__device__ __forceinline__ void number_down(const WS& ws, int r) {
+    ARec* R = &ws.recs[r];
+    if (r < ws.n_roots) {  // every tree is numbered from its own root
+        R->S = 0;
+        R->pos = 0;
+    }
+    if (R->kind == K_SPLIT) {
+        ARec* A = &ws.recs[R->child];
+        ARec* B = &ws.recs[R->child + 1];
+        A->S = R->S + 1;
+        B->S = R->S + 1 + A->splits;
+        A->pos = 1 + 2 * R->S;
+        B->pos = 2 + 2 * R->S;
+    }
+}
+
 __global__ void k_count_up_dev(WS ws, int L) {
     if (L >= ws.cnt->nlev) return;
     int b = ws.lvl_b[L], e = ws.lvl_e[L];
-    for (int r = b + blockIdx.x * blockDim.x + threadIdx.x; r < e; r += gridDim.x * blockDim.x) {
-        ARec* R = &ws.recs[r];
-        if (R->kind == K_SPLIT) R->splits = 1 + ws.recs[R->child].splits + ws.recs[R->child + 1].splits;
-        else if (R->kind == K_LEAF) R->splits = 0;
-    }
+    for (int r = b + blockIdx.x * blockDim.x + threadIdx.x; r < e; r += gridDim.x * blockDim.x) count_up(ws, r);
 }
 
 __global__ void k_number_down_dev(WS ws, int L) {
     if (L >= ws.cnt->nlev) return;
     int b = ws.lvl_b[L], e = ws.lvl_e[L];
-    for (int r = b + blockIdx.x * blockDim.x + threadIdx.x; r < e; r += gridDim.x * blockDim.x) {
-        ARec* R = &ws.recs[r];
-        if (r < ws.n_roots) {
-            R->S = 0;
-            R->pos = 0;
-        }
-        if (R->kind == K_SPLIT) {
-            ARec* A = &ws.recs[R->child];
-            ARec* B = &ws.recs[R->child + 1];
-            A->S = R->S + 1;
-            B->S = R->S + 1 + A->splits;
-            A->pos = 1 + 2 * R->S;
-            B->pos = 2 + 2 * R->S;
-        }
-    }
+    for (int r = b + blockIdx.x * blockDim.x + threadIdx.x; r < e; r += gridDim.x * blockDim.x) number_down(ws, r);
 }
 
 // Node counts (1 + 2 splits of the root), their offsets (one block, serial
@@ -1626,28 +1632,24 @@ __global__ void k_forest_counts(WS ws, int64_t* n_nodes, int64_t* node_off, int*
 
 __global__ void k_count_up(WS ws, int b, int e) {
     int r = b + blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= e) return;
-    ARec* R = &ws.recs[r];
-    if (R->kind == K_SPLIT) R->splits = 1 + ws.recs[R->child].splits + ws.recs[R->child + 1].splits;
-    else if (R->kind == K_LEAF) R->splits = 0;
-    // K_SUBTREE: set by k_subtree
+    if (r < e) count_up(ws, r);
 }
 
 __global__ void k_number_down(WS ws, int b, int e) {
     int r = b + blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= e) return;
-    ARec* R = &ws.recs[r];
-    if (r < ws.n_roots) {  // every tree is numbered from its own root
-        R->S = 0;
-        R->pos = 0;
+    if (r < e) number_down(ws, r);
+}
+
+// Both passes over all levels by one block (few records: a level's pass is
+// then its launch).
+__global__ void __launch_bounds__(1024) k_number_one(WS ws, int nlev) {
+    for (int L = nlev - 1; L >= 0; L--) {
+        for (int r = ws.lvl_b[L] + threadIdx.x; r < ws.lvl_e[L]; r += blockDim.x) count_up(ws, r);
+        __syncthreads();
     }
-    if (R->kind == K_SPLIT) {
-        ARec* A = &ws.recs[R->child];
-        ARec* B = &ws.recs[R->child + 1];
-        A->S = R->S + 1;
-        B->S = R->S + 1 + A->splits;
-        A->pos = 1 + 2 * R->S;
-        B->pos = 2 + 2 * R->S;
+    for (int L = 0; L < nlev; L++) {
+        for (int r = ws.lvl_b[L] + threadIdx.x; r < ws.lvl_e[L]; r += blockDim.x) number_down(ws, r);
+        __syncthreads();
     }
 }
 
@@ -1783,6 +1785,7 @@ __global__ void k_forest_reset(WS ws) {
     Counters* c = ws.cnt;
     c->rec_count = ws.n_roots;
     c->tile_count = 0;
+    c->turned = 0;
     c->small_count = 0;
     c->err = 0;
     c->max_depth = 0;
@@ -1892,8 +1895,11 @@ size_t ct_build_workspace_size(int64_t n, int32_t NB, int32_t factor) {
 namespace ct {
 
 // Phases A, B and C over the root records already in place (one per tree).
-// Returns the record count through *nrec_out; one host synchronisation per
-// phase-A level.
+//
+// The levels of phase A are launched ahead, as many as a balanced tree needs
+// and one, and only then waited for: a level with nothing left is seven empty
+// launches, waiting for the record counts of every level took three
+// synchronisations and copies each (80k cells: 1.79 -> 1.38 ms, 16M: 23.5 -> 23.2).
 static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, bool run_phase_a, int n_roots,
                         Counters* hc_out) {
     // a function attribute belongs to the current device (and context): set
@@ -1903,48 +1909,55 @@ static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, boo
     std::vector<int> level_b, level_e;
     level_b.push_back(0);
     level_e.push_back(n_roots);
-    int parity = 0;
     Counters hc;
+    int ahead = 2;
+    while (ahead < DEV_MAX_LEVELS - 4 && ((long long)SMALL << (ahead - 1)) < n) ahead++;
+    bool one_run = true;
     if (run_phase_a) {
+        const long long tile = std::min(TILE_MIN, std::max(512, n / (152 * 8)));  // tile_len_for
+        int parity = 0;
+        double width = n_roots;  // records of the level, at most
+        // the counters and the ranges of the levels run lie side by side
+        const size_t lvl_off = (size_t)((char*)ws.lvl_b - (char*)ws.cnt), end_off = (size_t)((char*)ws.lvl_e - (char*)ws.cnt);
+        std::vector<char> state(end_off + sizeof(int) * (DEV_MAX_LEVELS + 1));
         while (true) {
-            int lb = level_b.back(), le = level_e.back();
-            int width = le - lb;
-            // tiles for pending nodes of this level
-            cudaMemsetAsync(&ws.cnt->tile_count, 0, sizeof(int), st);
-            cudaMemsetAsync(&ws.cnt->turned, 0, sizeof(int), st);
-            int g = std::max(1, std::min((width + 3) / 4, 4096));
-            k_make_tiles<<<g, 128, 0, st>>>(ws, NB, n);
-            CT_CHECK_LAUNCH("make_tiles");
-            CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+            for (int i = 0; i < ahead; i++) {
+                const double pending = std::min(width, n_roots + (double)n / SMALL);
+                const long long ntiles = (long long)(n / tile + pending) + 1;
+                const int gd = (int)std::min((pending + 3) / 4 + 1, 65536.0), go = std::min(gd, 152 * 8);
+                k_make_tiles<<<std::min(gd, 4096), 128, 0, st>>>(ws, NB, n);
+                const int gt = (int)std::min<long long>(ntiles, 65536);
+                if (NB == 4) k_stats<DIM_OWN, true><<<gt, STATS4_THREADS, 0, st>>>(ws, parity, NB);
+                else k_stats<DIM_OWN, false><<<gt, STATS_THREADS, 0, st>>>(ws, parity, NB);
+                k_decide<DIM_OWN><<<gd, 128, 0, st>>>(ws, NB, (long long)cpl);
+                k_stats<DIM_OTHER, false><<<std::min(gt, 152 * 8), STATS_THREADS, 0, st>>>(ws, parity, NB);
+                k_decide<DIM_OTHER><<<go, 128, 0, st>>>(ws, NB, (long long)cpl);
+                k_scatter<<<gt, SCAT_THREADS, 0, st>>>(ws, parity, NB);
+                k_level_next<<<1, 32, 0, st>>>(ws, i);
+                parity = 1 - parity;
+                width = std::min(2.0 * width, 2.0 * n_roots + 2.0 * n / SMALL);
+            }
+            CT_CHECK_LAUNCH("phase A levels");
+            CT_CUDA(cudaMemcpyAsync(state.data(), ws.cnt, state.size(), cudaMemcpyDeviceToHost, st));
             CT_CUDA(cudaStreamSynchronize(st));
-            if (hc.err & 0x80000000u) return ct_fail(CT_ERR_WORKSPACE, "builder tile capacity exceeded");
-            int ntiles = hc.tile_count;
-            if (ntiles == 0) break;
-            const int gd = (width + 3) / 4;
-            if (NB == 4) k_stats<false, DIM_OWN, true><<<ntiles, STATS4_THREADS, 0, st>>>(ws, parity, NB);
-            else k_stats<false, DIM_OWN, false><<<ntiles, STATS_THREADS, 0, st>>>(ws, parity, NB);
-            k_decide<false, DIM_OWN><<<gd, 128, 0, st>>>(ws, NB, (long long)cpl);
-            k_stats<true, DIM_OTHER, false><<<std::min(ntiles, 152 * 8), STATS_THREADS, 0, st>>>(ws, parity, NB);
-            k_decide<true, DIM_OTHER><<<std::min(gd, 152 * 8), 128, 0, st>>>(ws, NB, (long long)cpl);
-            k_scatter<false><<<ntiles, SCAT_THREADS, 0, st>>>(ws, parity, NB);
-            CT_CHECK_LAUNCH("phase A level");
-            CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-            CT_CUDA(cudaStreamSynchronize(st));
+            memcpy(&hc, state.data(), sizeof(Counters));
             if (hc.err & 0x80000000u)
-                return ct_fail(CT_ERR_WORKSPACE, "builder node-record capacity exceeded (unbalanced tree)");
-            int nb_ = le, ne_ = hc.rec_count;
-            if (ne_ == nb_) break;
-            level_b.push_back(nb_);
-            level_e.push_back(ne_);
-            parity = 1 - parity;
-            // publish the next level range to the device
-            int range[2] = {nb_, ne_};
-            CT_CUDA(cudaMemcpyAsync(&ws.cnt->lb, range, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-            CT_CUDA(cudaStreamSynchronize(st));
+                return ct_fail(CT_ERR_WORKSPACE, "builder tile or node-record capacity exceeded (unbalanced tree)");
+            const int* lb = reinterpret_cast<const int*>(state.data() + lvl_off);
+            const int* le = reinterpret_cast<const int*>(state.data() + end_off);
+            for (int k = 1; k < hc.nlev; k++) {
+                level_b.push_back(lb[k]);
+                level_e.push_back(le[k]);
+            }
+            if (hc.done) break;
+            one_run = false;
+            ahead = 4;
+            k_levels_again<<<1, 1, 0, st>>>(ws);
         }
+    } else {
+        CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+        CT_CUDA(cudaStreamSynchronize(st));
     }
-    CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-    CT_CUDA(cudaStreamSynchronize(st));
     int nsmall = hc.small_count;
     if (nsmall > 0) {
         int blocks = (nsmall + SUB_WARPS - 1) / SUB_WARPS;
@@ -1952,22 +1965,25 @@ static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, boo
         CT_CHECK_LAUNCH("subtree");
     }
     // phase C: split counts bottom-up, pre-order ranks top-down
-    for (int L = (int)level_b.size() - 1; L >= 0; L--) {
-        int b = level_b[L], e = level_e[L];
-        k_count_up<<<(e - b + 255) / 256, 256, 0, st>>>(ws, b, e);
-    }
-    for (size_t L = 0; L < level_b.size(); L++) {
-        int b = level_b[L], e = level_e[L];
-        k_number_down<<<(e - b + 255) / 256, 256, 0, st>>>(ws, b, e);
+    if (one_run && n_roots == 1 && hc.rec_count <= 8192) {
+        k_number_one<<<1, 1024, 0, st>>>(ws, (int)level_b.size());
+    } else {
+        for (int L = (int)level_b.size() - 1; L >= 0; L--) {
+            int b = level_b[L], e = level_e[L];
+            k_count_up<<<(e - b + 255) / 256, 256, 0, st>>>(ws, b, e);
+        }
+        for (size_t L = 0; L < level_b.size(); L++) {
+            int b = level_b[L], e = level_e[L];
+            k_number_down<<<(e - b + 255) / 256, 256, 0, st>>>(ws, b, e);
+        }
     }
     CT_CHECK_LAUNCH("numbering");
     CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+    CT_CUDA(cudaMemcpyAsync(&hc_out->splits0, &ws.recs[0].splits, sizeof(long long), cudaMemcpyDeviceToHost, st));
     CT_CUDA(cudaStreamSynchronize(st));
     if (hc.err & CT_DEVERR_BUCKET)
         return ct_fail(CT_ERR_DEVICE, "tree construction failed: a cell centroid fell outside every bucket");
-    // remember the record count for the emit call
-    CT_CUDA(cudaMemcpyAsync(&ws.cnt->pad, &hc.rec_count, sizeof(int), cudaMemcpyHostToDevice, st));
-    CT_CUDA(cudaStreamSynchronize(st));
+    hc.splits0 = hc_out->splits0;
     *hc_out = hc;
     return CT_OK;
 }
@@ -1977,8 +1993,11 @@ static int emit_nodes(const WS& ws, int64_t n, long long n_nodes, const int64_t*
                       cudaStream_t st) {
     Counters hc;
     CT_CUDA(cudaMemcpyAsync(&hc, ws.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+    long long splits0 = 0;
+    CT_CUDA(cudaMemcpyAsync(&splits0, &ws.recs[0].splits, sizeof(long long), cudaMemcpyDeviceToHost, st));
     CT_CUDA(cudaStreamSynchronize(st));
-    int nrec = hc.pad;
+    int nrec = hc.rec_count;
+    if (n_nodes < 0) n_nodes = 1 + 2 * splits0;  // one tree
     NodesOut o{child, Lmax, Rmin, ptr, size, dim};
     k_emit_phaseA<<<(nrec + 255) / 256, 256, 0, st>>>(ws, nrec, n_nodes, o, node_off);
     if (hc.small_count > 0)
@@ -2023,10 +2042,7 @@ int ct_build_tree(const double* bb, int64_t n, int32_t NB, int64_t cpl, int32_t 
     Counters hc;
     int s = build_levels(ws, st, ni, NB, cpl, ni > SMALL, 1, &hc);
     if (s) return s;
-    long long root_splits = 0;
-    CT_CUDA(cudaMemcpyAsync(&root_splits, &ws.recs[0].splits, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    CT_CUDA(cudaStreamSynchronize(st));
-    if (n_nodes_host) *n_nodes_host = 1 + 2 * root_splits;
+    if (n_nodes_host) *n_nodes_host = 1 + 2 * hc.splits0;
     if (max_depth_host) *max_depth_host = hc.max_depth;
     return CT_OK;
 }
@@ -2037,10 +2053,7 @@ int ct_build_emit(const void* workspace, int64_t n, int32_t NB, int32_t factor, 
     if (NB < 2 || NB > NBMAX || factor < 1) return ct_fail(CT_ERR_ARG, "bad n_buckets / capacity_factor");
     WS ws;
     carve((char*)workspace, n, NB, factor, &ws);
-    long long root_splits = 0;
-    CT_CUDA(cudaMemcpyAsync(&root_splits, &ws.recs[0].splits, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    CT_CUDA(cudaStreamSynchronize(st));
-    return emit_nodes(ws, n, 1 + 2 * root_splits, nullptr, child, Lmax, Rmin, ptr, size, dim, bb_indices, st);
+    return emit_nodes(ws, n, -1, nullptr, child, Lmax, Rmin, ptr, size, dim, bb_indices, st);
 }
 
 size_t ct_build_forest_workspace_size(int64_t n_total, int32_t n_trees, int32_t NB, int32_t factor) {
@@ -2150,11 +2163,10 @@ int ct_build_forest_async(const double* bb, int64_t n_total, const int64_t* tree
     if (any_large) {
         for (int L = 0; L < DEV_MAX_LEVELS; L++) {
             const int parity = L & 1;
-            k_level_start<<<1, 32, 0, st>>>(ws);
             k_make_tiles<<<G, 128, 0, st>>>(ws, NB, ni);
-            k_stats<true, DIM_BOTH, false><<<G, STATS_THREADS, 0, st>>>(ws, parity, NB);
-            k_decide<true, DIM_BOTH><<<G, 128, 0, st>>>(ws, NB, (long long)cpl);
-            k_scatter<true><<<G, SCAT_THREADS, 0, st>>>(ws, parity, NB);
+            k_stats<DIM_BOTH, false><<<G, STATS_THREADS, 0, st>>>(ws, parity, NB);
+            k_decide<DIM_BOTH><<<G, 128, 0, st>>>(ws, NB, (long long)cpl);
+            k_scatter<<<G, SCAT_THREADS, 0, st>>>(ws, parity, NB);
             k_level_next<<<1, 32, 0, st>>>(ws, L);
         }
     }
