@@ -556,6 +556,16 @@ int ct_count_item_candidates(const ct_tree* tree, int32_t mode, const double* se
 int ct_write_item_candidates(const ct_tree* tree, int32_t mode, const double* segs, const int32_t* item_seg,
                              const int32_t* item_node, int64_t n_items, const int64_t* offsets, int32_t* cand_seg,
                              int32_t* cand_pos, void* stream);
+/* The same with the first spec_cap candidates of every item kept in spec
+ * (n_items x spec_cap int32) by the counting pass; the writing pass copies
+ * those and walks again only the items with more. */
+int ct_count_item_candidates_spec(const ct_tree* tree, int32_t mode, const double* segs, const int32_t* item_seg,
+                                  const int32_t* item_node, int64_t n_items, int64_t* counts, int32_t* spec,
+                                  int32_t spec_cap, void* stream);
+int ct_write_item_candidates_spec(const ct_tree* tree, int32_t mode, const double* segs, const int32_t* item_seg,
+                                  const int32_t* item_node, int64_t n_items, const int64_t* counts,
+                                  const int64_t* offsets, const int32_t* spec, int32_t spec_cap, int32_t* cand_seg,
+                                  int32_t* cand_pos, void* stream);
 int ct_segment_candidate_ranges(const int64_t* item_off, const int64_t* item_cnt, int64_t n,
                                 const int64_t* item_cand_off, const int64_t* item_cand_cnt, int64_t n_items,
                                 int64_t* cand_off, int64_t* cand_cnt, void* stream);

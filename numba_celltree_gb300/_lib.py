@@ -220,6 +220,9 @@ SIGNATURES = {
     "ct_write_edge_items": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _I64, _P, _I32, _P, _P, _P, _P]),
     "ct_count_item_candidates": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P]),
     "ct_write_item_candidates": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _P, _P]),
+    "ct_count_item_candidates_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _I32, _P]),
+    "ct_write_item_candidates_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _P, _P, _I64, _P, _P, _P, _I32,
+                                                     _P, _P, _P]),
     "ct_segment_candidate_ranges": (ctypes.c_int, [_P, _P, _I64, _P, _P, _I64, _P, _P, _P]),
     "ct_spatial_order_workspace_size": (_SZ, [_I64]),
     "ct_spatial_order": (ctypes.c_int, [_P, _I64, _I32, _P, _P, _P, _SZ, _P]),

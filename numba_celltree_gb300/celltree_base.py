@@ -506,7 +506,8 @@ class _GpuTree:
         items) -- items None (traverse again), ("spec", scratch, cap) with
         `keep` (the counting pass kept each segment's first `cap`
         candidates), or with a
-        cut the work items (item_seg, item_node, n_items, item offsets)."""
+        cut the work items (item_seg, item_node, n_items, item offsets, item
+        counts, scratch or None, cap; the scratch under the same limits)."""
         torch = _device.torch()
         lib = _lib.load()
         st = _device.stream()
@@ -545,14 +546,22 @@ class _GpuTree:
         _lib.check(lib.ct_write_edge_items(d, mode, P(segs_d), n, P(order), cut, P(ioff), P(iseg), P(inode), st),
                    "intersect_edges")
         iccnt = _device.empty((max(ni, 1),), torch.int64, self.device)
-        _lib.check(lib.ct_count_item_candidates(d, mode, P(segs_d), P(iseg), P(inode), ni, P(iccnt), st),
-                   "intersect_edges")
+        ispec, icap = None, int(self.SEG_SPEC_CAP)
+        while icap >= 8 and ni * icap * 4 > self.SEG_SPEC_MAX_BYTES:
+            icap //= 2
+        if keep and ni > 0 and (icap >= 8 or icap == self.SEG_SPEC_CAP):
+            ispec = _device.empty((ni, icap), torch.int32, self.device)
+            _lib.check(lib.ct_count_item_candidates_spec(d, mode, P(segs_d), P(iseg), P(inode), ni, P(iccnt),
+                                                         P(ispec), icap, st), "intersect_edges")
+        else:
+            _lib.check(lib.ct_count_item_candidates(d, mode, P(segs_d), P(iseg), P(inode), ni, P(iccnt), st),
+                       "intersect_edges")
         icoff, nc = self.scan(iccnt[:ni]) if ni > 0 else (iccnt[:0], 0)
         coff = _device.empty((n,), torch.int64, self.device)
         ccnt = _device.empty((n,), torch.int64, self.device)
         _lib.check(lib.ct_segment_candidate_ranges(P(ioff), P(icnt), n, P(icoff), P(iccnt), ni, P(coff), P(ccnt),
                                                    st), "intersect_edges")
-        return coff, ccnt, nc, (iseg, inode, ni, icoff)
+        return coff, ccnt, nc, (iseg, inode, ni, icoff, iccnt, ispec, icap)
 
     @staticmethod
     def chunk_ranges(counts: np.ndarray, max_results: int):
@@ -727,10 +736,15 @@ class _GpuTree:
                                                          P(cpos), st), "intersect_edges")
             del items
         else:
-            iseg, inode, ni, icoff = items
-            _lib.check(lib.ct_write_item_candidates(ctypes.byref(self.desc), mode, P(segs_d), P(iseg), P(inode), ni,
-                                                    P(icoff), P(cseg), P(cpos), st), "intersect_edges")
-            del items, iseg, inode, icoff
+            iseg, inode, ni, icoff, iccnt, ispec, icap = items
+            if ispec is None:
+                _lib.check(lib.ct_write_item_candidates(ctypes.byref(self.desc), mode, P(segs_d), P(iseg), P(inode),
+                                                        ni, P(icoff), P(cseg), P(cpos), st), "intersect_edges")
+            else:
+                _lib.check(lib.ct_write_item_candidates_spec(ctypes.byref(self.desc), mode, P(segs_d), P(iseg),
+                                                             P(inode), ni, P(iccnt), P(icoff), P(ispec), icap, P(cseg),
+                                                             P(cpos), st), "intersect_edges")
+            del items, iseg, inode, icoff, iccnt, ispec
         keep = _device.empty((max(nc, 1),), torch.uint8, self.device)
         xy_c = _device.empty((max(nc, 1), 2, 2), torch.float64, self.device)
         _lib.check(lib.ct_test_edge_candidates_u8(ctypes.byref(self.desc), mode, P(segs_d), P(cseg), P(cpos), nc,

@@ -560,9 +560,10 @@ __global__ void k_boxes_spec_emit(const int64_t* __restrict__ cnt, const int64_t
 }
 
 // Candidates of the segments whose count fits the counting pass's scratch.
+// (or the work items': item_seg)
 __global__ void k_edge_spec_emit(const int64_t* __restrict__ cnt, const int64_t* __restrict__ off, int64_t n,
-                                 const int* __restrict__ spec, int cap, int* __restrict__ cseg,
-                                 int* __restrict__ cpos) {
+                                 const int* __restrict__ item_seg, const int* __restrict__ spec, int cap,
+                                 int* __restrict__ cseg, int* __restrict__ cpos) {
     const int64_t total = n * (int64_t)cap;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
          k += (int64_t)gridDim.x * blockDim.x) {
@@ -570,7 +571,7 @@ __global__ void k_edge_spec_emit(const int64_t* __restrict__ cnt, const int64_t*
         const int c = (int)(k - i * cap);
         const int64_t m = cnt[i];
         if (m > cap || c >= m) continue;
-        cseg[off[i] + c] = (int)i;
+        cseg[off[i] + c] = item_seg ? item_seg[i] : (int)i;
         cpos[off[i] + c] = spec[k];
     }
 }
@@ -3373,6 +3374,36 @@ int ct_write_item_candidates(const ct_tree* t, int32_t mode, const double* segs,
     return CT_OK;
 }
 
+int ct_count_item_candidates_spec(const ct_tree* t, int32_t mode, const double* segs, const int32_t* item_seg,
+                                  const int32_t* item_node, int64_t n_items, int64_t* counts, int32_t* spec,
+                                  int32_t spec_cap, void* stream) {
+    int s = check_split(t, mode, 0);
+    if (s) return s;
+    if (n_items == 0) return CT_OK;
+    if (!spec || spec_cap < 1 || spec_cap > 4096) return ct_fail(CT_ERR_ARG, "spec_cap must be in [1, 4096]");
+    launch_edge_walk<false, false>(mode, make_q(t), (const double4*)segs, n_items, nullptr, item_seg, item_node, 0,
+                                   counts, nullptr, spec, spec_cap, nullptr, (cudaStream_t)stream);
+    CT_CHECK_LAUNCH("count_item_candidates_spec");
+    return CT_OK;
+}
+
+int ct_write_item_candidates_spec(const ct_tree* t, int32_t mode, const double* segs, const int32_t* item_seg,
+                                  const int32_t* item_node, int64_t n_items, const int64_t* counts,
+                                  const int64_t* offsets, const int32_t* spec, int32_t spec_cap, int32_t* cand_seg,
+                                  int32_t* cand_pos, void* stream) {
+    int s = check_split(t, mode, 0);
+    if (s) return s;
+    if (n_items == 0) return CT_OK;
+    if (!spec || spec_cap < 1 || spec_cap > 4096) return ct_fail(CT_ERR_ARG, "spec_cap must be in [1, 4096]");
+    cudaStream_t st = (cudaStream_t)stream;
+    k_edge_spec_emit<<<(unsigned)std::min<int64_t>(grid_of(n_items * (int64_t)spec_cap, 256), 152 * 16), 256, 0,
+                       st>>>(counts, offsets, n_items, item_seg, spec, spec_cap, cand_seg, cand_pos);
+    launch_edge_walk<false, true>(mode, make_q(t), (const double4*)segs, n_items, nullptr, item_seg, item_node, 0,
+                                  (int64_t*)offsets, cand_seg, cand_pos, spec_cap, counts, st);
+    CT_CHECK_LAUNCH("write_item_candidates_spec");
+    return CT_OK;
+}
+
 int ct_segment_candidate_ranges(const int64_t* item_off, const int64_t* item_cnt, int64_t n,
                                 const int64_t* item_cand_off, const int64_t* item_cand_cnt, int64_t n_items,
                                 int64_t* cand_off, int64_t* cand_cnt, void* stream) {
@@ -3423,7 +3454,7 @@ int ct_write_edge_candidates_spec(const ct_tree* t, int32_t mode, const double* 
     cudaStream_t st = (cudaStream_t)stream;
     TreeQ T = make_q(t);
     k_edge_spec_emit<<<(unsigned)std::min<int64_t>(grid_of(n * (int64_t)spec_cap, 256), 152 * 16), 256, 0, st>>>(
-        counts, offsets, n, spec, spec_cap, cand_seg, cand_pos);
+        counts, offsets, n, nullptr, spec, spec_cap, cand_seg, cand_pos);
     const int et = seg_threads(t);
     const double4* S = (const double4*)segs;
     const unsigned g = grid_of(n, et);
