@@ -663,6 +663,12 @@ int ct_pair_order(const int64_t* faces_a, int32_t n_max_vert_a, const int64_t* i
                   int32_t n_max_vert_b, const int64_t* indices_b, int64_t n, int32_t* order, void* workspace,
                   size_t workspace_bytes, void* stream);
 
+/* The same order for (box, face) pairs whose faces come up many times each:
+ * the faces' lengths are taken once (n_faces rows). */
+size_t ct_box_pair_order_workspace_size(int64_t n, int64_t n_faces);
+int ct_box_pair_order(const int64_t* faces, int32_t n_max_vert, int64_t n_faces, const int64_t* indices_face,
+                      int64_t n, int32_t* order, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Keeps the pairs with area > 0 (area != NULL) or flag != 0 (celltree.py:183,
  * 226, 268); outputs have capacity n; *total_host = kept count (synchronises). */
 size_t ct_compact_workspace_size(int64_t n);

@@ -199,6 +199,8 @@ SIGNATURES = {
     "ct_box_area_of_intersection_ordered": (ctypes.c_int, [_P, _P, _P, _I32, _P, _P, _I64, _P, _P, _P, _P]),
     "ct_pair_order_workspace_size": (_SZ, [_I64]),
     "ct_pair_order": (ctypes.c_int, [_P, _I32, _P, _P, _I32, _P, _I64, _P, _P, _SZ, _P]),
+    "ct_box_pair_order_workspace_size": (_SZ, [_I64, _I64]),
+    "ct_box_pair_order": (ctypes.c_int, [_P, _I32, _I64, _P, _I64, _P, _P, _SZ, _P]),
     "ct_liang_barsky_line_box_clip": (ctypes.c_int, [_P, _P, _P, _I64, _P, _P, _P, _P]),
     "ct_points_in_triangles": (ctypes.c_int, [_P, _P, _I64, _P, _I32, _I64, _P, _D, _P, _P, _P]),
     "ct_csr_workspace_size": (_SZ, [_I64]),

@@ -2292,6 +2292,31 @@ __global__ void __launch_bounds__(CL_THREADS) k_clip_area_small(
     out[i] = area;
 }
 
+__global__ void k_face_lengths(const int64_t* __restrict__ faces, int K, int64_t n, uint8_t* __restrict__ length) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        length[i] = (uint8_t)polygon_length(faces + i * K, K);
+}
+
+// The classes of (box, face) pairs from the faces' lengths, a byte each: for
+// batches with many pairs per face, whose rows are read from DRAM for every
+// pair otherwise (91M pairs on 5M faces 1.65 -> 0.42 ms).
+__global__ void __launch_bounds__(256) k_box_pair_keys(const uint8_t* __restrict__ length,
+                                                       const int64_t* __restrict__ ib, int64_t n,
+                                                       unsigned* __restrict__ key) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
+        int64_t b[4];
+        int l[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) b[u] = ib[min(i0 + u * step, n - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; u++) l[u] = length[b[u]];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i0 + u * step < n) key[i0 + u * step] = (unsigned)(8 + min(l[u] - 3, 7));
+    }
+}
+
 // 6-bit class of a pair: the polygon lengths (3 .. 10) of its two faces
 // (fa NULL: boxes, length 4)
 __global__ void k_pair_keys(const int64_t* __restrict__ fa, int Ka, const int64_t* __restrict__ ia,
@@ -3162,6 +3187,29 @@ int ct_pair_order(const int64_t* fa, int32_t Ka, const int64_t* ia, const int64_
     k_pair_keys<<<(unsigned)std::min<int64_t>(grid_of(n, 256), 152 * 8), 256, 0, st>>>(fa, Ka, ia, fb, Kb, ib, n, kin);
     CT_CHECK_LAUNCH("pair keys");
     return ct_radix_pass(kin, nullptr, n, 0, kout, order, (char*)ws + 2 * part, ws_bytes - 2 * part, stream);
+}
+
+int ct_box_pair_order(const int64_t* fb, int32_t Kb, int64_t n_faces, const int64_t* ib, int64_t n, int32_t* order,
+                      void* ws, size_t ws_bytes, void* stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (n < 0 || n > INT32_MAX || n_faces < 0) return ct_fail(CT_ERR_ARG, "pair or face count out of range");
+    if (!ws || ws_bytes < ct_box_pair_order_workspace_size(n, n_faces))
+        return ct_fail(CT_ERR_WORKSPACE, "pair order workspace");
+    if (n == 0) return CT_OK;
+    size_t part = ((size_t)n * sizeof(unsigned) + 255) / 256 * 256, lens = ((size_t)n_faces + 255) / 256 * 256;
+    uint8_t* length = (uint8_t*)ws;
+    unsigned* kin = (unsigned*)((char*)ws + lens);
+    unsigned* kout = (unsigned*)((char*)kin + part);
+    char* rest = (char*)kout + part;
+    k_face_lengths<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_of(n_faces, 256), 152 * 32)), 256, 0, st>>>(
+        fb, Kb, n_faces, length);
+    k_box_pair_keys<<<(unsigned)std::min<int64_t>(grid_of(n, 256), 152 * 8), 256, 0, st>>>(length, ib, n, kin);
+    CT_CHECK_LAUNCH("pair keys");
+    return ct_radix_pass(kin, nullptr, n, 0, kout, order, rest, ws_bytes - (size_t)(rest - (char*)ws), stream);
+}
+
+size_t ct_box_pair_order_workspace_size(int64_t n, int64_t n_faces) {
+    return ct_pair_order_workspace_size(n) + ((size_t)(n_faces > 0 ? n_faces : 1) + 255) / 256 * 256;
 }
 
 int ct_compact_pairs(const double* area, const uint8_t* flag, int64_t n, const int64_t* ii, const int64_t* jj,
