@@ -499,6 +499,16 @@ int ct_write_boxes_ws(const ct_tree* tree, const double* boxes, int64_t n, const
  * ct_count_boxes + ct_write_boxes. */
 int ct_count_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
                         int32_t* spec, int32_t spec_cap, void* stream);
+/* Large batches in one traversal: the counting pass keeps every terminal node
+ * with pairs (a leaf, or a subtree inside the box) as a record, ct_box_records_size
+ * bytes for `capacity` of them; the writing call expands them, or, when there
+ * were more, traverses again.  Same output as ct_count_boxes + ct_write_boxes. */
+size_t ct_box_records_size(int64_t capacity);
+int ct_count_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
+                           void* records, int64_t capacity, void* stream);
+int ct_write_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
+                           const int64_t* offsets, const void* records, int64_t capacity, int64_t* ii, int64_t* jj,
+                           void* stream);
 /* The same counts and scratch by one thread per box: faster for boxes of about
  * a cell that come in mesh order (query faces). */
 int ct_count_small_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,

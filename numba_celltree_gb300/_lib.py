@@ -211,6 +211,9 @@ SIGNATURES = {
     "ct_write_boxes_ws": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _I64, _I32, _P, _P, _P,
                                          ctypes.c_size_t, _P]),
     "ct_count_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I32, _P]),
+    "ct_box_records_size": (_SZ, [_I64]),
+    "ct_count_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _P]),
+    "ct_write_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _P, _P, _P]),
     "ct_count_small_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I32, _P]),
     "ct_write_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _P, _I32, _I64, _I32, _P, _P,
                                            _P, ctypes.c_size_t, _P]),

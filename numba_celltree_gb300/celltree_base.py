@@ -597,6 +597,12 @@ class _GpuTree:
     SPEC_CAP = 64
     SPEC_CAP_LARGE = 16
     SPEC_MAX_BYTES = 1 << 30
+    # other batches keep terminal nodes instead: room for BOX_RECORDS of 16
+    # bytes a box, as far as SPEC_MAX_BYTES goes (250k boxes of 0.2 to 100
+    # cells a side have 77 on average); below BOX_RECORDS_MIN a box the pairs
+    # of small boxes are kept after all
+    BOX_RECORDS = 256
+    BOX_RECORDS_MIN = 64
 
     def locate_boxes(self, boxes_d, config=None, budget=None, small=False):
         """Pairs (box, cell) of every box query, box-major in upstream order;
@@ -617,9 +623,15 @@ class _GpuTree:
         order = None
         if not small and self.in_spatial_order(n, config):
             order = self.spatial_order(boxes_d, 0)[0]
-        spec = None
+        spec = recs = None
         cap = self.SPEC_CAP if n <= self.SPEC_MAX_BOXES else self.SPEC_CAP_LARGE
-        if self.SPEC_MAX_BOXES > 0 and 0 < n and n * cap * 4 <= self.SPEC_MAX_BYTES:
+        most = min(n * self.BOX_RECORDS, self.SPEC_MAX_BYTES // 16)
+        if not small and self.SPEC_MAX_BOXES > 0 and 0 < n and most >= n * self.BOX_RECORDS_MIN:
+            # one traversal: the counting pass keeps the boxes' terminal nodes
+            recs = _device.empty((int(lib.ct_box_records_size(most)),), torch.uint8, self.device)
+            _lib.check(lib.ct_count_boxes_records(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
+                                                  _device.ptr(counts), _device.ptr(recs), most, st), "locate_boxes")
+        elif self.SPEC_MAX_BOXES > 0 and 0 < n and n * cap * 4 <= self.SPEC_MAX_BYTES:
             # one traversal: the counting pass also keeps each box's first pairs
             spec = _device.empty((n, cap), torch.int32, self.device)
             count = lib.ct_count_small_boxes_spec if small else lib.ct_count_boxes_spec
@@ -639,6 +651,11 @@ class _GpuTree:
         jj = _device.empty((total,), torch.int64, self.device)
         # the writing pass repeats the counting pass's traversal: a condition
         # it could report has been reported by the count
+        if recs is not None:
+            _lib.check(lib.ct_write_boxes_records(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
+                                                  _device.ptr(offsets), _device.ptr(recs), most, _device.ptr(ii),
+                                                  _device.ptr(jj), st), "locate_boxes")
+            return ii, jj
         if spec is not None:
             jm = int(config.get("job_cells") or 0)
             wsz = int(lib.ct_write_boxes_workspace_size(total, jm))
