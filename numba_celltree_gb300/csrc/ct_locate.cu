@@ -1218,8 +1218,10 @@ __device__ bool clip_box(const float2* L, int len, float X0, float X1, float Y0,
                          float4* out) {
     const float u = 5.9604644775390625e-08f;
     float bx0 = FLT_MAX, bx1 = -FLT_MAX, by0 = FLT_MAX, by1 = -FLT_MAX;
-    for (int k = 0; k < len; k++) {
-        const float2 P = L[k], Q = L[(k + 1 == len) ? 0 : k + 1];
+#pragma unroll
+    for (int k = 0; k < KMAX; k++) {
+        if (k >= len) break;
+        const float2 P = L[k], Q = k + 1 < KMAX && k + 1 < len ? L[k + 1 < KMAX ? k + 1 : 0] : L[0];
         const float dx = Q.x - P.x, dy = Q.y - P.y;
         float t0 = 0.0f, t1 = 1.0f;
         bool ok = true;
@@ -1252,8 +1254,11 @@ __device__ bool clip_box(const float2* L, int len, float X0, float X1, float Y0,
         const float cx = (c & 1) ? X1 : X0, cy = (c & 2) ? Y1 : Y0;
         int parity = 0;
         bool unsure = false;
-        float2 U = make_float2(L[len - 1].x - cx, L[len - 1].y - cy);
-        for (int k = 0; k < len; k++) {
+        const float2 last = len == KMAX ? L[KMAX - 1] : L[KMAX > 1 ? KMAX - 2 : 0];
+        float2 U = make_float2(last.x - cx, last.y - cy);
+#pragma unroll
+        for (int k = 0; k < KMAX; k++) {
+            if (k >= len) break;
             const float2 V = make_float2(L[k].x - cx, L[k].y - cy);
             if (V.x == U.x && V.y == U.y) continue;  // repeated vertex: no edge (geometry_utils.py:203-204)
             const float A = U.x * V.y - U.y * V.x;
@@ -1351,7 +1356,8 @@ __device__ __forceinline__ bool tri_box(const float2 (&V)[3], const float2 (&D)[
 // anchor); a grid cell's rectangle is placed relative to the anchor in float64
 // and rounded, with an error far below the slack.  (Ranges and vertices in
 // float64 were 90 instructions of the float64 unit per cell, 20 cycles each:
-// 4.0 ms for 16M cells, now 2.9.)
+// 4.0 ms for 16M cells, with float32 ones 2.9, with the vertices in registers
+// at 24 warps per SM 2.4.)
 // Triangles that are surely counter-clockwise take tri_box; other cells of
 // up to 4 vertices clip_box; cells with fewer than 3 vertices, more than 4
 // (clipping them cost more build time than it saved queries in measurements
@@ -1405,8 +1411,9 @@ __device__ __forceinline__ void cand_cell(int64_t j, float4 b, const double2* __
         ax = v.x - ox;
         ay = v.y - oy;
         L[0] = make_float2(0.0f, 0.0f);
-        for (int k = 1; k < len; k++) {
-            L[k] = rel[k - 1];
+#pragma unroll
+        for (int k = 1; k < (KMAX <= 4 ? KMAX : 1); k++) {
+            L[k] = k < len ? rel[k - 1] : make_float2(0.0f, 0.0f);
             Lm = fmaxf(Lm, fmaxf(fabsf(L[k].x), fabsf(L[k].y)));
             clip = clip && isfinite(L[k].x) && isfinite(L[k].y);
         }
@@ -1499,7 +1506,7 @@ __device__ __forceinline__ void cand_cell(int64_t j, float4 b, const double2* __
 }
 
 template <int MODE, int KMAX>
-__global__ void k_cand_lists(const float4* __restrict__ box, const double2* __restrict__ poly,
+__global__ void __launch_bounds__(256, 3) k_cand_lists(const float4* __restrict__ box, const double2* __restrict__ poly,
                              const float4* __restrict__ polyf, const uint8_t* __restrict__ plen32, int K, int64_t n, double ox, double oy, int gnx,
                              int gny, double x0, double y0, double sx, double sy, double cw, double ch, double m,
                              float Mf, float e2f, float ea, unsigned long long* __restrict__ count,
@@ -2198,7 +2205,10 @@ static void launch_cand_lists(const ct_tree* t, bool fill, double M, const CandS
         C.count, MODE == 1 ? t->cand_off : nullptr, MODE == 1 ? t->cand_idx : nullptr,                             \
         MODE == 1 ? (float4*)t->cand_lbox : nullptr, t->error_word, C.rec, MODE == 1 ? C.rec.ovf : nullptr,         \
         C.rec.ovf_count)
-    if (t->n_max_vert <= 4) {
+    if (t->n_max_vert <= 3) {
+        if (fill) CT_CAND_LISTS(1, 3);
+        else CT_CAND_LISTS(2, 3);
+    } else if (t->n_max_vert == 4) {
         if (fill) CT_CAND_LISTS(1, 4);
         else CT_CAND_LISTS(2, 4);
     } else {
