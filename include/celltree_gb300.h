@@ -502,13 +502,15 @@ int ct_count_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, con
 /* Large batches in one traversal: the counting pass keeps every terminal node
  * with pairs (a leaf, or a subtree inside the box) as a record, ct_box_records_size
  * bytes for `capacity` of them; the writing call expands them, or, when there
- * were more, traverses again.  Same output as ct_count_boxes + ct_write_boxes. */
+ * were more, traverses again.  Same output as ct_count_boxes + ct_write_boxes;
+ * inside (optional, total_pairs bytes): 1 for the pairs known to have the cell
+ * inside the box. */
 size_t ct_box_records_size(int64_t capacity);
 int ct_count_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
                            void* records, int64_t capacity, void* stream);
 int ct_write_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
-                           const int64_t* offsets, const void* records, int64_t capacity, int64_t* ii, int64_t* jj,
-                           void* stream);
+                           const int64_t* offsets, const void* records, int64_t capacity, int64_t total_pairs,
+                           int64_t* ii, int64_t* jj, uint8_t* inside, void* stream);
 /* The same counts and scratch by one thread per box: faster for boxes of about
  * a cell that come in mesh order (query faces). */
 int ct_count_small_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
@@ -674,10 +676,11 @@ int ct_pair_order(const int64_t* faces_a, int32_t n_max_vert_a, const int64_t* i
                   size_t workspace_bytes, void* stream);
 
 /* The same order for (box, face) pairs whose faces come up many times each:
- * the faces' lengths are taken once (n_faces rows). */
+ * the faces' lengths are taken once (n_faces rows).  inside: NULL, or a flag
+ * per pair that parts each class in two. */
 size_t ct_box_pair_order_workspace_size(int64_t n, int64_t n_faces);
 int ct_box_pair_order(const int64_t* faces, int32_t n_max_vert, int64_t n_faces, const int64_t* indices_face,
-                      int64_t n, int32_t* order, void* workspace, size_t workspace_bytes, void* stream);
+                      const uint8_t* inside, int64_t n, int32_t* order, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Keeps the pairs with area > 0 (area != NULL) or flag != 0 (celltree.py:183,
  * 226, 268); outputs have capacity n; *total_host = kept count (synchronises). */

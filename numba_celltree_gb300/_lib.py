@@ -200,7 +200,7 @@ SIGNATURES = {
     "ct_pair_order_workspace_size": (_SZ, [_I64]),
     "ct_pair_order": (ctypes.c_int, [_P, _I32, _P, _P, _I32, _P, _I64, _P, _P, _SZ, _P]),
     "ct_box_pair_order_workspace_size": (_SZ, [_I64, _I64]),
-    "ct_box_pair_order": (ctypes.c_int, [_P, _I32, _I64, _P, _I64, _P, _P, _SZ, _P]),
+    "ct_box_pair_order": (ctypes.c_int, [_P, _I32, _I64, _P, _P, _I64, _P, _P, _SZ, _P]),
     "ct_liang_barsky_line_box_clip": (ctypes.c_int, [_P, _P, _P, _I64, _P, _P, _P, _P]),
     "ct_points_in_triangles": (ctypes.c_int, [_P, _P, _I64, _P, _I32, _I64, _P, _D, _P, _P, _P]),
     "ct_csr_workspace_size": (_SZ, [_I64]),
@@ -213,7 +213,8 @@ SIGNATURES = {
     "ct_count_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I32, _P]),
     "ct_box_records_size": (_SZ, [_I64]),
     "ct_count_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _P]),
-    "ct_write_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _P, _P, _P]),
+    "ct_write_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _I64, _P, _P,
+                                              _P, _P]),
     "ct_count_small_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I32, _P]),
     "ct_write_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _P, _I32, _I64, _I32, _P, _P,
                                            _P, ctypes.c_size_t, _P]),

@@ -315,14 +315,15 @@ class CellTree2d(CellTree2dBase):
     def _intersect_boxes_dev(self, b_d, budget=None):
         t = self._tree
         torch = _device.torch()
-        res = t.locate_boxes(b_d, budget=budget)
+        res = t.locate_boxes(b_d, budget=budget, inside=True)
         if res is None:
             return None
-        ii, jj = res
+        ii, jj, inside = res
         n = int(ii.shape[0])
         area = _device.empty((n,), torch.float64, t.device)
         t.reset_error()
-        order = t.pair_order(None, 4, ii, t.elements, t.K, jj)
+        order = t.pair_order(None, 4, ii, t.elements, t.K, jj, inside)
+        del inside, res
         _lib.check(
             _lib.load().ct_box_area_of_intersection_ordered(
                 _device.ptr(b_d), _device.ptr(t.vertices), _device.ptr(t.elements), t.K, _device.ptr(ii),

@@ -604,13 +604,15 @@ class _GpuTree:
     BOX_RECORDS = 256
     BOX_RECORDS_MIN = 64
 
-    def locate_boxes(self, boxes_d, config=None, budget=None, small=False):
+    def locate_boxes(self, boxes_d, config=None, budget=None, small=False, inside=False):
         """Pairs (box, cell) of every box query, box-major in upstream order;
         with `budget`, returns None instead when the pairs would exceed it
         (the per-box counts are left in self.last_counts).  `small`: the boxes
         are about a cell each and come in mesh order (counted by a thread
-        each)."""
+        each).  `inside`: also a byte per pair, 1 where the cell is known to
+        lie inside the box (None when the batch gives none)."""
         n = int(boxes_d.shape[0])
+        ask = inside
         if config is None:
             config = self.cached("boxes", n)
         torch = _device.torch()
@@ -652,10 +654,13 @@ class _GpuTree:
         # the writing pass repeats the counting pass's traversal: a condition
         # it could report has been reported by the count
         if recs is not None:
+            # (only where pair_order makes use of it)
+            inside = inside and self.lengths_once(total, self.n, self.K)
+            whole = _device.empty((total,), torch.uint8, self.device) if inside else None
             _lib.check(lib.ct_write_boxes_records(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
-                                                  _device.ptr(offsets), _device.ptr(recs), most, _device.ptr(ii),
-                                                  _device.ptr(jj), st), "locate_boxes")
-            return ii, jj
+                                                  _device.ptr(offsets), _device.ptr(recs), most, total, _device.ptr(ii),
+                                                  _device.ptr(jj), _device.ptr(whole), st), "locate_boxes")
+            return (ii, jj, whole) if ask else (ii, jj)
         if spec is not None:
             jm = int(config.get("job_cells") or 0)
             wsz = int(lib.ct_write_boxes_workspace_size(total, jm))
@@ -666,14 +671,14 @@ class _GpuTree:
                                         total, jm, _device.ptr(ii), _device.ptr(jj), _device.ptr(ws), wsz, st),
                 "locate_boxes",
             )
-            return ii, jj
+            return (ii, jj, None) if ask else (ii, jj)
         if total < self.BOX_JOBS_MIN_PAIRS:
             _lib.check(
                 lib.ct_write_boxes(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
                                    _device.ptr(offsets), _device.ptr(ii), _device.ptr(jj), st),
                 "locate_boxes",
             )
-            return ii, jj
+            return (ii, jj, None) if ask else (ii, jj)
         jm = int(config.get("job_cells") or 0)
         wsz = int(lib.ct_write_boxes_workspace_size(total, jm))
         ws = _device.empty((wsz,), torch.uint8, self.device)
@@ -683,7 +688,7 @@ class _GpuTree:
                                   _device.ptr(ws), wsz, st),
             "locate_boxes",
         )
-        return ii, jj
+        return (ii, jj, None) if ask else (ii, jj)
 
     # cells from which a tree's node and cell records (about 130 bytes a cell)
     # outgrow the 129 MB of L2, so that the order of the queries matters: 1M
@@ -793,7 +798,10 @@ class _GpuTree:
     # (a pass over the cells, 47 us for 5M) instead of from every pair's row
     PAIR_LENGTHS_MIN = 4
 
-    def pair_order(self, fa, Ka: int, ia, fb, Kb: int, ib):
+    def lengths_once(self, pairs: int, cells: int, K: int) -> bool:
+        return K > 3 and pairs >= max(self.PAIR_ORDER_MIN, self.PAIR_LENGTHS_MIN * cells)
+
+    def pair_order(self, fa, Ka: int, ia, fb, Kb: int, ib, inside=None):
         """Processing order of the per-pair kernels (pairs of equal polygon
         lengths side by side), or None when every pair has the same lengths
         or the batch is small."""
@@ -804,12 +812,12 @@ class _GpuTree:
         torch = _device.torch()
         lib = _lib.load()
         order = _device.empty((n,), torch.int32, self.device)
-        if fa is None and n >= self.PAIR_LENGTHS_MIN * int(fb.shape[0]):
+        if fa is None and self.lengths_once(n, int(fb.shape[0]), Kb):
             nbytes = int(lib.ct_box_pair_order_workspace_size(n, int(fb.shape[0])))
             ws = _device.empty((nbytes,), torch.uint8, self.device)
-            _lib.check(lib.ct_box_pair_order(_device.ptr(fb), Kb, int(fb.shape[0]), _device.ptr(ib), n,
-                                             _device.ptr(order), _device.ptr(ws), nbytes, _device.stream()),
-                       "pair order")
+            _lib.check(lib.ct_box_pair_order(_device.ptr(fb), Kb, int(fb.shape[0]), _device.ptr(ib),
+                                             _device.ptr(inside), n, _device.ptr(order), _device.ptr(ws), nbytes,
+                                             _device.stream()), "pair order")
             return order
         nbytes = int(lib.ct_pair_order_workspace_size(n))
         ws = _device.empty((nbytes,), torch.uint8, self.device)

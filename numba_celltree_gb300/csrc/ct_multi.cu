@@ -328,6 +328,7 @@ struct BoxRecs {
     int4* rec;
     unsigned long long* count;  // records asked for
     int64_t cap;
+    uint8_t* inside;  // optional, per pair: the cell lies in a subtree inside the box
 };
 constexpr int REC_FLAG = (int)0x80000000u;
 
@@ -373,7 +374,7 @@ __device__ __forceinline__ void box_outputs(const TreeQ& T, int lane, int64_t sh
             for (int z = (int)o; z > 0; z--) kh &= kh - 1u;
             j = kp + __ffs(kh) - 1;
         }
-        put(ki, ka + o, j);
+        put(ki, ka + o, j, kall);
     }
 }
 
@@ -483,10 +484,11 @@ struct BoxWalk {
                 if (overlaps(S, ptr + k)) put(at, id, r++, ptr + k);
             share = 0;
         }
-        box_outputs(T, lane, share, at + rank, id, ptr, size, hit, all, [&](int i, int64_t k, int j) {
+        box_outputs(T, lane, share, at + rank, id, ptr, size, hit, all, [&](int i, int64_t k, int j, bool whole) {
             if (WRITE) {
                 ii[k] = i;
                 jj[k] = T.bbi[j];
+                if (recs.inside) recs.inside[k] = whole;
             } else {
                 spec[k] = (int)T.bbi[j];
             }
@@ -563,9 +565,10 @@ __global__ void __launch_bounds__(256) k_box_records(TreeQ T, const double4* __r
     const unsigned long long asked = *recs.count;
     if (asked > (unsigned long long)recs.cap) return;  // not all were kept: the boxes are walked again
     const int64_t n = (int64_t)asked, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    auto put = [&](int i, int64_t k, int j) {
+    auto put = [&](int i, int64_t k, int j, bool whole) {
         ii[k] = i;
         jj[k] = T.bbi[j];
+        if (recs.inside) recs.inside[k] = whole;
     };
     for (int64_t r0 = 32 * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r0 < n; r0 += 32 * warps) {
         const bool have = r0 + lane < n;
@@ -577,7 +580,7 @@ __global__ void __launch_bounds__(256) k_box_records(TreeQ T, const double4* __r
             const dbox b = load_box(reinterpret_cast<const double*>(boxes + id));
             int64_t k = at;
             for (int c = 0; c < r.w; c++)
-                if (boxes_intersect(b, leaf_box(T, r.z + c))) put(id, k++, r.z + c);
+                if (boxes_intersect(b, leaf_box(T, r.z + c))) put(id, k++, r.z + c, false);
         }
         const int64_t share = !have || big ? 0 : all ? r.w : __popc((unsigned)r.w);
         box_outputs(T, lane, share, at, id, r.z, all ? r.w : 0, all ? 0u : (unsigned)r.w, all, put);
@@ -2377,7 +2380,8 @@ __global__ void k_face_lengths(const int64_t* __restrict__ faces, int K, int64_t
 // batches with many pairs per face, whose rows are read from DRAM for every
 // pair otherwise (91M pairs on 5M faces 1.65 -> 0.42 ms).
 __global__ void __launch_bounds__(256) k_box_pair_keys(const uint8_t* __restrict__ length,
-                                                       const int64_t* __restrict__ ib, int64_t n,
+                                                       const int64_t* __restrict__ ib,
+                                                       const uint8_t* __restrict__ inside, int64_t n,
                                                        unsigned* __restrict__ key) {
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
@@ -2386,10 +2390,10 @@ __global__ void __launch_bounds__(256) k_box_pair_keys(const uint8_t* __restrict
 #pragma unroll
         for (int u = 0; u < 4; u++) b[u] = ib[min(i0 + u * step, n - 1)];
 #pragma unroll
-        for (int u = 0; u < 4; u++) l[u] = length[b[u]];
+        for (int u = 0; u < 4; u++) l[u] = 2 * min((int)length[b[u]] - 3, 7) + (inside && inside[min(i0 + u * step, n - 1)] ? 1 : 0);
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (i0 + u * step < n) key[i0 + u * step] = (unsigned)(8 + min(l[u] - 3, 7));
+            if (i0 + u * step < n) key[i0 + u * step] = (unsigned)l[u];
     }
 }
 
@@ -2909,7 +2913,7 @@ static int walk_tasks(int64_t n) {
 template <int MODE>
 static void launch_box_walk(const TreeQ& T, const double4* boxes, int64_t n, const int* order, int64_t* cnt_or_off,
                             int64_t* ii, int64_t* jj, int* spec, int spcap, const int64_t* spec_cnt,
-                            cudaStream_t st, BoxRecs recs = {nullptr, nullptr, 0}) {
+                            cudaStream_t st, BoxRecs recs = {nullptr, nullptr, 0, nullptr}) {
     const int per_warp = walk_tasks(n);
     k_box_walk<MODE><<<grid_of((n + per_warp - 1) / per_warp, WALK_WARPS), 32 * WALK_WARPS, 0, st>>>(
         T, boxes, n, order, per_warp, cnt_or_off, ii, jj, spec, spcap, spec_cnt, recs);
@@ -3127,8 +3131,8 @@ int ct_count_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const 
 }
 
 // records: a count, then the records
-static BoxRecs box_recs(void* records, int64_t capacity) {
-    return BoxRecs{(int4*)((char*)records + 256), (unsigned long long*)records, capacity};
+static BoxRecs box_recs(void* records, int64_t capacity, uint8_t* inside) {
+    return BoxRecs{(int4*)((char*)records + 256), (unsigned long long*)records, capacity, inside};
 }
 
 size_t ct_box_records_size(int64_t capacity) { return 256 + sizeof(int4) * (size_t)(capacity > 0 ? capacity : 1); }
@@ -3147,23 +3151,24 @@ int ct_count_boxes_records(const ct_tree* t, const double* boxes, int64_t n, con
     CT_CUDA(cudaMemsetAsync(records, 0, sizeof(unsigned long long), st));
     if (n == 0) return CT_OK;
     launch_box_walk<BOX_RECORD>(make_q(t), (const double4*)boxes, n, order, counts, nullptr, nullptr, nullptr, 0, nullptr,
-                                st, box_recs(records, capacity));
+                                st, box_recs(records, capacity, nullptr));
     CT_CHECK_LAUNCH("count_boxes_records");
     return CT_OK;
 }
 
 int ct_write_boxes_records(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order,
-                           const int64_t* offsets, const void* records, int64_t capacity, int64_t* ii, int64_t* jj,
-                           void* stream) {
+                           const int64_t* offsets, const void* records, int64_t capacity, int64_t total_pairs,
+                           int64_t* ii, int64_t* jj, uint8_t* inside, void* stream) {
     int s = check_tree(t);
     if (s) return s;
     if (n == 0) return CT_OK;
     if (!records || capacity < 1) return ct_fail(CT_ERR_ARG, "no records");
-    if (deep_tree(t)) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);
     cudaStream_t st = (cudaStream_t)stream;
+    if (inside && total_pairs > 0) CT_CUDA(cudaMemsetAsync(inside, 0, (size_t)total_pairs, st));
+    if (deep_tree(t)) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);
     const TreeQ T = make_q(t);
     const double4* B = (const double4*)boxes;
-    const BoxRecs R = box_recs((void*)records, capacity);
+    const BoxRecs R = box_recs((void*)records, capacity, inside);
     k_box_records<<<(unsigned)std::min<int64_t>((capacity + 255) / 256, 152 * 64), 256, 0, st>>>(T, B, R, offsets, ii, jj);
     launch_box_walk<BOX_WRITE>(T, B, n, order, (int64_t*)offsets, ii, jj, nullptr, 0, nullptr, st, R);
     CT_CHECK_LAUNCH("write_boxes_records");
@@ -3309,8 +3314,8 @@ int ct_pair_order(const int64_t* fa, int32_t Ka, const int64_t* ia, const int64_
     return ct_radix_pass(kin, nullptr, n, 0, kout, order, (char*)ws + 2 * part, ws_bytes - 2 * part, stream);
 }
 
-int ct_box_pair_order(const int64_t* fb, int32_t Kb, int64_t n_faces, const int64_t* ib, int64_t n, int32_t* order,
-                      void* ws, size_t ws_bytes, void* stream) {
+int ct_box_pair_order(const int64_t* fb, int32_t Kb, int64_t n_faces, const int64_t* ib, const uint8_t* inside,
+                      int64_t n, int32_t* order, void* ws, size_t ws_bytes, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (n < 0 || n > INT32_MAX || n_faces < 0) return ct_fail(CT_ERR_ARG, "pair or face count out of range");
     if (!ws || ws_bytes < ct_box_pair_order_workspace_size(n, n_faces))
@@ -3323,7 +3328,7 @@ int ct_box_pair_order(const int64_t* fb, int32_t Kb, int64_t n_faces, const int6
     char* rest = (char*)kout + part;
     k_face_lengths<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_of(n_faces, 256), 152 * 32)), 256, 0, st>>>(
         fb, Kb, n_faces, length);
-    k_box_pair_keys<<<(unsigned)std::min<int64_t>(grid_of(n, 256), 152 * 8), 256, 0, st>>>(length, ib, n, kin);
+    k_box_pair_keys<<<(unsigned)std::min<int64_t>(grid_of(n, 256), 152 * 8), 256, 0, st>>>(length, ib, inside, n, kin);
     CT_CHECK_LAUNCH("pair keys");
     return ct_radix_pass(kin, nullptr, n, 0, kout, order, rest, ws_bytes - (size_t)(rest - (char*)ws), stream);
 }

@@ -26,6 +26,11 @@ def test_records(oracle, cells_per_leaf, n, room):
     if n > 5:
         boxes[1:5] = [[3.0, 3.0, 2.0, 5.0], [7.0, 5.0, 2.0, 5.0], [np.nan, 5.0, 2.0, 5.0], [-np.inf, np.inf, 10.0, 11.0]]
     i, j = oracle.OracleCellTree2d(xy, f, -1, 4, cells_per_leaf).locate_boxes(boxes)
-    t.BOX_RECORDS, t.BOX_RECORDS_MIN = room, 1
-    gi, gj = t.locate_boxes(torch.as_tensor(boxes, device="cuda"))
-    assert np.array_equal(gi.cpu().numpy(), i) and np.array_equal(gj.cpu().numpy(), j)
+    t.BOX_RECORDS, t.BOX_RECORDS_MIN, t.lengths_once = room, 1, lambda *_: True
+    gi, gj, inside = (x.cpu().numpy() for x in t.locate_boxes(torch.as_tensor(boxes, device="cuda"), inside=True))
+    assert np.array_equal(gi, i) and np.array_equal(gj, j)
+    bb, flag = t.bb_coords.cpu().numpy()[gj], inside.astype(bool)
+    b = boxes[gi]
+    assert np.isin(inside, (0, 1)).all() and flag[gi == 0].all()
+    held = (b[:, 0] < bb[:, 0]) & (bb[:, 1] < b[:, 1]) & (b[:, 2] < bb[:, 2]) & (bb[:, 3] < b[:, 3])
+    assert held[flag].all()

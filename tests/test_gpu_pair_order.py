@@ -30,9 +30,16 @@ def test_same_order(k, n):
         if rows:
             _lib.check(lib.ct_pair_order(None, 4, P(ib), P(faces), k, P(jb), n, P(order), P(ws), int(size), st), "order")
         else:
-            _lib.check(lib.ct_box_pair_order(P(faces), k, m, P(jb), n, P(order), P(ws), int(size), st), "order")
+            _lib.check(lib.ct_box_pair_order(P(faces), k, m, P(jb), None, n, P(order), P(ws), int(size), st), "order")
         got.append(order)
+    inside = (torch.rand(n, device="cuda", generator=gen) < 0.5).to(torch.uint8)
+    order = torch.empty(n, dtype=torch.int32, device="cuda")
+    size = int(lib.ct_box_pair_order_workspace_size(n, m))
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.ct_box_pair_order(P(faces), k, m, P(jb), P(inside), n, P(order), P(ws), size, _device.stream()), "order")
     classes = (length.flatten()[jb] - 3).clamp(max=7)
+    halves = 2 * classes + inside
+    assert torch.equal(halves[order.long()], torch.sort(halves).values)
     for order in got:
         assert torch.equal(torch.sort(order).values, torch.arange(n, dtype=torch.int32, device="cuda"))
         assert torch.equal(classes[order.long()], torch.sort(classes).values)
