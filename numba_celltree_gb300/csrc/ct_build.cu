@@ -1919,7 +1919,9 @@ static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, boo
         double width = n_roots;  // records of the level, at most
         // the counters and the ranges of the levels run lie side by side
         const size_t lvl_off = (size_t)((char*)ws.lvl_b - (char*)ws.cnt), end_off = (size_t)((char*)ws.lvl_e - (char*)ws.cnt);
-        std::vector<char> state(end_off + sizeof(int) * (DEV_MAX_LEVELS + 1));
+        alignas(16) char state[2048];
+        const size_t state_bytes = end_off + sizeof(int) * (DEV_MAX_LEVELS + 1);
+        if (state_bytes > sizeof(state)) return ct_fail(CT_ERR_DEVICE, "builder counters do not fit their copy");
         while (true) {
             for (int i = 0; i < ahead; i++) {
                 const double pending = std::min(width, n_roots + (double)n / SMALL);
@@ -1938,13 +1940,13 @@ static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, boo
                 width = std::min(2.0 * width, 2.0 * n_roots + 2.0 * n / SMALL);
             }
             CT_CHECK_LAUNCH("phase A levels");
-            CT_CUDA(cudaMemcpyAsync(state.data(), ws.cnt, state.size(), cudaMemcpyDeviceToHost, st));
+            CT_CUDA(cudaMemcpyAsync(state, ws.cnt, state_bytes, cudaMemcpyDeviceToHost, st));
             CT_CUDA(cudaStreamSynchronize(st));
-            memcpy(&hc, state.data(), sizeof(Counters));
+            memcpy(&hc, state, sizeof(Counters));
             if (hc.err & 0x80000000u)
                 return ct_fail(CT_ERR_WORKSPACE, "builder tile or node-record capacity exceeded (unbalanced tree)");
-            const int* lb = reinterpret_cast<const int*>(state.data() + lvl_off);
-            const int* le = reinterpret_cast<const int*>(state.data() + end_off);
+            const int* lb = reinterpret_cast<const int*>(state + lvl_off);
+            const int* le = reinterpret_cast<const int*>(state + end_off);
             for (int k = 1; k < hc.nlev; k++) {
                 level_b.push_back(lb[k]);
                 level_e.push_back(le[k]);
