@@ -211,8 +211,8 @@ int ct_build_emit(const void* workspace, int64_t n_elements, int32_t n_buckets, 
  * the GPU (other streams, other host threads) race.
  * Extremely unbalanced trees that exceed the builder's record capacity return
  * CT_ERR_WORKSPACE; use ct_build_tree with a larger capacity_factor.
- * Not capturable in a CUDA graph: it synchronises the stream once per tree
- * level (ct_build_forest_async is the capturable build). */
+ * Not capturable in a CUDA graph: it synchronises the stream
+ * (ct_build_forest_async is the capturable build). */
 int ct_build_tree_noalloc(const double* bb_coords, int64_t n_elements, int32_t n_buckets, int64_t cells_per_leaf,
                           int64_t* child, double* Lmax, double* Rmin, int64_t* ptr, int64_t* size, uint8_t* dim,
                           int64_t node_capacity, int64_t* bb_indices, int64_t* n_nodes_host, int32_t* max_depth_host,

@@ -589,18 +589,19 @@ class _GpuTree:
     # pairs from which subtrees inside a box are written by a warp each after
     # the traversal (below, the extra launch costs more than it saves)
     BOX_JOBS_MIN_PAIRS = 1 << 20
-    # the counting pass keeps each box's first SPEC_CAP pairs (batches up to
+    # boxes counted by a thread each, and batches without room for records
+    # (below): the counting pass keeps each box's first SPEC_CAP pairs (up to
     # SPEC_MAX_BOXES boxes; SPEC_CAP_LARGE beyond, scratch up to
     # SPEC_MAX_BYTES), so boxes whose pairs fit are traversed once;
-    # SPEC_MAX_BOXES = 0 switches it off
+    # SPEC_MAX_BOXES = 0 switches both off
     SPEC_MAX_BOXES = 1 << 16
     SPEC_CAP = 64
     SPEC_CAP_LARGE = 16
     SPEC_MAX_BYTES = 1 << 30
-    # other batches keep terminal nodes instead: room for BOX_RECORDS of 16
-    # bytes a box, as far as SPEC_MAX_BYTES goes (250k boxes of 0.2 to 100
-    # cells a side have 77 on average); below BOX_RECORDS_MIN a box the pairs
-    # of small boxes are kept after all
+    # batches walked by warps keep terminal nodes instead: room for BOX_RECORDS
+    # of 16 bytes a box, as far as SPEC_MAX_BYTES goes and at least
+    # BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
+    # average, 10k of 0.2 to 4 cells 6)
     BOX_RECORDS = 256
     BOX_RECORDS_MIN = 64
 
