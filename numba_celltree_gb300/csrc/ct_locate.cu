@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(LOC_THREADS)
 // once by open_one, what that leaves by the traversal (stack in local memory).
 // The stages of large batches are launches of their own, each with its
 // queries packed; at a few thousand points their launches and dependent
-// chains are the time: 1000 points 54 -> 22 us of kernels.
+// chains are the time: 1000 points 54 -> 21 us of kernels.
 constexpr int SMALL_STACK = 128;
 
 template <int KT>
@@ -895,6 +895,62 @@ __global__ void __launch_bounds__(128) k_small(const __grid_constant__ TreeL T, 
     if (!cells_one<KT>(T, pp, i, (int)i, out, nullptr)) return;
     const int r = open_one(T, pp);
     out[i] = r == OPEN_LEFT ? traverse_local<KT>(T, pts, (int)i) : (int64_t)r;
+}
+
+// The smallest batches, a warp per point: every listed cell on a lane of its
+// own, float32 first and exactly where that leaves it, so that a point is one
+// chain of loads (offsets, entry, cell, vertices) whatever its cells; with a
+// lane per point the launch lasted as long as the point with the most cells
+// left open, one after another (1000 points: 21 -> 6 us).
+template <int KT>
+__global__ void __launch_bounds__(128) k_small_warp(const __grid_constant__ TreeL T, const double2* __restrict__ pts,
+                                                    int64_t n, int64_t* __restrict__ out) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const double2 pp = pts[i];
+    float px, py, dpx, dpy;
+    PtSplit P;
+    to_frame(pp.x, T.ohx, T.olx, &px, &dpx, &P.xh, &P.xl);
+    to_frame(pp.y, T.ohy, T.oly, &py, &dpy, &P.yh, &P.yl);
+    const float fx = (px - T.gx0) * T.gsx, fy = (py - T.gy0) * T.gsy;
+    const float xl = __fsub_rd(px, dpx), xh = __fadd_ru(px, dpx);
+    const float yl = __fsub_rd(py, dpy), yh = __fadd_ru(py, dpy);
+    int best = -1;
+    bool left = false;
+    if (fx >= 0.0f && fx < (float)T.gnx && fy >= 0.0f && fy < (float)T.gny) {
+        const int64_t g = (int64_t)(int)fy * T.gnx + (int)fx;
+        const int64_t s0 = T.coff[g], s1 = T.coff[g + 1];
+        for (int64_t b0 = s0; b0 < s1; b0 += 32) {
+            const int64_t k = b0 + lane;
+            int j = 0, r = CELL_FALSE;
+            if (k < s1) {
+                const float4 b = T.cbox[k];
+                j = T.cidx[k];
+                if (!(xh < b.x || xl > b.y || yh < b.z || yl > b.w)) {
+                    const int len32 = (int)T.plen32[j];
+                    int f = LF_UNSURE;
+                    if (len32 >= 3) {
+                        const float4* cell = T.polyf + (size_t)j * T.S4;
+                        float dx, dy, errd;
+                        local_delta(P, cell[0], &dx, &dy, &errd);
+                        f = leaf_filter_joined(dx, dy, errd, T.dabs, T.tolf, reinterpret_cast<const float2*>(cell + 1),
+                                               len32);
+                    }
+                    r = f == LF_INSIDE ? CELL_TRUE : f == LF_OUTSIDE ? CELL_FALSE : cell_exact(T, pp, P, j);
+                }
+            }
+            left = __any_sync(FULL, left || r == CELL_LEFT);
+            for (unsigned m = __ballot_sync(FULL, r == CELL_TRUE); m; m &= m - 1u) {
+                const int c = __shfl_sync(FULL, j, __ffs(m) - 1);
+                best = best < 0 ? c : first_met(T, pp, best, c);
+            }
+        }
+    } else {  // off the grid: off the mesh, or the traversal
+        left = !(xh < T.bx0 || xl > T.bx1 || yh < T.by0 || yl > T.by1);
+    }
+    if (lane == 0) out[i] = left ? traverse_local<KT>(T, pts, (int)i) : best < 0 ? -1 : T.bbi[best];
 }
 
 // ---------------------------------------------------------------------------
@@ -2336,6 +2392,10 @@ int ct_locate_bin(const ct_tree* t, const double* points, int64_t n, int32_t sor
     return CT_OK;
 }
 
+// A warp per point up to this many points, a lane beyond (1000 points 6 against
+// 21 us, 16000 13 / 23, 32000 22 / 23, 64000 39 / 27).
+constexpr int64_t SMALL_WARP_MAX = 32768;
+
 // One launch for unsorted batches up to this many points (beyond, packing the
 // open queries pays for its launches).
 static bool small_batch(const TreeL& T, int64_t n, int32_t sort_bits) {
@@ -2369,6 +2429,14 @@ int ct_locate_fast(const ct_tree* t, const double* points, int64_t n, double tol
     const int fast_bpsm = (t->tune_fast_bpsm >= 1 && t->tune_fast_bpsm <= 32) ? t->tune_fast_bpsm : 16;
     const bool direct = lists && T.node_ptr;
     if (direct && small_batch(T, n, G)) {
+        if (n <= SMALL_WARP_MAX) {
+            const unsigned gw = (unsigned)((n + 3) / 4);
+            if (T.K == 3) k_small_warp<3><<<gw, 128, 0, st>>>(T, P, n, out);
+            else if (T.K == 4) k_small_warp<4><<<gw, 128, 0, st>>>(T, P, n, out);
+            else k_small_warp<32><<<gw, 128, 0, st>>>(T, P, n, out);
+            CT_CHECK_LAUNCH("locate small");
+            return CT_OK;
+        }
         const unsigned gs = (unsigned)((n + 127) / 128);
         if (T.K == 3) k_small<3><<<gs, 128, 0, st>>>(T, P, n, out);
         else if (T.K == 4) k_small<4><<<gs, 128, 0, st>>>(T, P, n, out);
