@@ -583,6 +583,10 @@ __device__ __forceinline__ int first_met(const TreeL& T, double2 pp, int j, int 
     return r;
 }
 
+// A warp per point up to this many points, a lane beyond (1000 points 6 against
+// 21 us, 16000 13 / 23, 32000 22 / 23, 64000 39 / 27).
+constexpr int64_t SMALL_WARP_MAX = 32768;
+
 // The cell of an open query (-1: none), or OPEN_LEFT.
 constexpr int OPEN_LEFT = -2;
 
@@ -628,6 +632,56 @@ __device__ __forceinline__ int open_one(const TreeL& T, double2 pp) {
     return left ? OPEN_LEFT : best < 0 ? -1 : (int)T.bbi[best];
 }
 
+// The same by a warp: every listed cell on a lane of its own, float32 first and
+// exactly where that leaves it, so that a point is one chain of loads (offsets,
+// entry, cell, vertices) whatever its cells.  With a lane per point a launch
+// over few points lasts as long as the point with the most cells, one after
+// another (1000 points: 21 -> 6 us; 800 open ones of 80k 45 -> 9 us).
+__device__ __forceinline__ int open_warp(const TreeL& T, double2 pp, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    float px, py, dpx, dpy;
+    PtSplit P;
+    to_frame(pp.x, T.ohx, T.olx, &px, &dpx, &P.xh, &P.xl);
+    to_frame(pp.y, T.ohy, T.oly, &py, &dpy, &P.yh, &P.yl);
+    const float fx = (px - T.gx0) * T.gsx, fy = (py - T.gy0) * T.gsy;
+    const float xl = __fsub_rd(px, dpx), xh = __fadd_ru(px, dpx);
+    const float yl = __fsub_rd(py, dpy), yh = __fadd_ru(py, dpy);
+    int best = -1;
+    bool left = false;
+    if (fx >= 0.0f && fx < (float)T.gnx && fy >= 0.0f && fy < (float)T.gny) {
+        const int64_t g = (int64_t)(int)fy * T.gnx + (int)fx;
+        const int64_t s0 = T.coff[g], s1 = T.coff[g + 1];
+        for (int64_t b0 = s0; b0 < s1; b0 += 32) {
+            const int64_t k = b0 + lane;
+            int j = 0, r = CELL_FALSE;
+            if (k < s1) {
+                const float4 b = T.cbox[k];
+                j = T.cidx[k];
+                if (!(xh < b.x || xl > b.y || yh < b.z || yl > b.w)) {
+                    const int len32 = (int)T.plen32[j];
+                    int f = LF_UNSURE;
+                    if (len32 >= 3) {
+                        const float4* cell = T.polyf + (size_t)j * T.S4;
+                        float dx, dy, errd;
+                        local_delta(P, cell[0], &dx, &dy, &errd);
+                        f = leaf_filter_joined(dx, dy, errd, T.dabs, T.tolf, reinterpret_cast<const float2*>(cell + 1),
+                                               len32);
+                    }
+                    r = f == LF_INSIDE ? CELL_TRUE : f == LF_OUTSIDE ? CELL_FALSE : cell_exact(T, pp, P, j);
+                }
+            }
+            left = __any_sync(FULL, left || r == CELL_LEFT);
+            for (unsigned m = __ballot_sync(FULL, r == CELL_TRUE); m; m &= m - 1u) {
+                const int c = __shfl_sync(FULL, j, __ffs(m) - 1);
+                best = best < 0 ? c : first_met(T, pp, best, c);
+            }
+        }
+    } else {  // off the grid: off the mesh, or the traversal
+        left = !(xh < T.bx0 || xl > T.bx1 || yh < T.by0 || yl > T.by1);
+    }
+    return left ? OPEN_LEFT : best < 0 ? -1 : (int)T.bbi[best];
+}
+
 // Stage 2b where the lists have what open_one needs: the open queries
 // (sorted positions in qlist), those it leaves to ovf.
 __global__ void __launch_bounds__(LOC_THREADS)
@@ -635,6 +689,19 @@ __global__ void __launch_bounds__(LOC_THREADS)
            const int* __restrict__ qlist, const int* __restrict__ qcount, int64_t n, int64_t* __restrict__ out,
            int* __restrict__ ovf, int* __restrict__ ovf_count) {
     const int64_t nq = min((int64_t)*qcount, n);
+    if (nq <= SMALL_WARP_MAX) {
+        const int lane = threadIdx.x & 31;
+        const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+        for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nq; t += warps) {
+            const int i = qlist[t], oi = order ? order[i] : i;
+            const int r = open_warp(T, pts[oi], lane);
+            if (lane == 0) {
+                if (r == OPEN_LEFT) ovf[atomicAdd(ovf_count, 1)] = oi;
+                else out[oi] = r;
+            }
+        }
+        return;
+    }
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nq; base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t t = base + threadIdx.x;
         bool left = false;
@@ -897,60 +964,14 @@ __global__ void __launch_bounds__(128) k_small(const __grid_constant__ TreeL T, 
     out[i] = r == OPEN_LEFT ? traverse_local<KT>(T, pts, (int)i) : (int64_t)r;
 }
 
-// The smallest batches, a warp per point: every listed cell on a lane of its
-// own, float32 first and exactly where that leaves it, so that a point is one
-// chain of loads (offsets, entry, cell, vertices) whatever its cells; with a
-// lane per point the launch lasted as long as the point with the most cells
-// left open, one after another (1000 points: 21 -> 6 us).
 template <int KT>
 __global__ void __launch_bounds__(128) k_small_warp(const __grid_constant__ TreeL T, const double2* __restrict__ pts,
                                                     int64_t n, int64_t* __restrict__ out) {
-    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= n) return;
-    const double2 pp = pts[i];
-    float px, py, dpx, dpy;
-    PtSplit P;
-    to_frame(pp.x, T.ohx, T.olx, &px, &dpx, &P.xh, &P.xl);
-    to_frame(pp.y, T.ohy, T.oly, &py, &dpy, &P.yh, &P.yl);
-    const float fx = (px - T.gx0) * T.gsx, fy = (py - T.gy0) * T.gsy;
-    const float xl = __fsub_rd(px, dpx), xh = __fadd_ru(px, dpx);
-    const float yl = __fsub_rd(py, dpy), yh = __fadd_ru(py, dpy);
-    int best = -1;
-    bool left = false;
-    if (fx >= 0.0f && fx < (float)T.gnx && fy >= 0.0f && fy < (float)T.gny) {
-        const int64_t g = (int64_t)(int)fy * T.gnx + (int)fx;
-        const int64_t s0 = T.coff[g], s1 = T.coff[g + 1];
-        for (int64_t b0 = s0; b0 < s1; b0 += 32) {
-            const int64_t k = b0 + lane;
-            int j = 0, r = CELL_FALSE;
-            if (k < s1) {
-                const float4 b = T.cbox[k];
-                j = T.cidx[k];
-                if (!(xh < b.x || xl > b.y || yh < b.z || yl > b.w)) {
-                    const int len32 = (int)T.plen32[j];
-                    int f = LF_UNSURE;
-                    if (len32 >= 3) {
-                        const float4* cell = T.polyf + (size_t)j * T.S4;
-                        float dx, dy, errd;
-                        local_delta(P, cell[0], &dx, &dy, &errd);
-                        f = leaf_filter_joined(dx, dy, errd, T.dabs, T.tolf, reinterpret_cast<const float2*>(cell + 1),
-                                               len32);
-                    }
-                    r = f == LF_INSIDE ? CELL_TRUE : f == LF_OUTSIDE ? CELL_FALSE : cell_exact(T, pp, P, j);
-                }
-            }
-            left = __any_sync(FULL, left || r == CELL_LEFT);
-            for (unsigned m = __ballot_sync(FULL, r == CELL_TRUE); m; m &= m - 1u) {
-                const int c = __shfl_sync(FULL, j, __ffs(m) - 1);
-                best = best < 0 ? c : first_met(T, pp, best, c);
-            }
-        }
-    } else {  // off the grid: off the mesh, or the traversal
-        left = !(xh < T.bx0 || xl > T.bx1 || yh < T.by0 || yl > T.by1);
-    }
-    if (lane == 0) out[i] = left ? traverse_local<KT>(T, pts, (int)i) : best < 0 ? -1 : T.bbi[best];
+    const int r = open_warp(T, pts[i], lane);
+    if (lane == 0) out[i] = r == OPEN_LEFT ? traverse_local<KT>(T, pts, (int)i) : (int64_t)r;
 }
 
 // ---------------------------------------------------------------------------
@@ -2391,10 +2412,6 @@ int ct_locate_bin(const ct_tree* t, const double* points, int64_t n, int32_t sor
     CT_CHECK_LAUNCH("locate order");
     return CT_OK;
 }
-
-// A warp per point up to this many points, a lane beyond (1000 points 6 against
-// 21 us, 16000 13 / 23, 32000 22 / 23, 64000 39 / 27).
-constexpr int64_t SMALL_WARP_MAX = 32768;
 
 // One launch for unsorted batches up to this many points (beyond, packing the
 // open queries pays for its launches).
