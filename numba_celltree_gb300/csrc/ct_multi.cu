@@ -1944,22 +1944,47 @@ __global__ void k_gather_results(const int64_t* __restrict__ perm, int64_t total
 // (31M hits of 1M segments: 2.6 ms) this reads the hits once and writes the
 // results once (1.3 ms).
 // ---------------------------------------------------------------------------
+// Hits of every segment: eight lanes a segment, the warp together for those
+// of more than 256 candidates (a warp per segment and 32 candidates at a time:
+// 1M segments 177 -> 80 us, 1000 sections 48 -> 35).
 __global__ void __launch_bounds__(256) k_hit_counts(const uint8_t* __restrict__ keep,
                                                     const int64_t* __restrict__ coff,
                                                     const int64_t* __restrict__ ccnt, const int* __restrict__ order,
                                                     int64_t n, int64_t* __restrict__ counts,
                                                     unsigned long long* __restrict__ longest) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const int64_t groups = ((int64_t)gridDim.x * blockDim.x) >> 3;
     int64_t most = 0;
-    for (int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < n; s += warps) {
-        const int64_t c0 = coff[s], m = ccnt[s];
-        int64_t c = 0;
-        for (int64_t k = 0; k < m; k += 32)
-            c += __popc(__ballot_sync(0xffffffffu, k + lane < m && keep[c0 + k + lane]));
+    // (the same number of rounds in all lanes of a warp)
+    for (int64_t s0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; s0 < n; s0 += groups) {
+        const int64_t s = s0 + (lane >> 3);
+        int64_t c0 = 0, m = 0, c = 0;
+        if (s < n) {
+            c0 = coff[s];
+            m = ccnt[s];
+        }
+        if (m <= 256)
+            for (int64_t k = sub; k < m; k += 8) c += keep[c0 + k] != 0;
+        for (unsigned w = __ballot_sync(FULL, m > 256 && sub == 0); w; w &= w - 1u) {
+            const int src = __ffs(w) - 1;
+            const int64_t wc0 = __shfl_sync(FULL, c0, src), wm = __shfl_sync(FULL, m, src);
+            int64_t x = 0;
+            for (int64_t k = lane; k < wm; k += 128) {
+                int h = keep[wc0 + k] != 0;
+#pragma unroll
+                for (int u = 1; u < 4; u++) h += k + 32 * u < wm && keep[wc0 + k + 32 * u] != 0;
+                x += h;
+            }
+            x += __shfl_xor_sync(FULL, x, 16);
+            x += __shfl_xor_sync(FULL, x, 8);
+            if ((lane >> 3) == (src >> 3)) c = x;  // summed over its eight lanes below
+        }
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o, 8);
         most = max(most, c);
-        if (lane == 0) counts[order ? (int64_t)order[s] : s] = c;
+        if (sub == 0 && s < n) counts[order ? (int64_t)order[s] : s] = c;
     }
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
     if (lane == 0 && most > 0) atomicMax(longest, (unsigned long long)most);
 }
 
@@ -3765,7 +3790,7 @@ int ct_edge_hit_counts(const uint8_t* keep, const int64_t* cand_off, const int64
     int64_t* sums = (int64_t*)ws;
     CT_CUDA(cudaMemsetAsync(sums + nb, 0, 2 * sizeof(int64_t), st));
     if (n > 0) {
-        k_hit_counts<<<(unsigned)std::min<int64_t>(grid_of(n, 8), 152 * 16), 256, 0, st>>>(
+        k_hit_counts<<<(unsigned)std::min<int64_t>(grid_of(n, 32), 152 * 16), 256, 0, st>>>(
             keep, cand_off, cand_cnt, order, n, counts, (unsigned long long*)(sums + nb + 1));
         k_scan_reduce<<<(unsigned)nb, SCAN_T, 0, st>>>(counts, n, sums);
         k_scan_sums<<<1, SCAN_T, 0, st>>>(sums, nb);
