@@ -1469,8 +1469,8 @@ struct CandRecs {
 // region meets, each counted in count[g] and, by MODE, recorded or written.
 template <int MODE, int KMAX>
 __device__ __forceinline__ void cand_cell(int64_t j, float4 b, const double2* __restrict__ poly,
-                                          const float4* __restrict__ polyf, const uint8_t* __restrict__ plen32, int K,
-                                          double ox, double oy, int gnx,
+                                          const float4* __restrict__ polyf, const uint8_t* __restrict__ plen,
+                                          const uint8_t* __restrict__ plen32, int K, double ox, double oy, int gnx,
                                           int gny, double x0, double y0, double sx, double sy, double cw, double ch,
                                           double m, float Mf, float e2f, float ea,
                                           unsigned long long* __restrict__ count, const int64_t* __restrict__ off,
@@ -1490,7 +1490,18 @@ __device__ __forceinline__ void cand_cell(int64_t j, float4 b, const double2* __
     float2 L[KMAX];
     float Lm = 0.0f;
     if (clip) {
-        const double2 v = poly[(size_t)j * K];
+        // the anchor is the first vertex that differs from the one before it
+        // (pack_cell): not vertex 0 where a ring is closed by repeating it
+        const double2* pv = poly + (size_t)j * K;
+        double2 v = pv[0];
+        const int full = plen ? (int)plen[j] : K;
+        if (full != len) {
+            double2 before = pv[full - 1];
+            for (int k = 1; k < full && v.x == before.x && v.y == before.y; k++) {
+                before = v;
+                v = pv[k];
+            }
+        }
         ax = v.x - ox;
         ay = v.y - oy;
         L[0] = make_float2(0.0f, 0.0f);
@@ -1590,8 +1601,9 @@ __device__ __forceinline__ void cand_cell(int64_t j, float4 b, const double2* __
 
 template <int MODE, int KMAX>
 __global__ void __launch_bounds__(256, 3) k_cand_lists(const float4* __restrict__ box, const double2* __restrict__ poly,
-                             const float4* __restrict__ polyf, const uint8_t* __restrict__ plen32, int K, int64_t n, double ox, double oy, int gnx,
-                             int gny, double x0, double y0, double sx, double sy, double cw, double ch, double m,
+                             const float4* __restrict__ polyf, const uint8_t* __restrict__ plen,
+                             const uint8_t* __restrict__ plen32, int K, int64_t n, double ox, double oy, int gnx, int gny,
+                             double x0, double y0, double sx, double sy, double cw, double ch, double m,
                              float Mf, float e2f, float ea, unsigned long long* __restrict__ count,
                              const int64_t* __restrict__ off,
                              int* __restrict__ idx, float4* __restrict__ lbox, unsigned int* __restrict__ err,
@@ -1599,8 +1611,8 @@ __global__ void __launch_bounds__(256, 3) k_cand_lists(const float4* __restrict_
     const int64_t nj = cells ? (int64_t)*cells_count : n;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nj; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = cells ? (int64_t)cells[t] : t;
-        cand_cell<MODE, KMAX>(j, box[j], poly, polyf, plen32, K, ox, oy, gnx, gny, x0, y0, sx, sy, cw, ch, m, Mf, e2f, ea, count,
-                              off, idx, lbox, err, rec);
+        cand_cell<MODE, KMAX>(j, box[j], poly, polyf, plen, plen32, K, ox, oy, gnx, gny, x0, y0, sx, sy, cw, ch, m, Mf,
+                              e2f, ea, count, off, idx, lbox, err, rec);
     }
 }
 
@@ -2128,11 +2140,11 @@ __global__ void k_fx_cand_lists(const __grid_constant__ ct_forest_index X, const
         unsigned long long* count = X.cand_count + go;
         const int64_t* off = MODE == 1 ? X.cand_off + go : nullptr;
         if (T.K <= 4)
-            cand_cell<MODE, 4>(j, b, T.poly, T.polyf, T.plen32, T.K, T.ox, T.oy, T.gnx, T.gny, (double)T.gx0, (double)T.gy0,
+            cand_cell<MODE, 4>(j, b, T.poly, T.polyf, T.plen, T.plen32, T.K, T.ox, T.oy, T.gnx, T.gny, (double)T.gx0, (double)T.gy0,
                                (double)T.gsx, (double)T.gsy, cw, ch, m, Mf, e2f, ea, count, off, X.cand_idx,
                                (float4*)X.cand_lbox, X.error_word, none);
         else
-            cand_cell<MODE, 32>(j, b, T.poly, T.polyf, T.plen32, T.K, T.ox, T.oy, T.gnx, T.gny, (double)T.gx0, (double)T.gy0,
+            cand_cell<MODE, 32>(j, b, T.poly, T.polyf, T.plen, T.plen32, T.K, T.ox, T.oy, T.gnx, T.gny, (double)T.gx0, (double)T.gy0,
                                 (double)T.gsx, (double)T.gsy, cw, ch, m, Mf, e2f, ea, count, off, X.cand_idx,
                                 (float4*)X.cand_lbox, X.error_word, none);
     }
@@ -2280,8 +2292,8 @@ static void launch_cand_lists(const ct_tree* t, bool fill, double M, const CandS
     unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
 #define CT_CAND_LISTS(MODE, KMAX)                                                                                  \
     k_cand_lists<MODE, KMAX><<<blocks, 256, 0, st>>>(                                                              \
-        (const float4*)t->cand_box, (const double2*)t->poly_f64, (const float4*)t->poly_f32, t->poly_len32,        \
-        t->n_max_vert, n, t->origin[0],                                                                            \
+        (const float4*)t->cand_box, (const double2*)t->poly_f64, (const float4*)t->poly_f32,                       \
+        t->n_max_vert == 3 ? nullptr : t->poly_len, t->poly_len32, t->n_max_vert, n, t->origin[0],                 \
         t->origin[1], t->grid_nx, t->grid_ny, t->grid_x0, t->grid_y0, t->grid_sx, t->grid_sy,                     \
         1.0 / (double)t->grid_sx, 1.0 / (double)t->grid_sy, grid_margin(t),                                       \
         float_up(M), float_up(grid_margin(t) + M), (float)(4.0 * (double)t->abs_eps),                             \
