@@ -290,10 +290,13 @@ int ct_locate_points(const ct_tree* tree, const double* points, int64_t n, doubl
  * ordered along a Morton curve over the tree bbox (radix sort by the top
  * sort_bits of a 24-bit key, 4096 x 4096 grid; sort_bits 0 = input order,
  * else 8, 16 or 24), located through the candidate lists (a float32 pass that
- * settles most queries) and a float32 traversal of the rest that collects
- * candidate cells for queries whose float32 leaf test is ambiguous, then
- * finished by float64 tests of those candidates (and a float64 traversal for
- * the rare query with too many candidates).  Above 2^23 queries the list
+ * settles most queries); the others' listed cells are tested exactly, and the
+ * rare query that leaves open is traversed.  Without lists, or for a tree
+ * whose node ranges do not nest, the others go through a float32 traversal
+ * that collects candidate cells for queries whose float32 leaf test is
+ * ambiguous, float64 tests of those candidates, and a float64 traversal for
+ * the rare query with too many candidates.  Unsorted batches of at most 65536
+ * queries with lists take one launch.  Above 2^23 queries the list
  * results go out through a bucketed scatter (the workspace's sort buffers).
  * Output identical to ct_locate_points.
  * Workspace: ct_locate_workspace_size(n, sort_bits) bytes. */
@@ -310,9 +313,11 @@ int ct_locate_fast(const ct_tree* tree, const double* points, int64_t n, double 
                    int64_t* out, void* workspace, size_t workspace_bytes, void* stream);
 int ct_locate_exact(const ct_tree* tree, const double* points, int64_t n, double tolerance, int32_t sort_bits,
                     int64_t* out, void* workspace, size_t workspace_bytes, void* stream);
-/* counts_host4: queries sent to the overflow pass, queries with candidate
- * records, candidate pairs, queries the candidate lists left to the
- * traversal -- of the last float32 pass (synchronises). */
+/* counts_host4: queries sent to the last (traversing) pass, queries with
+ * candidate records, candidate pairs (these two 0 where the listed cells are
+ * tested exactly), queries the candidate lists left open -- of the last
+ * float32 pass (synchronises).  All 0 after a batch that took one launch: it
+ * deferred nothing. */
 int ct_locate_deferred_count(const void* workspace, int64_t n, int32_t sort_bits, int64_t* counts_host4, void* stream);
 
 /* A batch of face trees (no upstream counterpart): the points of every tree

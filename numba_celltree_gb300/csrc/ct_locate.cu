@@ -946,6 +946,7 @@ __global__ void __launch_bounds__(LOC_THREADS)
 // queries packed; at a few thousand points their launches and dependent
 // chains are the time: 1000 points 54 -> 21 us of kernels.
 constexpr int SMALL_STACK = 128;
+constexpr int N_COUNTERS = 16;  // of the workspace (LocWS)
 
 template <int KT>
 __device__ __noinline__ int64_t traverse_local(const TreeL& T, const double2* __restrict__ pts, int i) {
@@ -953,9 +954,15 @@ __device__ __noinline__ int64_t traverse_local(const TreeL& T, const double2* __
     return traverse_exact<KT>(T, pts, i, s, 1);
 }
 
+// Nothing is deferred to a later pass: the workspace's counters say so.
+__device__ __forceinline__ void nothing_deferred(int* __restrict__ counters) {
+    if (blockIdx.x == 0 && threadIdx.x < N_COUNTERS) counters[threadIdx.x] = 0;
+}
+
 template <int KT>
 __global__ void __launch_bounds__(128) k_small(const __grid_constant__ TreeL T, const double2* __restrict__ pts,
-                                               int64_t n, int64_t* __restrict__ out) {
+                                               int64_t n, int64_t* __restrict__ out, int* __restrict__ counters) {
+    nothing_deferred(counters);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double2 pp = pts[i];
@@ -966,7 +973,8 @@ __global__ void __launch_bounds__(128) k_small(const __grid_constant__ TreeL T, 
 
 template <int KT>
 __global__ void __launch_bounds__(128) k_small_warp(const __grid_constant__ TreeL T, const double2* __restrict__ pts,
-                                                    int64_t n, int64_t* __restrict__ out) {
+                                                    int64_t n, int64_t* __restrict__ out, int* __restrict__ counters) {
+    nothing_deferred(counters);
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (i >= n) return;
@@ -2439,7 +2447,10 @@ int ct_locate_fast(const ct_tree* t, const double* points, int64_t n, double tol
     if (s) return s;
     LocWS L;
     carve_loc(ws, n, G, &L);
-    if (n == 0) return CT_OK;
+    if (n == 0) {
+        CT_CUDA(cudaMemsetAsync(L.counters, 0, N_COUNTERS * sizeof(int), st));
+        return CT_OK;
+    }
     const double2* P = (const double2*)points;
     const int* ord = G > 0 ? L.order : nullptr;
     size_t smem = (size_t)T.stack * LOC_THREADS * sizeof(int);
@@ -2460,20 +2471,20 @@ int ct_locate_fast(const ct_tree* t, const double* points, int64_t n, double tol
     if (direct && small_batch(T, n, G)) {
         if (n <= SMALL_WARP_MAX) {
             const unsigned gw = (unsigned)((n + 3) / 4);
-            if (T.K == 3) k_small_warp<3><<<gw, 128, 0, st>>>(T, P, n, out);
-            else if (T.K == 4) k_small_warp<4><<<gw, 128, 0, st>>>(T, P, n, out);
-            else k_small_warp<32><<<gw, 128, 0, st>>>(T, P, n, out);
+            if (T.K == 3) k_small_warp<3><<<gw, 128, 0, st>>>(T, P, n, out, L.counters);
+            else if (T.K == 4) k_small_warp<4><<<gw, 128, 0, st>>>(T, P, n, out, L.counters);
+            else k_small_warp<32><<<gw, 128, 0, st>>>(T, P, n, out, L.counters);
             CT_CHECK_LAUNCH("locate small");
             return CT_OK;
         }
         const unsigned gs = (unsigned)((n + 127) / 128);
-        if (T.K == 3) k_small<3><<<gs, 128, 0, st>>>(T, P, n, out);
-        else if (T.K == 4) k_small<4><<<gs, 128, 0, st>>>(T, P, n, out);
-        else k_small<32><<<gs, 128, 0, st>>>(T, P, n, out);
+        if (T.K == 3) k_small<3><<<gs, 128, 0, st>>>(T, P, n, out, L.counters);
+        else if (T.K == 4) k_small<4><<<gs, 128, 0, st>>>(T, P, n, out, L.counters);
+        else k_small<32><<<gs, 128, 0, st>>>(T, P, n, out, L.counters);
         CT_CHECK_LAUNCH("locate small");
         return CT_OK;
     }
-    CT_CUDA(cudaMemsetAsync(L.counters, 0, 64, st));
+    CT_CUDA(cudaMemsetAsync(L.counters, 0, N_COUNTERS * sizeof(int), st));
     unsigned grid_b =
         lists ? (unsigned)std::min<int64_t>((n + LOC_THREADS - 1) / LOC_THREADS, (int64_t)sms * fast_bpsm) : grid;
     // many sorted queries: list results by sorted position, then one bucketed scatter
