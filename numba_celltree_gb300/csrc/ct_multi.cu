@@ -314,11 +314,10 @@ struct WalkBox {  // 88 bytes: an odd number of 8-byte words, so lanes of differ
     unsigned long long kx0, kx1, ky0, ky1;
     float qx0, qx1, qy0, qy1;  // the box in the float32 frame, rounded inward
     float ox0, ox1, oy0, oy1;  // and outward
-    int64_t base;
-    int id;
+    int64_t base, id;
     bool keys, idx;
-    int64_t pad;
 };
+static_assert(sizeof(WalkBox) == 88, "see above");
 
 // A terminal node of a box's walk with pairs, kept by the counting pass: the
 // box (top bit: the whole subtree lies inside it), the rank of the first pair
@@ -335,8 +334,8 @@ constexpr int REC_FLAG = (int)0x80000000u;
 // The outputs of the lanes' terminal nodes (`share` each), 32 at a time:
 // put(box, output index, leaf position) per lane; whole subtrees give their
 // leaves by decreasing position, each leaf's cells by increasing position.
-template <class Put>
-__device__ __forceinline__ void box_outputs(const TreeQ& T, int lane, int64_t share, int64_t at, int id, int ptr,
+template <class Id, class Put>
+__device__ __forceinline__ void box_outputs(const TreeQ& T, int lane, int64_t share, int64_t at, Id id, int ptr,
                                             int size, unsigned hit, bool all, const Put& put) {
     const unsigned FULL = 0xffffffffu;
     int64_t incl = share;
@@ -356,7 +355,7 @@ __device__ __forceinline__ void box_outputs(const TreeQ& T, int lane, int64_t sh
         const int kp = __shfl_sync(FULL, ptr, k), ks = __shfl_sync(FULL, size, k);
         unsigned kh = __shfl_sync(FULL, hit, k);
         const int64_t ka = __shfl_sync(FULL, at, k);
-        const int ki = __shfl_sync(FULL, id, k);
+        const Id ki = __shfl_sync(FULL, id, k);
         const bool kall = __shfl_sync(FULL, (int)all, k) != 0;
         if (t >= total) continue;
         int j;
@@ -468,7 +467,7 @@ struct BoxWalk {
                 if (lane == 0) first = atomicAdd(recs.count, (unsigned long long)__popc(b));
                 first = __shfl_sync(FULL, first, 0) + __popc(b & ((1u << lane) - 1u));
                 if (keep && first < (unsigned long long)recs.cap)
-                    recs.rec[first] = make_int4(S.id | (all ? REC_FLAG : 0),
+                    recs.rec[first] = make_int4((int)S.id | (all ? REC_FLAG : 0),
                                                 (int)rank | (!all && size > 32 ? REC_FLAG : 0), ptr,
                                                 all || size > 32 ? size : (int)hit);
             }
@@ -476,7 +475,7 @@ struct BoxWalk {
         }
         if (!WRITE && !spec) return;
         const int64_t at = have ? S.base : 0;
-        const int id = have ? S.id : 0;
+        const int64_t id = have ? S.id : 0;
         int64_t share = WRITE ? c : min(c, max((int64_t)0, (int64_t)spcap - rank));
         if (!all && size > 32) {  // a large leaf: its own lane
             int64_t r = rank;
@@ -484,7 +483,7 @@ struct BoxWalk {
                 if (overlaps(S, ptr + k)) put(at, id, r++, ptr + k);
             share = 0;
         }
-        box_outputs(T, lane, share, at + rank, id, ptr, size, hit, all, [&](int i, int64_t k, int j, bool whole) {
+        box_outputs(T, lane, share, at + rank, id, ptr, size, hit, all, [&](int64_t i, int64_t k, int j, bool whole) {
             if (WRITE) {
                 ii[k] = i;
                 jj[k] = T.bbi[j];
@@ -543,7 +542,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const dou
                 S.ox1 = __double2float_ru(x1);
                 S.oy0 = __double2float_rd(y0);
                 S.oy1 = __double2float_ru(y1);
-                S.id = (int)i;
+                S.id = i;
                 S.base = WRITE ? cnt_or_off[i] : i * (int64_t)spcap;
             }
         }
