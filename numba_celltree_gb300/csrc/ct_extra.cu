@@ -147,7 +147,8 @@ __global__ void k_row_search(const int64_t* __restrict__ rows, int64_t n_pairs, 
 constexpr int CSR_SHORT = 8;
 
 // v[k] + v[k + o] for k < o, o = 4, 2, 1; entries above m are zeros (m, the
-// longest of the warp's short rows, is the same in all lanes).
+// longest of the warp's short rows, is the same in all lanes).  A sum that
+// starts from 0.0 never is -0.0, so neither is this one.
 __device__ __forceinline__ double csr_tree(double (&v)[CSR_SHORT], int m) {
     if (m > 4) {
 #pragma unroll
@@ -157,7 +158,8 @@ __device__ __forceinline__ double csr_tree(double (&v)[CSR_SHORT], int m) {
         v[0] += v[2];
         v[1] += v[3];
     }
-    return m > 1 ? v[0] + v[1] : v[0];
+    const double sum = m > 1 ? v[0] + v[1] : v[0];
+    return sf_zero(sum) ? 0.0 : sum;
 }
 
 __device__ __forceinline__ double csr_quotient(double a, double b) {
