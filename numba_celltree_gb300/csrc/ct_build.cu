@@ -43,7 +43,8 @@ constexpr int NBMAX = 32;          // maximum n_buckets
 constexpr int STATS_THREADS = 256; // threads of the stats CTAs
 constexpr int SCAT_THREADS = 128;  // threads of the scatter CTAs
 constexpr int STATS4_THREADS = 64; // threads of the stats CTAs for 4 buckets
-constexpr int TILE_MIN = 2048;     // minimum cells per tile
+constexpr int TILE_MIN = 2048;     // minimum cells per tile, TILE_FLOOR where that leaves too few tiles
+constexpr int TILE_FLOOR = 512;
 constexpr int MAX_TILES = 2048;    // maximum tiles per node
 constexpr int SUB_WARPS = 2;       // warps per CTA in the subtree kernel (10.5 KB of shared memory each)
 
@@ -137,6 +138,10 @@ static size_t carve(char* base, int64_t n, int NB, int factor, WS* ws, int n_tre
     int64_t nn = n > 0 ? n : 1;
     int rec_cap = (int)std::min<int64_t>(INT32_MAX / 4,
                                          (int64_t)factor * (8 * (nn / SMALL) + 64) + 3 * (int64_t)n_trees);
+    // tiles of a level: at most n / TILE_FLOOR full ones and a part of one for
+    // each pending node (of more than SMALL cells), within twice rec_cap's
+    // 8 n / SMALL
+    static_assert(TILE_FLOOR >= SMALL, "a level's tiles may outgrow tile_cap");
     int tile_cap = (int)std::min<int64_t>(INT32_MAX / 4, 2 * (nn / TILE_MIN) + 2 * (int64_t)rec_cap + 64);
     WS w;
     for (int b = 0; b < 2; b++) {
@@ -449,10 +454,19 @@ __global__ void k_root_resolve(WS ws, int n) {
 // level).
 __device__ __forceinline__ int tile_len_for(int size, int n) {
     int t = (size + MAX_TILES - 1) / MAX_TILES;
-    t = max(t, min(TILE_MIN, max(512, n / (152 * 8))));
+    t = max(t, min(TILE_MIN, max(TILE_FLOOR, n / (152 * 8))));
     t = (t + STATS_THREADS - 1) / STATS_THREADS * STATS_THREADS;
     return t;
 }
+
+// Bits of Counters::err: 0x80000000 a capacity was exceeded (ERR_TILES: the
+// tiles', so the level's tiles are not all listed), 0x40000000 a node's
+// position is outside its tree's range (emission).
+constexpr unsigned ERR_TILES = 0x20000000u;
+
+// Whether the level's kernels have nothing to do: the last level is behind
+// them, or its tiles are not all listed (tile_count then counts past the list).
+__device__ __forceinline__ bool level_over(const WS& ws) { return ws.cnt->done || (ws.cnt->err & ERR_TILES); }
 
 // One warp per record of the current level: make tiles for pending nodes and
 // reset their stats slots.
@@ -472,7 +486,7 @@ __global__ void k_make_tiles(WS ws, int NB, int n) {
         if (lane == 0) t0 = atomicAdd(&ws.cnt->tile_count, nt);
         t0 = __shfl_sync(0xffffffffu, t0, 0);
         if (t0 + nt > ws.tile_cap) {
-            if (lane == 0) atomicOr(&ws.cnt->err, 0x80000000u);
+            if (lane == 0) atomicOr(&ws.cnt->err, 0x80000000u | ERR_TILES);
             continue;
         }
         for (int j = lane; j < nt; j += 32) {
@@ -518,7 +532,7 @@ __global__ void __launch_bounds__(NB4 ? STATS4_THREADS : STATS_THREADS, NB4 ? 12
     const unsigned FULL = 0xffffffffu;
     const unsigned long long KZ = 0x8000000000000000ull;  // fkey(0)
     if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
-    const int nt = ws.cnt->done ? 0 : ws.cnt->tile_count;
+    const int nt = level_over(ws) ? 0 : ws.cnt->tile_count;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         __syncthreads();  // the previous tile's readers are done with the shared arrays
         const int r = ws.tile_rec[t];
@@ -660,7 +674,7 @@ __global__ void k_decide(WS ws, int NB, long long cpl) {
     const unsigned FULL = 0xffffffffu;
     int lane = threadIdx.x & 31;
     int w = threadIdx.x >> 5;  // blockDim = 128
-    if (ws.cnt->done) return;
+    if (level_over(ws)) return;
     if (DIMS == DIM_OTHER && !ws.cnt->turned) return;
     int lb = ws.cnt->lb, le = ws.cnt->le;
     const int step = (int)gridDim.x * 4;
@@ -885,7 +899,7 @@ __global__ void __launch_bounds__(SCAT_THREADS) k_scatter(WS ws, int parity, int
     static_assert(ROWS <= 32, "a lane per (round's part, warp)");
     __shared__ int first[ROWS][NBMAX];  // cells of (part, warp) per bucket, then where the first goes
     const unsigned FULL = 0xffffffffu;
-    const int nt = ws.cnt->done ? 0 : ws.cnt->tile_count;
+    const int nt = level_over(ws) ? 0 : ws.cnt->tile_count;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         __syncthreads();
         int r = ws.tile_rec[t];
@@ -1914,7 +1928,7 @@ static int build_levels(WS& ws, cudaStream_t st, int n, int NB, int64_t cpl, boo
     while (ahead < DEV_MAX_LEVELS - 4 && ((long long)SMALL << (ahead - 1)) < n) ahead++;
     bool one_run = true;
     if (run_phase_a) {
-        const long long tile = std::min(TILE_MIN, std::max(512, n / (152 * 8)));  // tile_len_for
+        const long long tile = std::min(TILE_MIN, std::max(TILE_FLOOR, n / (152 * 8)));  // tile_len_for
         int parity = 0;
         double width = n_roots;  // records of the level, at most
         // the counters and the ranges of the levels run lie side by side
