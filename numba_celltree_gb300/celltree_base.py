@@ -547,7 +547,8 @@ class _GpuTree:
                    "intersect_edges")
         iccnt = _device.empty((max(ni, 1),), torch.int64, self.device)
         ispec, icap = None, int(self.SEG_SPEC_CAP)
-        while icap >= 8 and ni * icap * 4 > self.SEG_SPEC_MAX_BYTES:
+        room = self.scratch_room(min(ni * icap * 4, self.SEG_SPEC_MAX_BYTES))
+        while icap >= 8 and ni * icap * 4 > room:
             icap //= 2
         if keep and ni > 0 and (icap >= 8 or icap == self.SEG_SPEC_CAP):
             ispec = _device.empty((ni, icap), torch.int32, self.device)
@@ -586,6 +587,21 @@ class _GpuTree:
         free, _ = torch.cuda.mem_get_info(self.device)
         return max(1 << 20, int(free // 4 // max(bytes_per_result, 1)))
 
+    # bytes of optional scratch from which the free memory is looked at
+    SCRATCH_CHECK_MIN = 1 << 26
+
+    def scratch_room(self, nbytes: int) -> int:
+        """How much of an optional scratch of nbytes (one that saves a second
+        traversal) to take: all of a small one, else at most a quarter of the
+        memory that is free on the device or held unused by the allocator."""
+        if nbytes <= self.SCRATCH_CHECK_MIN:
+            return nbytes
+        torch = _device.torch()
+        free, _ = torch.cuda.mem_get_info(self.device)
+        if free // 4 < nbytes:
+            free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        return max(self.SCRATCH_CHECK_MIN, min(nbytes, int(free) // 4))
+
     # pairs from which subtrees inside a box are written by a warp each after
     # the traversal (below, the extra launch costs more than it saves)
     BOX_JOBS_MIN_PAIRS = 1 << 20
@@ -599,8 +615,8 @@ class _GpuTree:
     SPEC_CAP_LARGE = 16
     SPEC_MAX_BYTES = 1 << 30
     # batches walked by warps keep terminal nodes instead: room for BOX_RECORDS
-    # of 16 bytes a box, as far as SPEC_MAX_BYTES goes and at least
-    # BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
+    # of 16 bytes a box, as far as SPEC_MAX_BYTES and scratch_room go and at
+    # least BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
     # average, 10k of 0.2 to 4 cells 6)
     BOX_RECORDS = 256
     BOX_RECORDS_MIN = 64
@@ -628,8 +644,10 @@ class _GpuTree:
             order = self.spatial_order(boxes_d, 0)[0]
         spec = recs = None
         cap = self.SPEC_CAP if n <= self.SPEC_MAX_BOXES else self.SPEC_CAP_LARGE
-        most = min(n * self.BOX_RECORDS, self.SPEC_MAX_BYTES // 16)
-        if not small and self.SPEC_MAX_BOXES > 0 and 0 < n and most >= n * self.BOX_RECORDS_MIN:
+        most = 0
+        if not small and self.SPEC_MAX_BOXES > 0 and self.max_depth + 2 <= self.BATCHED_MAX_STACK:
+            most = self.scratch_room(min(n * self.BOX_RECORDS * 16, self.SPEC_MAX_BYTES)) // 16
+        if n > 0 and most > 0 and most >= n * self.BOX_RECORDS_MIN:
             # one traversal: the counting pass keeps the boxes' terminal nodes
             recs = _device.empty((int(lib.ct_box_records_size(most)),), torch.uint8, self.device)
             _lib.check(lib.ct_count_boxes_records(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
