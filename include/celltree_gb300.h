@@ -485,10 +485,11 @@ int ct_count_boxes(const ct_tree* tree, const double* boxes, int64_t n, const in
  * in traversal order -- upstream's locate_boxes output order. */
 int ct_write_boxes(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, const int64_t* offsets,
                    int64_t* ii, int64_t* jj, void* stream);
-/* The same output; subtrees of at least min_job_cells cells (0: 8) wholly
- * inside a query box (box index) are queued in the workspace and their cells
- * written by one warp per subtree, coalesced, after the traversal, instead
- * of by the box's own thread.  total_pairs: the scanned total (sizes the
+/* The same output; large subtrees wholly inside a query box (box index) are
+ * queued in the workspace and their cells written coalesced after the
+ * traversal, instead of by the box's own warp: those of at least
+ * min_job_cells cells (0: the default), but never of fewer than 256 (8 in
+ * trees deeper than the traversal stacks).  total_pairs: the scanned total (sizes the
  * queue); workspace: ct_write_boxes_workspace_size(total_pairs,
  * min_job_cells) bytes, in use until the enqueued work has run. */
 size_t ct_write_boxes_workspace_size(int64_t total_pairs, int32_t min_job_cells);
@@ -505,9 +506,10 @@ int ct_write_boxes_ws(const ct_tree* tree, const double* boxes, int64_t n, const
 int ct_count_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
                         int32_t* spec, int32_t spec_cap, void* stream);
 /* Large batches in one traversal: the counting pass keeps every terminal node
- * with pairs (a leaf, or a subtree inside the box) as a record, ct_box_records_size
- * bytes for `capacity` of them; the writing call expands them, or, when there
- * were more, traverses again.  Same output as ct_count_boxes + ct_write_boxes;
+ * with pairs (a leaf, or a subtree inside the box, large ones in parts) as a
+ * record, ct_box_records_size bytes for `capacity` of them; the writing call
+ * expands them, or, when there were more, traverses again (and uses the
+ * records' memory as scratch).  Same output as ct_count_boxes + ct_write_boxes;
  * inside (optional, total_pairs bytes): 1 for the pairs known to have the cell
  * inside the box. */
 size_t ct_box_records_size(int64_t capacity);

@@ -617,8 +617,11 @@ class _GpuTree:
     # batches walked by warps keep terminal nodes instead: room for BOX_RECORDS
     # of 16 bytes a box, as far as SPEC_MAX_BYTES and scratch_room go and at
     # least BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
-    # average, 10k of 0.2 to 4 cells 6)
+    # average, 10k of 0.2 to 4 cells 6); fewer boxes than BOX_RECORDS_BOXES may be
+    # large and have the room of so many, 16 MB (one around 4.1M of 5M cells 142
+    # ms with its whole subtrees written by its warp in a second walk, now 5.3)
     BOX_RECORDS = 256
+    BOX_RECORDS_BOXES = 4096
     BOX_RECORDS_MIN = 64
 
     def locate_boxes(self, boxes_d, config=None, budget=None, small=False, inside=False):
@@ -646,7 +649,8 @@ class _GpuTree:
         cap = self.SPEC_CAP if n <= self.SPEC_MAX_BOXES else self.SPEC_CAP_LARGE
         most = 0
         if not small and self.SPEC_MAX_BOXES > 0 and self.max_depth + 2 <= self.BATCHED_MAX_STACK:
-            most = self.scratch_room(min(n * self.BOX_RECORDS * 16, self.SPEC_MAX_BYTES)) // 16
+            most = max(n, self.BOX_RECORDS_BOXES) * self.BOX_RECORDS
+            most = self.scratch_room(min(most * 16, self.SPEC_MAX_BYTES)) // 16
         if n > 0 and most > 0 and most >= n * self.BOX_RECORDS_MIN:
             # one traversal: the counting pass keeps the boxes' terminal nodes
             recs = _device.empty((int(lib.ct_box_records_size(most)),), torch.uint8, self.device)

@@ -323,13 +323,21 @@ static_assert(sizeof(WalkBox) == 88, "see above");
 // box (top bit: the whole subtree lies inside it), the rank of the first pair
 // within the box (top bit: a leaf of more than 32 cells), the first leaf
 // position, and the leaf's overlapping cells as bits or the number of cells.
+// A whole subtree of more than two parts of `part` cells is kept in parts
+// that begin at leaves: a warp of k_box_records takes 32 records, and one
+// warp alone would write the pairs of a box around the mesh (one box around
+// 5M cells 183 ms, in parts 0.85).  The writing pass leaves whole subtrees
+// to k_box_records in the same form, where it has the room.
 struct BoxRecs {
     int4* rec;
-    unsigned long long* count;  // records asked for
+    unsigned long long* count;   // records the counting pass asked for (null: there was none)
+    unsigned long long* pushed;  // records of the writing pass
     int64_t cap;
+    int part;
     uint8_t* inside;  // optional, per pair: the cell lies in a subtree inside the box
 };
 constexpr int REC_FLAG = (int)0x80000000u;
+constexpr int REC_PART = 256;
 
 // The outputs of the lanes' terminal nodes (`share` each), 32 at a time:
 // put(box, output index, leaf position) per lane; whole subtrees give their
@@ -435,6 +443,45 @@ struct BoxWalk {
         }
     }
 
+    // Keeps `parts` records of each lane's node r (of a whole subtree, or one);
+    // whether the lane's fit.  `whole`: all of a lane's or none.
+    __device__ __forceinline__ bool keep_records(unsigned long long* count, int parts, bool whole, int4 r) const {
+        const unsigned FULL = 0xffffffffu;
+        const unsigned some = __ballot_sync(FULL, parts > 0), many = __ballot_sync(FULL, parts > 1);
+        if (!some) return false;
+        int before = __popc(some & ((1u << lane) - 1u)), total = __popc(some);
+        if (many) {
+            int incl = parts;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += t;
+            }
+            before = incl - parts;
+            total = __shfl_sync(FULL, incl, 31);
+        }
+        unsigned long long first = 0;
+        if (lane == 0) first = atomicAdd(count, (unsigned long long)total);
+        first = __shfl_sync(FULL, first, 0) + (unsigned)before;
+        const unsigned long long cap = (unsigned long long)recs.cap;
+        const bool fits = first + (unsigned)parts <= cap;
+        if (parts == 1 && fits) recs.rec[first] = r;
+        for (unsigned m = many; m; m &= m - 1u) {
+            const int src = __ffs(m) - 1, k = __shfl_sync(FULL, parts, src);
+            const unsigned long long at = __shfl_sync(FULL, first, src);
+            const int id = __shfl_sync(FULL, r.x, src), rank = __shfl_sync(FULL, r.y, src);
+            const int ptr = __shfl_sync(FULL, r.z, src), end = ptr + __shfl_sync(FULL, r.w, src);
+            const bool none = whole && at + (unsigned)k > cap;  // slots before the end get no cells
+            for (int t = lane; t < k && at + (unsigned)t < cap; t += 32) {
+                int p0 = ptr, p1 = end;
+                if (t > 0) p0 = max(ptr, min(T.lstart[ptr + t * recs.part], ptr + t * recs.part));
+                if (t + 1 < k) p1 = max(p0, min(T.lstart[ptr + (t + 1) * recs.part], end));
+                recs.rec[at + (unsigned)t] = none ? make_int4(id, 0, ptr, 0) : make_int4(id, rank + (end - p1), p0, p1 - p0);
+            }
+        }
+        return parts > 0 && fits;
+    }
+
     __device__ __forceinline__ void emit(int v, unsigned meta, bool have) const {
         const unsigned FULL = 0xffffffffu;
         const int qi = have ? (int)(meta & WALK_QMASK) : -1;
@@ -460,23 +507,20 @@ struct BoxWalk {
         }
         const int64_t rank = walk_rank<int64_t>(qi, c, have, lane, emitted);
         if (MODE == BOX_RECORD) {
-            const bool keep = c > 0;
-            const unsigned b = __ballot_sync(FULL, keep);
-            if (b) {
-                unsigned long long first = 0;
-                if (lane == 0) first = atomicAdd(recs.count, (unsigned long long)__popc(b));
-                first = __shfl_sync(FULL, first, 0) + __popc(b & ((1u << lane) - 1u));
-                if (keep && first < (unsigned long long)recs.cap)
-                    recs.rec[first] = make_int4((int)S.id | (all ? REC_FLAG : 0),
-                                                (int)rank | (!all && size > 32 ? REC_FLAG : 0), ptr,
-                                                all || size > 32 ? size : (int)hit);
-            }
+            const int parts = c == 0 ? 0 : all && c >= 2 * recs.part ? (int)c / recs.part : 1;
+            keep_records(recs.count, parts, false,
+                         make_int4((int)S.id | (all ? REC_FLAG : 0), (int)rank | (!all && size > 32 ? REC_FLAG : 0), ptr,
+                                   all || size > 32 ? size : (int)hit));
             return;
         }
         if (!WRITE && !spec) return;
         const int64_t at = have ? S.base : 0;
         const int64_t id = have ? S.id : 0;
         int64_t share = WRITE ? c : min(c, max((int64_t)0, (int64_t)spcap - rank));
+        if (WRITE && recs.rec) {  // whole subtrees to k_box_records
+            const int parts = all && c >= recs.part ? (int)c / recs.part : 0;
+            if (keep_records(recs.pushed, parts, true, make_int4((int)id | REC_FLAG, (int)rank, ptr, size))) share = 0;
+        }
         if (!all && size > 32) {  // a large leaf: its own lane
             int64_t r = rank;
             for (int k = 0; k < size && share > 0; k++)
@@ -555,15 +599,17 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const dou
     if (!WRITE && valid) cnt_or_off[i] = counts[wi][lane];
 }
 
-// The pairs of the counting pass's records, a warp per 32 of them: no second
-// walk (91M pairs of 250k boxes: 1.20 ms, the walk again 4.45).
+// The pairs of the counting pass's records (of the writing pass's, when those
+// did not all fit), a warp per 32 of them: no second walk (91M pairs of 250k
+// boxes: 1.20 ms, the walk again 4.45).
 __global__ void __launch_bounds__(256) k_box_records(TreeQ T, const double4* __restrict__ boxes, BoxRecs recs,
                                                      const int64_t* __restrict__ off, int64_t* __restrict__ ii,
                                                      int64_t* __restrict__ jj) {
     const int lane = threadIdx.x & 31;
-    const unsigned long long asked = *recs.count;
-    if (asked > (unsigned long long)recs.cap) return;  // not all were kept: the boxes are walked again
-    const int64_t n = (int64_t)asked, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const unsigned long long cap = (unsigned long long)recs.cap, asked = recs.count ? *recs.count : cap + 1;
+    // not all were kept: the boxes have been walked again, but for these
+    const int64_t n = (int64_t)(asked <= cap ? asked : min(*recs.pushed, cap));
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     auto put = [&](int i, int64_t k, int j, bool whole) {
         ii[k] = i;
         jj[k] = T.bbi[j];
@@ -2942,7 +2988,7 @@ static int walk_tasks(int64_t n) {
 template <int MODE>
 static void launch_box_walk(const TreeQ& T, const double4* boxes, int64_t n, const int* order, int64_t* cnt_or_off,
                             int64_t* ii, int64_t* jj, int* spec, int spcap, const int64_t* spec_cnt,
-                            cudaStream_t st, BoxRecs recs = {nullptr, nullptr, 0, nullptr}) {
+                            cudaStream_t st, BoxRecs recs = {}) {
     const int per_warp = walk_tasks(n);
     k_box_walk<MODE><<<grid_of((n + per_warp - 1) / per_warp, WALK_WARPS), 32 * WALK_WARPS, 0, st>>>(
         T, boxes, n, order, per_warp, cnt_or_off, ii, jj, spec, spcap, spec_cnt, recs);
@@ -3113,6 +3159,35 @@ size_t ct_write_boxes_workspace_size(int64_t total_pairs, int32_t min_job_cells)
     return 256 + (size_t)cap * sizeof(BoxJob);
 }
 
+// records: the two counts, then the records
+static BoxRecs box_recs(void* records, int64_t capacity, uint8_t* inside) {
+    unsigned long long* counts = (unsigned long long*)records;
+    return BoxRecs{(int4*)((char*)records + 256), counts, counts + 1, capacity, REC_PART, inside};
+}
+
+static void launch_box_records(const TreeQ& T, const double4* boxes, const BoxRecs& R, const int64_t* off, int64_t* ii,
+                               int64_t* jj, cudaStream_t st) {
+    k_box_records<<<(unsigned)std::min<int64_t>((R.cap + 255) / 256, 152 * 64), 256, 0, st>>>(T, boxes, R, off, ii, jj);
+}
+
+// The boxes walked (those of spec_cnt above spec_cap, if given), their whole
+// subtrees left to k_box_records in the job workspace.
+static int walk_boxes_ws(const TreeQ& T, const double4* boxes, int64_t n, const int* order, const int64_t* off,
+                         int spec_cap, const int64_t* spec_cnt, int64_t total_pairs, int min_job_cells, int64_t* ii,
+                         int64_t* jj, void* ws, cudaStream_t st) {
+    BoxRecs R = {};
+    if (T.nbx && n < INT32_MAX) {  // (without the box index no subtree is known to lie inside)
+        const int jm = box_job_min(min_job_cells);
+        R = box_recs(ws, (total_pairs > 0 ? total_pairs : 0) / jm + 1, nullptr);
+        R.count = nullptr;
+        R.part = std::max(jm, REC_PART);
+        CT_CUDA(cudaMemsetAsync(R.pushed, 0, sizeof(unsigned long long), st));
+    }
+    launch_box_walk<BOX_WRITE>(T, boxes, n, order, (int64_t*)off, ii, jj, nullptr, spec_cap, spec_cnt, st, R);
+    if (R.rec) launch_box_records(T, boxes, R, off, ii, jj, st);
+    return CT_OK;
+}
+
 int ct_write_boxes_ws(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order,
                       const int64_t* offsets, int64_t total_pairs, int32_t min_job_cells, int64_t* ii, int64_t* jj,
                       void* ws, size_t ws_bytes, void* stream) {
@@ -3124,8 +3199,14 @@ int ct_write_boxes_ws(const ct_tree* t, const double* boxes, int64_t n, const in
         return ct_fail(CT_ERR_WORKSPACE, "write_boxes workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     TreeQ T = make_q(t);
-    // no box index: no subtrees; the warps' walk writes them by itself
-    if (!T.nbx || !deep_tree(t)) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);
+    if (!deep_tree(t)) {
+        int s2 = walk_boxes_ws(T, (const double4*)boxes, n, order, offsets, 0, nullptr, total_pairs, min_job_cells, ii, jj,
+                               ws, st);
+        if (s2) return s2;
+        CT_CHECK_LAUNCH("write_boxes");
+        return CT_OK;
+    }
+    if (!T.nbx) return ct_write_boxes(t, boxes, n, order, offsets, ii, jj, stream);  // no box index: no subtrees
     const int jm = box_job_min(min_job_cells);
     unsigned long long* njobs = (unsigned long long*)ws;
     BoxJob* jobs = (BoxJob*)((char*)ws + 256);
@@ -3159,11 +3240,6 @@ int ct_count_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const 
     return CT_OK;
 }
 
-// records: a count, then the records
-static BoxRecs box_recs(void* records, int64_t capacity, uint8_t* inside) {
-    return BoxRecs{(int4*)((char*)records + 256), (unsigned long long*)records, capacity, inside};
-}
-
 size_t ct_box_records_size(int64_t capacity) { return 256 + sizeof(int4) * (size_t)(capacity > 0 ? capacity : 1); }
 
 int ct_count_boxes_records(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
@@ -3177,7 +3253,7 @@ int ct_count_boxes_records(const ct_tree* t, const double* boxes, int64_t n, con
         CT_CUDA(cudaMemsetAsync(records, 0xff, sizeof(unsigned long long), st));
         return ct_count_boxes(t, boxes, n, order, counts, stream);
     }
-    CT_CUDA(cudaMemsetAsync(records, 0, sizeof(unsigned long long), st));
+    CT_CUDA(cudaMemsetAsync(records, 0, 2 * sizeof(unsigned long long), st));
     if (n == 0) return CT_OK;
     launch_box_walk<BOX_RECORD>(make_q(t), (const double4*)boxes, n, order, counts, nullptr, nullptr, nullptr, 0, nullptr,
                                 st, box_recs(records, capacity, nullptr));
@@ -3198,8 +3274,8 @@ int ct_write_boxes_records(const ct_tree* t, const double* boxes, int64_t n, con
     const TreeQ T = make_q(t);
     const double4* B = (const double4*)boxes;
     const BoxRecs R = box_recs((void*)records, capacity, inside);
-    k_box_records<<<(unsigned)std::min<int64_t>((capacity + 255) / 256, 152 * 64), 256, 0, st>>>(T, B, R, offsets, ii, jj);
     launch_box_walk<BOX_WRITE>(T, B, n, order, (int64_t*)offsets, ii, jj, nullptr, 0, nullptr, st, R);
+    launch_box_records(T, B, R, offsets, ii, jj, st);
     CT_CHECK_LAUNCH("write_boxes_records");
     return CT_OK;
 }
@@ -3237,7 +3313,8 @@ int ct_write_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const 
     int64_t* off = (int64_t*)offsets;
     const double4* B = (const double4*)boxes;
     if (!deep_tree(t)) {
-        launch_box_walk<BOX_WRITE>(T, B, n, order, off, ii, jj, nullptr, spec_cap, counts, st);
+        int s2 = walk_boxes_ws(T, B, n, order, off, spec_cap, counts, total_pairs, min_job_cells, ii, jj, ws, st);
+        if (s2) return s2;
         CT_CHECK_LAUNCH("write_boxes_spec");
         return CT_OK;
     }
