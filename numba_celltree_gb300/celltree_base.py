@@ -500,14 +500,15 @@ class _GpuTree:
     SEG_SPEC_CAP = 128
     SEG_SPEC_MAX_BYTES = 1 << 31
 
-    def edge_candidate_ranges(self, segs_d, mode: int, order, cut, keep: bool = False):
+    def edge_candidate_ranges(self, segs_d, mode: int, order, cut, keep: bool = False, item_scratch: bool = True):
         """Every segment's candidate offset and count (device int64) and the
         candidate total, and what the writing pass uses: (coff, ccnt, total,
         items) -- items None (traverse again), ("spec", scratch, cap) with
         `keep` (the counting pass kept each segment's first `cap`
         candidates), or with a
         cut the work items (item_seg, item_node, n_items, item offsets, item
-        counts, scratch or None, cap; the scratch under the same limits)."""
+        counts, scratch or None, cap; the scratch under the same limits, and
+        only with `item_scratch`)."""
         torch = _device.torch()
         lib = _lib.load()
         st = _device.stream()
@@ -547,10 +548,9 @@ class _GpuTree:
                    "intersect_edges")
         iccnt = _device.empty((max(ni, 1),), torch.int64, self.device)
         ispec, icap = None, int(self.SEG_SPEC_CAP)
-        room = self.scratch_room(min(ni * icap * 4, self.SEG_SPEC_MAX_BYTES))
-        while icap >= 8 and ni * icap * 4 > room:
+        while icap >= 8 and ni * icap * 4 > self.SEG_SPEC_MAX_BYTES:
             icap //= 2
-        if keep and ni > 0 and (icap >= 8 or icap == self.SEG_SPEC_CAP):
+        if keep and item_scratch and ni > 0 and (icap >= 8 or icap == self.SEG_SPEC_CAP):
             ispec = _device.empty((ni, icap), torch.int32, self.device)
             _lib.check(lib.ct_count_item_candidates_spec(d, mode, P(segs_d), P(iseg), P(inode), ni, P(iccnt),
                                                          P(ispec), icap, st), "intersect_edges")
@@ -587,21 +587,6 @@ class _GpuTree:
         free, _ = torch.cuda.mem_get_info(self.device)
         return max(1 << 20, int(free // 4 // max(bytes_per_result, 1)))
 
-    # bytes of optional scratch from which the free memory is looked at
-    SCRATCH_CHECK_MIN = 1 << 26
-
-    def scratch_room(self, nbytes: int) -> int:
-        """How much of an optional scratch of nbytes (one that saves a second
-        traversal) to take: all of a small one, else at most a quarter of the
-        memory that is free on the device or held unused by the allocator."""
-        if nbytes <= self.SCRATCH_CHECK_MIN:
-            return nbytes
-        torch = _device.torch()
-        free, _ = torch.cuda.mem_get_info(self.device)
-        if free // 4 < nbytes:
-            free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
-        return max(self.SCRATCH_CHECK_MIN, min(nbytes, int(free) // 4))
-
     # pairs from which subtrees inside a box are written by a warp each after
     # the traversal (below, the extra launch costs more than it saves)
     BOX_JOBS_MIN_PAIRS = 1 << 20
@@ -615,14 +600,21 @@ class _GpuTree:
     SPEC_CAP_LARGE = 16
     SPEC_MAX_BYTES = 1 << 30
     # batches walked by warps keep terminal nodes instead: room for BOX_RECORDS
-    # of 16 bytes a box, as far as SPEC_MAX_BYTES and scratch_room go and at
-    # least BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
+    # of 16 bytes a box, as far as SPEC_MAX_BYTES goes and at least
+    # BOX_RECORDS_MIN a box (250k boxes of 0.2 to 100 cells a side have 77 on
     # average, 10k of 0.2 to 4 cells 6); fewer boxes than BOX_RECORDS_BOXES may be
     # large and have the room of so many, 16 MB (one around 4.1M of 5M cells 142
     # ms with its whole subtrees written by its warp in a second walk, now 5.3)
     BOX_RECORDS = 256
     BOX_RECORDS_BOXES = 4096
     BOX_RECORDS_MIN = 64
+
+    def box_records(self, n: int, small: bool) -> int:
+        """Records the counting pass of n boxes has room for (0: it keeps none)."""
+        if n == 0 or small or self.SPEC_MAX_BOXES <= 0 or self.max_depth + 2 > self.BATCHED_MAX_STACK:
+            return 0
+        most = min(max(n, self.BOX_RECORDS_BOXES) * self.BOX_RECORDS, self.SPEC_MAX_BYTES // 16)
+        return most if most >= n * self.BOX_RECORDS_MIN else 0
 
     def locate_boxes(self, boxes_d, config=None, budget=None, small=False, inside=False):
         """Pairs (box, cell) of every box query, box-major in upstream order;
@@ -631,6 +623,16 @@ class _GpuTree:
         are about a cell each and come in mesh order (counted by a thread
         each).  `inside`: also a byte per pair, 1 where the cell is known to
         lie inside the box (None when the batch gives none)."""
+        torch = _device.torch()
+        most = self.box_records(int(boxes_d.shape[0]), small)
+        if most > 0:
+            try:
+                return self._locate_boxes(boxes_d, config, budget, small, inside, most)
+            except torch.cuda.OutOfMemoryError:
+                pass  # once more without the records' room, after that frame's memory is given back
+        return self._locate_boxes(boxes_d, config, budget, small, inside, 0)
+
+    def _locate_boxes(self, boxes_d, config, budget, small, inside, most):
         n = int(boxes_d.shape[0])
         ask = inside
         if config is None:
@@ -647,11 +649,7 @@ class _GpuTree:
             order = self.spatial_order(boxes_d, 0)[0]
         spec = recs = None
         cap = self.SPEC_CAP if n <= self.SPEC_MAX_BOXES else self.SPEC_CAP_LARGE
-        most = 0
-        if not small and self.SPEC_MAX_BOXES > 0 and self.max_depth + 2 <= self.BATCHED_MAX_STACK:
-            most = max(n, self.BOX_RECORDS_BOXES) * self.BOX_RECORDS
-            most = self.scratch_room(min(most * 16, self.SPEC_MAX_BYTES)) // 16
-        if n > 0 and most > 0 and most >= n * self.BOX_RECORDS_MIN:
+        if most > 0:
             # one traversal: the counting pass keeps the boxes' terminal nodes
             recs = _device.empty((int(lib.ct_box_records_size(most)),), torch.uint8, self.device)
             _lib.check(lib.ct_count_boxes_records(ctypes.byref(self.desc), _device.ptr(boxes_d), n, _device.ptr(order),
@@ -751,9 +749,19 @@ class _GpuTree:
         the traversal and the cell test read nodes and cells that the segments
         before have brought into L2.  1M short segments on 5M cells read 19 KB
         of DRAM each in their own order."""
+        torch = _device.torch()
         n = int(segs_d.shape[0])
         if config is None:
             config = self.cached("segments", n)
+        if self.edge_cut(config, n) is not None:
+            try:
+                return self._locate_edges(segs_d, mode, config, budget, True)
+            except torch.cuda.OutOfMemoryError:
+                pass  # once more without the work items' scratch, after that frame's memory is given back
+        return self._locate_edges(segs_d, mode, config, budget, False)
+
+    def _locate_edges(self, segs_d, mode: int, config, budget, item_scratch):
+        n = int(segs_d.shape[0])
         torch = _device.torch()
         lib = _lib.load()
         st = _device.stream()
@@ -764,7 +772,8 @@ class _GpuTree:
         if self.in_spatial_order(n, config):
             order, segs_d = self.spatial_order(segs_d, 1)
         P = _device.ptr
-        coff, ccnt, nc, items = self.edge_candidate_ranges(segs_d, mode, None, self.edge_cut(config, n), keep=True)
+        coff, ccnt, nc, items = self.edge_candidate_ranges(segs_d, mode, None, self.edge_cut(config, n), True,
+                                                           item_scratch)
         if budget is not None and nc > budget:
             self.last_counts = ccnt
             if order is not None:

@@ -1,6 +1,8 @@
-"""Optional scratch of the box and segment queries: kept within a quarter of
-the free memory, and not taken where the traversal does not use it; the results
-stay the same."""
+"""Optional scratch of the box and segment queries: left out where the device
+has no room for it, and not taken where the traversal does not use it; the
+results stay the same."""
+
+import contextlib
 
 import numpy as np
 import pytest
@@ -9,7 +11,20 @@ from numba_celltree_gb300 import synthetic as syn
 
 pytestmark = pytest.mark.gpu
 
-FREE = 320 << 20
+
+@contextlib.contextmanager
+def room(nbytes):
+    """This process may hold nbytes more than it holds now."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.mem_get_info()[1]
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + nbytes) / total)
+    try:
+        yield
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
 
 
 def peak(fn):
@@ -25,32 +40,20 @@ def peak(fn):
     return out, torch.cuda.max_memory_allocated() - base
 
 
-def small_device(monkeypatch):
-    """A device with FREE bytes left and nothing cached."""
-    import torch
-
-    total = torch.cuda.mem_get_info()[1]
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (FREE, total))
-    monkeypatch.setattr(torch.cuda, "memory_reserved", torch.cuda.memory_allocated)
-
-
-@pytest.mark.parametrize("n", [40_000, 100_000])  # fewer records a box; none
-def test_box_records(monkeypatch, n):
+def test_box_records():
     import torch
 
     from numba_celltree_gb300 import CellTree2d
 
+    n = 100_000
     xy, f = syn.quad_mesh(60, seed=41)
     t = CellTree2d(xy, f, -1)._tree
     b = torch.as_tensor(syn.random_boxes(n, (0, 0), (1, 1), 0.01, 0.03, seed=42), device="cuda")
-    t.locate_boxes(b[:100])  # the box index
     want = t.locate_boxes(b)
-    with monkeypatch.context() as m:
-        small_device(m)
-        got, most = peak(lambda: t.locate_boxes(b))
+    assert t.box_records(n, False) * 16 > 300 << 20
+    with room(200 << 20):
+        got = t.locate_boxes(b)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
-    # pairs, counts and offsets, order and scans, and the scratch
-    assert most <= 16 * len(want[0]) + 64 * n + FREE // 4 + (4 << 20)
 
 
 def test_no_box_records_for_deep_trees():
@@ -68,7 +71,7 @@ def test_no_box_records_for_deep_trees():
     assert most <= 16 * len(got[0]) + 64 * n + n * t.SPEC_CAP * 4 + (4 << 20)
 
 
-def test_work_items(monkeypatch):
+def test_work_items():
     import torch
 
     from numba_celltree_gb300 import CellTree2d
@@ -76,18 +79,11 @@ def test_work_items(monkeypatch):
     xy, f = syn.quad_mesh(300, seed=44)
     t = CellTree2d(xy, f, -1)._tree
     rng = np.random.default_rng(45)
-    s = torch.as_tensor(rng.uniform(0, 1, (8000, 2, 2)), device="cuda")
-    cfg = {"split": 16}  # many items
+    s = torch.as_tensor(rng.uniform(0, 1, (4000, 2, 2)), device="cuda")
+    cfg = {"split": 1}  # an item for about every candidate
     want = t.locate_edges(s, 1, cfg)
-    cut = t.edge_cut(cfg, len(s))
-    ni = t.edge_candidate_ranges(s, 1, None, cut)[3][2]
-    assert ni * t.SEG_SPEC_CAP * 4 > FREE // 4  # the scratch would not fit
-    taken = []
-    empty = torch.empty
-    with monkeypatch.context() as m:
-        small_device(m)
-        m.setattr(torch, "empty", lambda *a, **k: (taken.append(x := empty(*a, **k)), x)[1])
+    ni = t.edge_candidate_ranges(s, 1, None, t.edge_cut(cfg, 4000))[3][2]
+    assert ni * t.SEG_SPEC_CAP * 4 > 300 << 20
+    with room(200 << 20):
         got = t.locate_edges(s, 1, cfg)
     assert all(torch.equal(torch.nan_to_num(a), torch.nan_to_num(b)) for a, b in zip(got, want))
-    spec = [x for x in taken if x.dtype == torch.int32 and x.ndim == 2]
-    assert spec and all(x.numel() * 4 <= FREE // 4 for x in spec)
