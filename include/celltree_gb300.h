@@ -518,10 +518,21 @@ int ct_count_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, 
 int ct_write_boxes_records(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
                            const int64_t* offsets, const void* records, int64_t capacity, int64_t total_pairs,
                            int64_t* ii, int64_t* jj, uint8_t* inside, void* stream);
-/* The same counts and scratch by one thread per box: faster for boxes of about
- * a cell that come in mesh order (query faces). */
+/* The same counts and scratch by one thread per box: faster for many boxes of
+ * a few cells that come in mesh order or in spatial order.  spec NULL and
+ * spec_cap 0: counts alone, for ct_write_small_boxes, which writes the pairs
+ * the same way (workspace: ct_write_boxes_workspace_size(total_pairs, 0)). */
 int ct_count_small_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
                               int64_t* counts, int32_t* spec, int32_t spec_cap, void* stream);
+int ct_write_small_boxes(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
+                         const int64_t* offsets, int64_t total_pairs, int64_t* ii, int64_t* jj, void* workspace,
+                         size_t workspace_bytes, void* stream);
+/* A look at up to 1024 boxes spread over the batch, for the choice between the
+ * two forms: result_host2[0] = the cells they may overlap on average, at the
+ * tree's mean cell size, [1] = the share of them within 16 cells of the box
+ * after them (workspace: 16 bytes; synchronises). */
+int ct_box_sample(const ct_tree* tree, const double* boxes, int64_t n, double* result_host2, void* workspace,
+                  size_t workspace_bytes, void* stream);
 int ct_write_boxes_spec(const ct_tree* tree, const double* boxes, int64_t n, const int32_t* order,
                         const int64_t* counts, const int64_t* offsets, const int32_t* spec, int32_t spec_cap,
                         int64_t total_pairs, int32_t min_job_cells, int64_t* ii, int64_t* jj, void* workspace,

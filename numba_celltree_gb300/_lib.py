@@ -216,6 +216,8 @@ SIGNATURES = {
     "ct_write_boxes_records": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I64, _I64, _P, _P,
                                               _P, _P]),
     "ct_count_small_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _I32, _P]),
+    "ct_write_small_boxes": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _I64, _P, _P, _P, _SZ, _P]),
+    "ct_box_sample": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, ctypes.POINTER(_D), _P, _SZ, _P]),
     "ct_write_boxes_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _P, _I64, _P, _P, _P, _P, _I32, _I64, _I32, _P, _P,
                                            _P, ctypes.c_size_t, _P]),
     "ct_count_edge_candidates_spec": (ctypes.c_int, [ctypes.POINTER(CtTree), _I32, _P, _I64, _P, _P, _P, _I32, _P]),

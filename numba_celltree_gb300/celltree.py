@@ -366,8 +366,10 @@ class CellTree2d(CellTree2dBase):
         _lib.check(lib.ct_counter_clockwise(_device.ptr(v_d), _device.ptr(f_d), n, K, st), "counter_clockwise")
         bb = _device.empty((n, 4), torch.float64, t.device)
         _lib.check(lib.ct_face_bboxes(_device.ptr(v_d), _device.ptr(f_d), n, K, _device.ptr(bb), st), "face_bboxes")
-        # as many faces as a quarter of the tree's cells and enough threads:
-        # the boxes are a few cells each
+        # as many faces as a quarter of the tree's cells and enough threads: taken
+        # for boxes of a few cells in mesh order without a look (against a thread
+        # a box in order of size, 2M faces on 5M cells 7.1 -> 6.7 ms, shuffled
+        # 9.3 -> 9.2; 70k of 0.5 to 30 cells a side on 250k cells 2.3 -> 1.2)
         si, sj = t.locate_boxes(bb, small=n >= t.WORK_ORDER_MIN and 4 * n >= t.n)
         m = int(si.shape[0])
         flag = _device.empty((m,), torch.uint8, t.device)

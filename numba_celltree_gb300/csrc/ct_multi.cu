@@ -103,10 +103,11 @@ struct BoxJob {
 };
 constexpr int BOX_JOB_MIN = 8;  // default: smaller subtrees are written in line
 
-// One thread per box: boxes of about a cell each that come in mesh order (the
-// query faces of locate_faces), whose neighbouring lanes take the same path --
-// 1M faces on 500k cells 0.38 ms, by warps (below) 0.6 ms -- and, with DEEP,
-// trees deeper than the warps' walk takes.
+// One thread per box: large batches of boxes of a few cells each (query faces;
+// boxes whose sizes were looked at), whose neighbouring lanes take the same
+// path in mesh order or spatial order -- 1M faces on 500k cells 0.38 ms, by
+// warps (below) 0.6 ms -- and, with DEEP, trees deeper than the warps' walk
+// takes.
 template <bool WRITE, bool DEEP>
 __global__ void __launch_bounds__(256) k_boxes(TreeQ T, const double4* __restrict__ boxes, int64_t n,
                                                const int* __restrict__ order, int64_t* __restrict__ cnt_or_off,
@@ -2833,6 +2834,41 @@ __global__ void k_spatial_keys(const double4* __restrict__ q, int64_t n, int kin
     }
 }
 
+// At most BOX_SAMPLE boxes spread over the batch, a thread each: the mean of
+// the cells they may overlap, in cells of side c, and the share whose middle
+// lies within 16 cells of the next box's.
+constexpr int BOX_SAMPLE = 1024;
+__global__ void __launch_bounds__(BOX_SAMPLE) k_box_sample(const double4* __restrict__ boxes, int64_t n, float W,
+                                                           float H, float c, double* __restrict__ out) {
+    __shared__ float part[2][32];
+    const int m = (int)min(n, (int64_t)BOX_SAMPLE), k = threadIdx.x;
+    float v[2] = {0.0f, 0.0f};
+    if (k < m) {
+        const int64_t i = (int64_t)((double)n / m * k);
+        const double4 b = boxes[i], d = boxes[min(i + 1, n - 1)];
+        // NaN counts as no extent (and as far away)
+        const float w = (float)(b.y - b.x), h = (float)(b.w - b.z);
+        v[0] = (fminf(fmaxf(w, 0.0f), W) / c + 1.0f) * (fminf(fmaxf(h, 0.0f), H) / c + 1.0f);
+        const float dx = (float)(d.x - b.x) + 0.5f * ((float)(d.y - d.x) - w);
+        const float dy = (float)(d.z - b.z) + 0.5f * ((float)(d.w - d.z) - h);
+        v[1] = fabsf(dx) <= 16.0f * c && fabsf(dy) <= 16.0f * c ? 1.0f : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+        if ((k & 31) == 0) part[q][k >> 5] = v[q];
+    }
+    __syncthreads();
+    if (k < 32) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            v[q] = part[q][k];
+            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+            if (k == 0) out[q] = (double)v[q] / m;
+        }
+    }
+}
+
 __global__ void k_gather_rows(const double4* __restrict__ q, const int* __restrict__ order, int64_t n,
                               double4* __restrict__ out) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -3280,10 +3316,60 @@ int ct_write_boxes_records(const ct_tree* t, const double* boxes, int64_t n, con
     return CT_OK;
 }
 
+int ct_box_sample(const ct_tree* t, const double* boxes, int64_t n, double* result_host2, void* ws, size_t ws_bytes,
+                  void* stream) {
+    int s = check_tree(t);
+    if (s) return s;
+    if (n < 0 || !result_host2) return ct_fail(CT_ERR_ARG, "bad arguments");
+    result_host2[0] = result_host2[1] = 0.0;
+    if (n == 0 || t->n_elements <= 0) return CT_OK;
+    if (!ws || ws_bytes < 2 * sizeof(double)) return ct_fail(CT_ERR_WORKSPACE, "workspace too small");
+    cudaStream_t st = (cudaStream_t)stream;
+    const double W = t->bbox[1] - t->bbox[0], H = t->bbox[3] - t->bbox[2], m = (double)t->n_elements;
+    const double c = W > 0.0 && H > 0.0 ? std::sqrt(W / m * H) : std::max(W, H) / m;  // (cells in a line)
+    k_box_sample<<<1, BOX_SAMPLE, 0, st>>>((const double4*)boxes, n, (float)W, (float)H,
+                                           c > 1e-37 ? (float)std::min(c, 1e37) : 1e-37f, (double*)ws);
+    CT_CHECK_LAUNCH("box sample");
+    CT_CUDA(cudaMemcpyAsync(result_host2, ws, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CT_CUDA(cudaStreamSynchronize(st));
+    return CT_OK;
+}
+
+int ct_write_small_boxes(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order,
+                         const int64_t* offsets, int64_t total_pairs, int64_t* ii, int64_t* jj, void* ws,
+                         size_t ws_bytes, void* stream) {
+    int s = check_tree(t);
+    if (s) return s;
+    if (n == 0) return CT_OK;
+    if (deep_tree(t)) return ct_write_boxes_ws(t, boxes, n, order, offsets, total_pairs, 0, ii, jj, ws, ws_bytes, stream);
+    if (!ws || ws_bytes < ct_write_boxes_workspace_size(total_pairs, 0))
+        return ct_fail(CT_ERR_WORKSPACE, "write_boxes workspace too small");
+    cudaStream_t st = (cudaStream_t)stream;
+    const TreeQ T = make_q(t);
+    unsigned long long* njobs = (unsigned long long*)ws;
+    BoxJob* jobs = T.nbx ? (BoxJob*)((char*)ws + 256) : nullptr;
+    const int64_t cap = (total_pairs > 0 ? total_pairs : 0) / BOX_JOB_MIN + 1;
+    CT_CUDA(cudaMemsetAsync(njobs, 0, sizeof(unsigned long long), st));
+    const int bt = box_threads(t);
+    k_boxes<true, false><<<grid_of(n, bt), bt, 0, st>>>(T, (const double4*)boxes, n, order, (int64_t*)offsets, ii, jj,
+                                                       jobs, njobs, cap, BOX_JOB_MIN);
+    if (jobs) k_box_jobs<<<152 * 8, 256, 0, st>>>(jobs, njobs, cap, T.lstart, T.bbi, ii, jj, T.err);
+    CT_CHECK_LAUNCH("write_small_boxes");
+    return CT_OK;
+}
+
 int ct_count_small_boxes_spec(const ct_tree* t, const double* boxes, int64_t n, const int32_t* order, int64_t* counts,
                               int32_t* spec, int32_t spec_cap, void* stream) {
     int s = check_tree(t);
     if (s) return s;
+    if (!spec && spec_cap == 0) {  // counts alone
+        if (n == 0 || deep_tree(t)) return ct_count_boxes(t, boxes, n, order, counts, stream);
+        const int bt = box_threads(t);
+        k_boxes<false, false><<<grid_of(n, bt), bt, 0, (cudaStream_t)stream>>>(make_q(t), (const double4*)boxes, n, order,
+                                                                              counts, nullptr, nullptr);
+        CT_CHECK_LAUNCH("count_small_boxes");
+        return CT_OK;
+    }
     if (n == 0 || deep_tree(t)) return ct_count_boxes_spec(t, boxes, n, order, counts, spec, spec_cap, stream);
     if (!spec || spec_cap < 1 || spec_cap > 4096) return ct_fail(CT_ERR_ARG, "spec_cap must be in [1, 4096]");
     if (t->n_elements >= INT32_MAX) return ct_fail(CT_ERR_ARG, "tree size out of range");
