@@ -589,6 +589,11 @@ constexpr int64_t SMALL_WARP_MAX = 32768;
 
 // The cell of an open query (-1: none), or OPEN_LEFT.
 constexpr int OPEN_LEFT = -2;
+// Entries of a list that a lane goes through for an open query (the bits of
+// its mask).  The lists pass has gone through all of a longer one; a second
+// time takes longer than the traversal.  1M vertices of a mesh whose cells
+// grow 3000-fold, most lists of more: 18.8 ms the list again, 9.0 traversed.
+constexpr int OPEN_LIST_MAX = 32;
 
 __device__ __forceinline__ int open_one(const TreeL& T, double2 pp) {
     float px, py, dpx, dpy;
@@ -600,10 +605,10 @@ __device__ __forceinline__ int open_one(const TreeL& T, double2 pp) {
     const int64_t g = (int64_t)(int)fy * T.gnx + (int)fx;
     const float xl = __fsub_rd(px, dpx), xh = __fadd_ru(px, dpx);
     const float yl = __fsub_rd(py, dpy), yh = __fadd_ru(py, dpy);
-    const int64_t s1 = T.coff[g + 1];
+    const int64_t s0 = T.coff[g], s1 = T.coff[g + 1];
+    if (s1 - s0 > OPEN_LIST_MAX) return OPEN_LEFT;
     // float32 first: the lanes then meet at the float64 work, of which a point
     // near one edge has its two cells, wherever these stand in the list
-    const int64_t s0 = T.coff[g];
     unsigned todo = 0;
     int best = -1;
     bool left = false;
@@ -619,8 +624,7 @@ __device__ __forceinline__ int open_one(const TreeL& T, double2 pp) {
                 r = leaf_filter_joined(dx, dy, errd, T.dabs, T.tolf, reinterpret_cast<const float2*>(cell + 1), len32);
             }
             if (r == LF_INSIDE) best = best < 0 ? j : first_met(T, pp, best, j);
-            else if (r == LF_UNSURE && k - s0 < 32) todo |= 1u << (int)(k - s0);
-            else if (r == LF_UNSURE) left = true;
+            else if (r == LF_UNSURE) todo |= 1u << (int)(k - s0);
         }
     }
     for (; todo; todo &= todo - 1u) {
