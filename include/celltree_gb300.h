@@ -117,8 +117,9 @@ typedef struct ct_tree {
      * never results; an autotuner picks them per GPU and problem size. */
     int32_t tune_cells_bpsm;  /* candidate-list pass compiled for 4, 6 or 8 resident blocks per SM (default 6) */
     int32_t tune_fast_bpsm;   /* grid of the open-query traversal in blocks per SM, 1 .. 32 (default 16) */
-    int32_t tune_query_threads; /* block size of the box and segment traversals: 64, 128 or 256
-                                   (default 256 boxes, 128 segments; segments take at most 128) */
+    int32_t tune_query_threads; /* block size of the box and segment traversals: 64, 128 or 256 (default
+                                   256 boxes, 128 segments; segments take at most 128); boxes walked by
+                                   warps take half of it (1, 2 or 4 warps) */
     int32_t tune_fp64_stack;  /* stack entries of the plain float64 locate: 0 = smallest that fits, 64 or 512 */
     /* parent of every node (device, n_nodes int32, -1 for the root; filled by
      * ct_pack_tree when not NULL).  Trees deeper than the traversal stacks

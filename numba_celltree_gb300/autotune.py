@@ -3,19 +3,23 @@
 The library's kernels take a few launch shapes that change their speed but
 never their results: how finely the batched point location sorts its queries
 (``sort_bits``), the occupancy the candidate-list kernel is compiled for
-(``cells_bpsm``), the grid of the open-query traversal (``fast_bpsm``), the
-block size and work ordering of the box and segment traversals, the stack of
-the plain float64 form, and the density of the start-node grid and candidate
-lists built with a tree (``grid_density``).  The best choice depends on the
-GPU, on the mesh (size, cells per leaf) and on the batch, so a tuner times
-the candidates on a sample of a real call the first time a problem of that
-size class is seen, and keeps the fastest in a small JSON cache keyed by GPU
-and problem bucket (log2 of the cell and query counts):
+(``cells_bpsm``), the grid of the open-query kernel (``fast_bpsm``), the block
+size and spatial order of the box and segment traversals (``threads``,
+``work_order``), the stack of the plain float64 form, and the density of the
+start-node grid and candidate lists built with a tree (``grid_density``).
+The best choice depends on the GPU, on the mesh (size, cells per leaf) and on
+the batch.  Point location times the candidates on a sample of a real call the
+first time a problem of that size class is seen; box and segment traversals
+and the index density are timed when asked (``CellTree2d.autotune``; 20k to
+300k boxes and segments on 114k and 5M cells ran within 3 % of the best shape
+by default, too little to time candidates in a call that did not ask).  The
+fastest is kept in a small JSON cache keyed by GPU and
+problem bucket (log2 of the cell and query counts):
 
 * ``NUMBA_CELLTREE_GB300_TUNING`` -- path of the cache file (default
   ``~/.cache/numba_celltree_gb300/tuning.json``);
-* ``NUMBA_CELLTREE_GB300_AUTOTUNE`` -- ``1`` (default) tunes at first use,
-  ``0`` uses cached entries and the library defaults only.
+* ``NUMBA_CELLTREE_GB300_AUTOTUNE`` -- ``1`` (default) tunes point location
+  at first use, ``0`` uses cached entries and the library defaults only.
 
 ``cells_per_leaf`` and ``n_buckets`` shape the tree itself (its ``nodes`` and
 ``bb_indices``, which must equal the upstream package's for the same
@@ -60,9 +64,9 @@ SPACE: Dict[str, Dict[str, list]] = {
 
 # batches from which a call tunes itself at first use (smaller ones run the
 # defaults: tuning them would cost more than it saves)
-TUNE_MIN = {"locate": 1 << 20, "fp64": 1 << 20, "boxes": 1 << 16, "segments": 1 << 16}
+TUNE_MIN = {"locate": 1 << 20, "fp64": 1 << 20}
 # queries of the sample a tuning run times
-SAMPLE_MAX = {"locate": 1 << 22, "fp64": 1 << 20, "boxes": 1 << 16, "segments": 1 << 15}
+SAMPLE_MAX = {"locate": 1 << 22, "fp64": 1 << 20}
 
 
 def enabled() -> bool:

@@ -254,6 +254,9 @@ class _GpuTree:
         return self._gpu
 
     def tune_key(self, kind: str, n_queries: int) -> str:
+        if kind in ("boxes", "segments"):
+            # (entries without the mark are of versions whose work_order was by size)
+            return autotune.cache_key(kind, self.gpu(), self.n, n_queries, K=self.K, order="spatial")
         return autotune.cache_key(kind, self.gpu(), self.n, n_queries, K=self.K)
 
     def cached(self, kind: str, n_queries: int) -> dict:
@@ -281,20 +284,6 @@ class _GpuTree:
             return bool(torch.cuda.is_current_stream_capturing())
         except Exception:  # pragma: no cover
             return False
-
-    def maybe_tune(self, kind: str, n_queries: int, run, sample_n: int) -> dict:
-        """The launch shape for a batch of n_queries; tunes it first (timing
-        `run(cfg)` on a sample of sample_n queries) when autotuning is on,
-        the batch is large enough, nothing is cached for its bucket and no
-        stream capture is running."""
-        key = self.tune_key(kind, n_queries)
-        if key in self._tuned:
-            return self._tuned[key]
-        cached_entry = autotune.cache().get(key)
-        if (cached_entry is None and autotune.enabled() and n_queries >= autotune.TUNE_MIN[kind]
-                and not self._capturing()):
-            self._tuned[key] = self.tune(kind, key, run, sample_n)
-        return self.cached(kind, n_queries)
 
     def tune(self, kind: str, key: str, run, sample_n: int) -> dict:
         """Coordinate descent over the knobs of `kind` (one knob at a time,
@@ -759,9 +748,12 @@ class _GpuTree:
     ORDER_MIN_CELLS = 1 << 20
 
     def in_spatial_order(self, n: int, config: dict) -> bool:
-        """Whether a batch of n boxes / segments runs in spatial order."""
-        return n > 0 and (bool(config.get("work_order")) or
-                          (n >= self.WORK_ORDER_MIN and self.n >= self.ORDER_MIN_CELLS))
+        """Whether a batch of n boxes / segments runs in spatial order:
+        config["work_order"] True or False, None the rule by sizes."""
+        want = config.get("work_order")
+        if want is None:
+            want = n >= self.WORK_ORDER_MIN and self.n >= self.ORDER_MIN_CELLS
+        return n > 0 and bool(want)
 
     def spatial_order(self, q_d, kind: int):
         """Permutation of box (kind 0) / segment (kind 1) queries by a 256 x

@@ -35,6 +35,7 @@ struct TreeQ {
     int64_t n_nodes;
     dbox bbox;
     int K;
+    int box_warps, seg_warps;  // warps per block of the walks by warps
     bool finite;  // all node bounds and cell boxes finite: order comparisons on integer keys
     // box index (ct_pack_box_index; null when not built)
     const double4* bbl;        // cell boxes in leaf order
@@ -541,7 +542,7 @@ struct BoxWalk {
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const double4* __restrict__ boxes, int64_t n,
+__global__ void __launch_bounds__(32 * WALK_WARPS, WALK_BLOCKS) k_box_walk(TreeQ T, const double4* __restrict__ boxes, int64_t n,
                                                               const int* __restrict__ order, int per_warp,
                                                               int64_t* __restrict__ cnt_or_off,
                                                               int64_t* __restrict__ ii, int64_t* __restrict__ jj,
@@ -549,11 +550,10 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const dou
                                                               const int64_t* __restrict__ spec_cnt, BoxRecs recs) {
     constexpr bool WRITE = MODE == BOX_WRITE;
     if (WRITE && recs.count && *recs.count <= (unsigned long long)recs.cap) return;  // written from the records
-    __shared__ WalkBuf bufs[WALK_WARPS];
-    __shared__ WalkBox qs[WALK_WARPS][WALK_Q];
-    __shared__ int64_t counts[WALK_WARPS][WALK_Q];
+    extern __shared__ __align__(16) unsigned char walk_smem[];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const int64_t t0 = ((int64_t)blockIdx.x * WALK_WARPS + wi) * per_warp;
+    WalkShared<WalkBox, int64_t>& S0 = reinterpret_cast<WalkShared<WalkBox, int64_t>*>(walk_smem)[wi];
+    const int64_t t0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + wi) * per_warp;
     if (t0 >= n) return;
     const bool valid = lane < per_warp && t0 + lane < n;
     int64_t i = 0;
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const dou
             b.ymax = q4.w;
             start = boxes_intersect(b, T.bbox);
             if (start) {
-                WalkBox& S = qs[wi][lane];
+                WalkBox& S = S0.query[lane];
                 S.keys = T.finite && not_nan(b.xmin) && not_nan(b.xmax) && not_nan(b.ymin) && not_nan(b.ymax);
                 S.kx0 = fkey(b.xmin);
                 S.kx1 = fkey(b.xmax);
@@ -592,12 +592,12 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_box_walk(TreeQ T, const dou
             }
         }
     }
-    if (lane < WALK_Q) counts[wi][lane] = 0;
-    const int nq = walk_begin(bufs[wi], start ? 0 : -1, lane);
-    BoxWalk<MODE> pol{T, boxes, qs[wi], counts[wi], lane, ii, jj, spec, spcap, recs};
-    walk(pol, bufs[wi], nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
+    if (lane < WALK_Q) S0.count[lane] = 0;
+    const int nq = walk_begin(S0.buf, start ? 0 : -1, lane);
+    BoxWalk<MODE> pol{T, boxes, S0.query, S0.count, lane, ii, jj, spec, spcap, recs};
+    walk(pol, S0.buf, nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
     __syncwarp();
-    if (!WRITE && valid) cnt_or_off[i] = counts[wi][lane];
+    if (!WRITE && valid) cnt_or_off[i] = S0.count[lane];
 }
 
 // The pairs of the counting pass's records (of the writing pass's, when those
@@ -996,16 +996,15 @@ struct SegWalk {
 };
 
 template <int MODE, bool ITEMS, bool WRITE>
-__global__ void __launch_bounds__(32 * WALK_WARPS) k_edge_walk(
+__global__ void __launch_bounds__(32 * WALK_WARPS, WALK_BLOCKS) k_edge_walk(
     TreeQ T, const double4* __restrict__ segs, int64_t n, const int* __restrict__ order,
     const int* __restrict__ item_seg, const int* __restrict__ item_node, int cut, int per_warp,
     int64_t* __restrict__ cnt_or_off, int* __restrict__ out_seg, int* __restrict__ out_val, int spcap,
     const int64_t* __restrict__ spec_cnt) {
-    __shared__ WalkBuf bufs[WALK_WARPS];
-    __shared__ WalkSeg qs[WALK_WARPS][WALK_Q];
-    __shared__ int counts[WALK_WARPS][WALK_Q];
+    extern __shared__ __align__(16) unsigned char walk_smem[];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const int64_t t0 = ((int64_t)blockIdx.x * WALK_WARPS + wi) * per_warp;
+    WalkShared<WalkSeg, int>& S0 = reinterpret_cast<WalkShared<WalkSeg, int>*>(walk_smem)[wi];
+    const int64_t t0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + wi) * per_warp;
     if (t0 >= n) return;
     const bool valid = lane < per_warp && t0 + lane < n;
     int64_t row = 0;
@@ -1029,7 +1028,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_edge_walk(
             if (start >= 0) {
                 const dpt V = vsub(b, a);
                 const EdgeKeys K = edge_keys(T, a, b);
-                WalkSeg& S = qs[wi][lane];
+                WalkSeg& S = S0.query[lane];
                 S.kax = K.kax;
                 S.kay = K.kay;
                 S.kbx = K.kbx;
@@ -1043,12 +1042,12 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) k_edge_walk(
             }
         }
     }
-    if (lane < WALK_Q) counts[wi][lane] = 0;
-    const int nq = walk_begin(bufs[wi], start, lane);
-    SegWalk<MODE, ITEMS, WRITE> pol{T, segs, qs[wi], counts[wi], lane, cut, out_seg, out_val, spcap};
-    walk(pol, bufs[wi], nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
+    if (lane < WALK_Q) S0.count[lane] = 0;
+    const int nq = walk_begin(S0.buf, start, lane);
+    SegWalk<MODE, ITEMS, WRITE> pol{T, segs, S0.query, S0.count, lane, cut, out_seg, out_val, spcap};
+    walk(pol, S0.buf, nq, lane, (int64_t)per_warp * (T.n_nodes + 1), T.err);
     __syncwarp();
-    if (!WRITE && valid) cnt_or_off[row] = counts[wi][lane];
+    if (!WRITE && valid) cnt_or_off[row] = S0.count[lane];
 }
 
 // Trees deeper than the walk's reserve: one thread per segment through the
@@ -2875,6 +2874,16 @@ __global__ void k_gather_rows(const double4* __restrict__ q, const int* __restri
         out[i] = q[order[i]];
 }
 
+// block sizes of the traversal kernels (the tree's launch shape, else the defaults)
+static int box_threads(const ct_tree* t) {
+    int b = t->tune_query_threads;
+    return (b == 64 || b == 128 || b == 256) ? b : 256;
+}
+static int seg_threads(const ct_tree* t) {
+    int b = t->tune_query_threads;
+    return (b == 64 || b == 128) ? b : 128;
+}
+
 TreeQ make_q(const ct_tree* t) {
     TreeQ T;
     T.nf = (const float4*)t->nodes_f32;
@@ -2891,6 +2900,8 @@ TreeQ make_q(const ct_tree* t) {
     T.bbox.ymax = t->bbox[3];
     T.K = t->n_max_vert;
     T.finite = t->bounds_finite != 0;
+    T.box_warps = box_threads(t) / 64;  // 1, 2, 4
+    T.seg_warps = seg_threads(t) / 32;  // 2, 4
     const bool box_index = t->node_box && t->leaf_start && t->bb_leaf && T.finite;
     T.bbl = box_index ? (const double4*)t->bb_leaf : nullptr;
     T.nbx = box_index ? (const NodeBox*)t->node_box : nullptr;
@@ -3026,7 +3037,9 @@ static void launch_box_walk(const TreeQ& T, const double4* boxes, int64_t n, con
                             int64_t* ii, int64_t* jj, int* spec, int spcap, const int64_t* spec_cnt,
                             cudaStream_t st, BoxRecs recs = {}) {
     const int per_warp = walk_tasks(n);
-    k_box_walk<MODE><<<grid_of((n + per_warp - 1) / per_warp, WALK_WARPS), 32 * WALK_WARPS, 0, st>>>(
+    const int w = T.box_warps;
+    const size_t smem = w * sizeof(WalkShared<WalkBox, int64_t>);
+    k_box_walk<MODE><<<grid_of((n + per_warp - 1) / per_warp, w), 32 * w, smem, st>>>(
         T, boxes, n, order, per_warp, cnt_or_off, ii, jj, spec, spcap, spec_cnt, recs);
 }
 
@@ -3035,13 +3048,15 @@ static void launch_edge_walk(int mode, const TreeQ& T, const double4* segs, int6
                              const int* item_seg, const int* item_node, int cut, int64_t* cnt_or_off, int* out_seg,
                              int* out_val, int spcap, const int64_t* spec_cnt, cudaStream_t st) {
     const int per_warp = walk_tasks(n);
-    const unsigned g = grid_of((n + per_warp - 1) / per_warp, WALK_WARPS);
+    const int w = T.seg_warps;
+    const unsigned g = grid_of((n + per_warp - 1) / per_warp, w);
+    const size_t smem = w * sizeof(WalkShared<WalkSeg, int>);
     if (mode == 0)
-        k_edge_walk<0, ITEMS, WRITE><<<g, 32 * WALK_WARPS, 0, st>>>(T, segs, n, order, item_seg, item_node, cut,
+        k_edge_walk<0, ITEMS, WRITE><<<g, 32 * w, smem, st>>>(T, segs, n, order, item_seg, item_node, cut,
                                                                     per_warp, cnt_or_off, out_seg, out_val, spcap,
                                                                     spec_cnt);
     else
-        k_edge_walk<1, ITEMS, WRITE><<<g, 32 * WALK_WARPS, 0, st>>>(T, segs, n, order, item_seg, item_node, cut,
+        k_edge_walk<1, ITEMS, WRITE><<<g, 32 * w, smem, st>>>(T, segs, n, order, item_seg, item_node, cut,
                                                                     per_warp, cnt_or_off, out_seg, out_val, spcap,
                                                                     spec_cnt);
 }
@@ -3109,7 +3124,6 @@ int ct_pack_box_index(ct_tree* t, void* scratch, size_t scratch_bytes, void* str
     return CT_OK;
 }
 
-// block sizes of the traversal kernels (the tree's launch shape, else the defaults)
 // Polygons of up to 8 vertices take the shared-memory clip, longer ones the
 // general one (shared memory of a block: 31, 33 and 41 KB for clippers of up
 // to 3, 4 and 8 vertices).
@@ -3134,15 +3148,6 @@ static void launch_clip_area(const double4* boxes, const double* va, const int64
         else if (Kb <= 4) go(std::integral_constant<int, 4>());
         else go(std::integral_constant<int, 8>());
     }
-}
-
-static int box_threads(const ct_tree* t) {
-    int b = t->tune_query_threads;
-    return (b == 64 || b == 128 || b == 256) ? b : 256;
-}
-static int seg_threads(const ct_tree* t) {
-    int b = t->tune_query_threads;
-    return (b == 64 || b == 128) ? b : 128;
 }
 
 static int check_tree(const ct_tree* t) {

@@ -24,7 +24,8 @@
 #include "ct_common.cuh"
 
 constexpr int WALK_CAP = 512;      // nodes per queue (two per warp)
-constexpr int WALK_WARPS = 4;      // warps per block
+constexpr int WALK_WARPS = 4;      // warps per block, at most and by default
+constexpr int WALK_BLOCKS = 8;     // such blocks per SM (28 KB of shared memory each)
 // Queries per warp, at most.  More (16, 32, let in a few at a time) fill the
 // rounds of tiny queries better but leave fewer warps, and the heavy ones of
 // a batch end later: 250k boxes of very different sizes 33.5 -> 34.2 -> 35.6
@@ -41,6 +42,14 @@ enum { WALK_DROP = 0, WALK_OPEN = 1, WALK_LEAF = 2, WALK_ALL = 3 };
 struct WalkBuf {
     int node[2][WALK_CAP];
     unsigned short meta[2][WALK_CAP];
+};
+
+// A warp's shared memory: its queue, the queries, results reported of each.
+template <class Query, class Count>
+struct WalkShared {
+    WalkBuf buf;
+    Query query[WALK_Q];
+    Count count[WALK_Q];
 };
 
 // Puts the first nodes (-1: none) of the warp's queries (lane = query) into
