@@ -335,7 +335,7 @@ struct BoxRecs {
     unsigned long long* count;   // records the counting pass asked for (null: there was none)
     unsigned long long* pushed;  // records of the writing pass
     int64_t cap;
-    int part;
+    int part;  // of the writing pass (of the counting pass: REC_PART)
     uint8_t* inside;  // optional, per pair: the cell lies in a subtree inside the box
 };
 constexpr int REC_FLAG = (int)0x80000000u;
@@ -473,11 +473,12 @@ struct BoxWalk {
             const unsigned long long at = __shfl_sync(FULL, first, src);
             const int id = __shfl_sync(FULL, r.x, src), rank = __shfl_sync(FULL, r.y, src);
             const int ptr = __shfl_sync(FULL, r.z, src), end = ptr + __shfl_sync(FULL, r.w, src);
+            const int part = MODE == BOX_RECORD ? REC_PART : recs.part;
             const bool none = whole && at + (unsigned)k > cap;  // slots before the end get no cells
             for (int t = lane; t < k && at + (unsigned)t < cap; t += 32) {
                 int p0 = ptr, p1 = end;
-                if (t > 0) p0 = max(ptr, min(T.lstart[ptr + t * recs.part], ptr + t * recs.part));
-                if (t + 1 < k) p1 = max(p0, min(T.lstart[ptr + (t + 1) * recs.part], end));
+                if (t > 0) p0 = max(ptr, min(T.lstart[ptr + t * part], ptr + t * part));
+                if (t + 1 < k) p1 = max(p0, min(T.lstart[ptr + (t + 1) * part], end));
                 recs.rec[at + (unsigned)t] = none ? make_int4(id, 0, ptr, 0) : make_int4(id, rank + (end - p1), p0, p1 - p0);
             }
         }
@@ -509,7 +510,7 @@ struct BoxWalk {
         }
         const int64_t rank = walk_rank<int64_t>(qi, c, have, lane, emitted);
         if (MODE == BOX_RECORD) {
-            const int parts = c == 0 ? 0 : all && c >= 2 * recs.part ? (int)c / recs.part : 1;
+            const int parts = c == 0 ? 0 : all && c >= 2 * REC_PART ? (int)c / REC_PART : 1;
             keep_records(recs.count, parts, false,
                          make_int4((int)S.id | (all ? REC_FLAG : 0), (int)rank | (!all && size > 32 ? REC_FLAG : 0), ptr,
                                    all || size > 32 ? size : (int)hit));
