@@ -2654,6 +2654,10 @@ __global__ void __launch_bounds__(128) k_barycentric_small(const double2* __rest
 #pragma unroll
     for (int k = 3; k < KT; k++)
         if (k == len - 1) last = idx[k];
+    if (last == idx[0]) {  // a closed ring: an edge of no length, never clear
+        bary_general(pp, f, (const double*)v, faces, K, tol, w);
+        return;
+    }
     double2 poly[KT];
 #pragma unroll
     for (int k = 0; k < KT; k++) poly[k] = k < len ? v[idx[k]] : make_double2(0.0, 0.0);

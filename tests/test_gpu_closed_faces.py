@@ -47,3 +47,13 @@ def test_batch(oracle, form):
     for g, (v, e, p) in zip(got, ((xy, f, pts[:5000]), (x2, f2, p2))):
         g = g.cpu().numpy() if hasattr(g, "cpu") else np.asarray(g)
         assert np.array_equal(g, oracle.OracleCellTree2d(v, e, -1).locate_points(p))
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_weights(oracle, form):
+    from numba_celltree_gb300 import CellTree2d
+
+    xy, f, pts = inputs(form, (0.0, 0.0))
+    wi, ww = oracle.OracleCellTree2d(xy, f, -1).compute_barycentric_weights(pts[:5000])
+    gi, gw = CellTree2d(xy, f, -1).compute_barycentric_weights(pts[:5000])
+    assert np.array_equal(gi, wi) and np.array_equal(gw, ww, equal_nan=True)
