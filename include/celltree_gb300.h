@@ -449,7 +449,9 @@ int ct_exclusive_scan(const int64_t* in, int64_t n, int64_t* out, void* workspac
  * counterpart): a permutation grouping queries of similar size (box area /
  * segment length with a cell-size margin, 8-bit log classes), so one
  * warp's queries take similar time.  Passing it as `order` below changes no
- * result: counts and pairs stay indexed and ordered by query. */
+ * result: counts and pairs stay indexed and ordered by query.  It pays where a
+ * query is a thread's (trees deeper than the traversal stacks); for the walks
+ * by warps ct_spatial_order is the better one. */
 size_t ct_work_order_workspace_size(int64_t n);
 int ct_work_order(const double* queries, int64_t n, int32_t kind, double cell_size, int32_t* order, void* workspace,
                   size_t workspace_bytes, void* stream);
@@ -566,9 +568,9 @@ int ct_write_edge_candidates_spec(const ct_tree* tree, int32_t mode, const doubl
                                   const int32_t* order, const int64_t* counts, const int64_t* offsets,
                                   const int32_t* spec, int32_t spec_cap, int32_t* cand_seg, int32_t* cand_pos,
                                   void* stream);
-/* The same candidates with each segment's traversal split across threads
- * (no upstream counterpart; a long segment's traversal otherwise runs on one
- * thread).  ct_count/write_edge_items cut every segment's traversal `cut`
+/* The same candidates with each segment's traversal split across warps (no
+ * upstream counterpart; a long segment's traversal otherwise runs on one
+ * warp).  ct_count/write_edge_items cut every segment's traversal `cut`
  * levels below the root: the nodes at that depth (and the leaves above it)
  * it reaches, in traversal order, as work items (segment, node), segment-
  * major at the scanned per-segment offsets.  ct_count/write_item_candidates
@@ -631,12 +633,16 @@ int ct_finish_edge_hits(const ct_tree* tree, const double* segs, const int32_t* 
 /* Diagnostics for tests of the segment test's float32 certificates (face
  * trees): per (segment, leaf position) pair, out[3t] = upstream's float64
  * Cohen-Sutherland verdict (1 accept, 0 reject), out[3t+1] = the float32
- * interval verdict used by ct_test_edge_candidates (1, 0, or -1 undecided),
+ * interval verdict of the cell test's general form (1, 0, or -1 undecided),
  * out[3t+2] = 1 when the traversal's line filter surely misses the cell's
  * box (needs bb_leaf32).  A certificate is sound when out[3t+1] is -1 or
  * equals out[3t], and out[3t+2] = 1 only where out[3t] = 0. */
 int ct_cs_certificates(const ct_tree* tree, const double* segs, const int32_t* cand_seg, const int32_t* cand_pos,
                        int64_t n_cand, int8_t* out, void* stream);
+/* The same results in four calls that synchronise nothing, for callers that
+ * allocate for every candidate: the cell test (keep int64, to be scanned into
+ * pos), the hits in candidate order with each segment's offset and count, and
+ * the sort below. */
 int ct_test_edge_candidates(const ct_tree* tree, int32_t mode, const double* segs, const int32_t* cand_seg,
                             const int32_t* cand_pos, int64_t n_cand, int64_t* keep, double* xy, void* stream);
 int ct_compact_edge_hits(const ct_tree* tree, const int64_t* keep, const int64_t* pos, int64_t n_cand,
@@ -808,6 +814,7 @@ int ct_points_in_triangles(const double* points, const int64_t* face_indices, in
  * mean[r] = sum(w x[col]) / sum(w) over row r (NaN without weight),
  * weight_sum[r] = sum(w) (may be NULL). */
 size_t ct_csr_workspace_size(int64_t n_rows);
+/* (row_ptr is found by binary search; the workspace is not used any more) */
 int ct_csr_row_ptr(const int64_t* rows, int64_t n_pairs, int64_t n_rows, int64_t* row_ptr, void* workspace,
                    size_t workspace_bytes, unsigned int* error_word, void* stream);
 int ct_csr_weighted_mean(const int64_t* row_ptr, const int64_t* cols, const double* weights, int64_t n_rows,

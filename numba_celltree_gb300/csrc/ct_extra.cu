@@ -12,8 +12,6 @@
 #include "ct_internal.h"
 #include "ct_sf64.cuh"
 
-extern "C" size_t ct_scan_workspace_size(int64_t n);
-
 namespace cte {
 
 // point_inside_box geometry_utils.py:528-529 (strict)
@@ -287,7 +285,8 @@ int ct_points_in_triangles(const double* points, const int64_t* face_indices, in
 }
 
 size_t ct_csr_workspace_size(int64_t n_rows) {
-    return ((size_t)8 * (size_t)(n_rows + 1) + 255) / 256 * 256 + ct_scan_workspace_size(n_rows + 1);
+    (void)n_rows;
+    return 256;  // not used: an interface of callers
 }
 
 int ct_csr_row_ptr(const int64_t* rows, int64_t n_pairs, int64_t n_rows, int64_t* row_ptr, void* ws,
