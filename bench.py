@@ -935,7 +935,7 @@ def main():
             "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
             "traffic": (round(tpp * n) if tpp is not None else None),
             "kernel": "float32 pass: ctl::k_cells<3> (candidate lists, results by sorted position) + "
-                      "ctl::k_res_bucket + ctl::k_res_unbucket (their scatter) + ctl::k_fast<3> (open queries)",
+                      "ctl::k_res_bucket + ctl::k_res_unbucket (their scatter) + ctl::k_open (open queries)",
             "kernel_ms": round(ms_fast, 3)}
     result = {
         "metric": METRIC,
