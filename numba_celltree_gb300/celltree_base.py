@@ -576,11 +576,10 @@ class _GpuTree:
         free, _ = torch.cuda.mem_get_info(self.device)
         return max(1 << 20, int(free // 4 // max(bytes_per_result, 1)))
 
-    # pairs from which subtrees inside a box are written by a warp each after
+    # pairs from which large subtrees inside a box are queued and written after
     # the traversal (below, the extra launch costs more than it saves)
     BOX_JOBS_MIN_PAIRS = 1 << 20
-    # boxes counted by a thread each, and batches without room for records
-    # (below): the counting pass keeps each box's first SPEC_CAP pairs (up to
+    # boxes counted by a thread each, and batches without records (below): the counting pass keeps each box's first SPEC_CAP pairs (up to
     # SPEC_MAX_BOXES boxes; SPEC_CAP_LARGE beyond, scratch up to
     # SPEC_MAX_BYTES), so boxes whose pairs fit are traversed once;
     # SPEC_MAX_BOXES = 0 switches both off
